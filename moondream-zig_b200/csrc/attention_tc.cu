@@ -59,6 +59,7 @@ namespace {
 using namespace tc;
 
 constexpr int ABQ = 128, ABKV = 64;
+constexpr int MASK_CHUNKS = 4;
 constexpr int ATTN_THREADS = 224;   // producer, S issuer, 4 softmax warps, PV issuer
 constexpr float LOG2E_F = 1.4426950408889634f;
 constexpr float RESCALE_THRESHOLD = 8.0f;  // log2 units a row maximum may grow before O is rescaled
@@ -66,7 +67,11 @@ constexpr float RESCALE_THRESHOLD = 8.0f;  // log2 units a row maximum may grow 
 struct AttnTcParams {
     int q_len, kv_len, causal_pos;
     float scale_log2;
-    const uint8_t* mask;  // [q_len, kv_len] or null
+    // explicit mask (null: none), as mask_bits_kernel leaves it: bit e of words[tile * q_pad + row] = key 64 * tile + e is
+    // visible to that row, and the span of tiles a query block sees at all, in MASK_CHUNKS parts
+    const unsigned long long* mask_words;
+    const int2* mask_span;
+    int q_pad;
     // 4-D tensor maps (dim 0 = head dimension d; dims 1..3 = row, head, batch in order of ascending stride):
     // which map dimension carries the row / head / batch index, for q and for k, v
     int q_dim_row, q_dim_head, q_dim_batch, kv_dim_row, kv_dim_head, kv_dim_batch;
@@ -77,10 +82,11 @@ struct AttnTcParams {
 // Item w -> (query block, head, batch).  Causal: the last query blocks see the most keys, so they come first
 // (longest items first when a CTA takes several); otherwise the query blocks of one (batch, head) are neighbours,
 // so the CTAs that run together share K and V in L2.
+template <bool MASKED>
 __device__ __forceinline__ void attn_item(const AttnTcParams& p, int w, int& qblk, int& head, int& batch) {
     const int hb = p.n_heads * p.n_batch;
     int r;
-    if (p.causal_pos >= 0) { qblk = p.n_qblk - 1 - w / hb; r = w % hb; }
+    if (MASKED || p.causal_pos >= 0) { qblk = p.n_qblk - 1 - w / hb; r = w % hb; }
     else { qblk = w % p.n_qblk; r = w / p.n_qblk; }
     head = r % p.n_heads;
     batch = r / p.n_heads;
@@ -92,10 +98,72 @@ __device__ __forceinline__ int attn_walk(const AttnTcParams& p, int it) {
     const long long w = (long long)it * gridDim.x + c;
     return w < p.n_items ? (int)w : -1;
 }
-__device__ __forceinline__ int attn_tiles(const AttnTcParams& p, int q0) {
+// Number of key tiles of a query block, and the first of them.
+template <bool MASKED>
+__device__ __forceinline__ int attn_tiles(const AttnTcParams& p, int qblk, int& first) {
+    first = 0;
+    if (MASKED) {
+        int lo = INT_MAX, hi = 0;
+#pragma unroll
+        for (int c = 0; c < MASK_CHUNKS; ++c) {
+            const int2 s = __ldcg(p.mask_span + qblk * MASK_CHUNKS + c);
+            lo = min(lo, s.x);
+            hi = max(hi, s.y);
+        }
+        if (lo >= hi) return 0;
+        first = lo;
+        return hi - lo;
+    }
     int kv_end = p.kv_len;
-    if (p.causal_pos >= 0) kv_end = min(kv_end, p.causal_pos + min(q0 + ABQ, p.q_len));
+    if (p.causal_pos >= 0) kv_end = min(kv_end, p.causal_pos + min(qblk * ABQ + ABQ, p.q_len));
     return (kv_end + ABKV - 1) / ABKV;
+}
+
+// A byte mask [q_len, kv_len] as bits, one 64-bit word per row and key tile, and the span of tiles in which some row of a query
+// block sees a key (the attention skips the others, as its causal form does; a row that sees no key at all gives zeros).
+// The attention used to read the bytes itself, every thread the 64 of its own row: with 32 heads that is 32 times the whole
+// mask in single-byte loads of 32 different lines each, and it took 178 us for 32 heads, 761 rows and 761 keys.  With the
+// words (one coalesced 8-byte load per row and tile, requested a tile ahead) it takes about as long as the causal form.
+// Grid (query blocks, MASK_CHUNKS): a block packs its part of the tiles for 128 rows, a warp four rows at a time.  The loads
+// stay single bytes because rows start at any address; a warp's 32 are consecutive.  An image's attention, a causal mask's
+// making, this attention with it and one of a single token: 209 -> 54 us.
+__global__ void __launch_bounds__(1024)
+mask_bits_kernel(const uint8_t* __restrict__ mask, unsigned long long* __restrict__ words, int2* __restrict__ span, int q_len,
+                 int kv_len, int q_pad) {
+    __shared__ int lo, hi;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nt = (kv_len + ABKV - 1) / ABKV, per = (nt + MASK_CHUNKS - 1) / MASK_CHUNKS;
+    const int t0 = blockIdx.y * per, t1 = min(nt, t0 + per);
+    if (threadIdx.x == 0) { lo = INT_MAX; hi = 0; }
+    md_pdl_launch_dependents();
+    __syncthreads();
+    md_pdl_wait();
+    const int row0 = blockIdx.x * ABQ + warp * 4;
+    for (int t = t0; t < t1; ++t) {
+        const int key = t * ABKV + lane;
+        bool a[4], b[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const uint8_t* m = mask + (size_t)(row0 + r) * kv_len;
+            a[r] = row0 + r < q_len && key < kv_len && m[key] != 0;
+            b[r] = row0 + r < q_len && key + 32 < kv_len && m[key + 32] != 0;
+        }
+        unsigned long long w = 0ull, any = 0ull;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const unsigned long long v =
+                (unsigned long long)__ballot_sync(0xffffffffu, a[r]) | ((unsigned long long)__ballot_sync(0xffffffffu, b[r]) << 32);
+            any |= v;
+            if (lane == r) w = v;
+        }
+        if (lane < 4) words[(size_t)t * q_pad + row0 + lane] = w;
+        if (lane == 0 && any) {
+            atomicMin(&lo, t);
+            atomicMax(&hi, t + 1);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) span[blockIdx.x * MASK_CHUNKS + blockIdx.y] = make_int2(lo, hi);
 }
 
 struct AttnTcMaps {
@@ -118,7 +186,7 @@ template <int D> struct AttnCfg {
     static constexpr int SMEM = 1024 + Q_BYTES + STAGES * STAGE_BYTES + V_STAGES * V_STAGE_BYTES + OUT_BYTES + 256;  // 101.25 / 73.25 KB
 };
 
-template <int D>
+template <int D, bool MASKED>
 __global__ void __launch_bounds__(ATTN_THREADS, 2)
 attn_tc_kernel(const __grid_constant__ AttnTcMaps tm, AttnTcParams p, md_devflags* flags) {
     using Cfg = AttnCfg<D>;
@@ -203,9 +271,9 @@ attn_tc_kernel(const __grid_constant__ AttnTcMaps tm, AttnTcParams p, md_devflag
         // ------------------------------------------------------------------ TMA producer
         if (lane == 0) {
             uint32_t kst = 0, kpar = 1, vst = 0, vpar = 1;  // ring slots and the parities that say "slot free"
-            int ck[4] = {0, 0, 0, 0};
+            int ck[4] = {0, 0, 0, 0}, first = 0;
             auto load_k = [&](int j) {
-                ck[p.kv_dim_row] = j * ABKV;
+                ck[p.kv_dim_row] = (first + j) * ABKV;
                 mbar_wait(b_kempty + 8 * kst, kpar, abort_flag, flags, 11);
                 const uint32_t kfull = b_kfull + 8 * kst, kdst = sm_k + kst * Cfg::STAGE_BYTES;
                 mbar_expect_tx(kfull, Cfg::STAGE_BYTES);
@@ -216,8 +284,8 @@ attn_tc_kernel(const __grid_constant__ AttnTcMaps tm, AttnTcParams p, md_devflag
             int it = 0;
             for (int w; (w = attn_walk(p, it)) >= 0; ++it) {
                 int qblk, head, batch;
-                attn_item(p, w, qblk, head, batch);
-                const int q0 = qblk * ABQ, nt = attn_tiles(p, q0);
+                attn_item<MASKED>(p, w, qblk, head, batch);
+                const int q0 = qblk * ABQ, nt = attn_tiles<MASKED>(p, qblk, first);
                 int cq[4] = {0, 0, 0, 0};
                 cq[p.q_dim_row] = q0; cq[p.q_dim_head] = head; cq[p.q_dim_batch] = batch;
                 ck[p.kv_dim_head] = head; ck[p.kv_dim_batch] = batch;
@@ -229,7 +297,7 @@ attn_tc_kernel(const __grid_constant__ AttnTcMaps tm, AttnTcParams p, md_devflag
                 if (nt > 0) load_k(0);
                 for (int j = 0; j < nt; ++j) {
                     if (j + 1 < nt) load_k(j + 1);
-                    ck[p.kv_dim_row] = j * ABKV;
+                    ck[p.kv_dim_row] = (first + j) * ABKV;
                     mbar_wait(b_vempty + 8 * vst, vpar, abort_flag, flags, 10);
                     const uint32_t vfull = b_vfull + 8 * vst, vdst = sm_v + vst * Cfg::V_STAGE_BYTES;
                     mbar_expect_tx(vfull, Cfg::V_STAGE_BYTES);
@@ -262,8 +330,9 @@ attn_tc_kernel(const __grid_constant__ AttnTcMaps tm, AttnTcParams p, md_devflag
             int it = 0;
             for (int w; (w = attn_walk(p, it)) >= 0; ++it) {
                 int qblk, head, batch;
-                attn_item(p, w, qblk, head, batch);
-                const int nt = attn_tiles(p, qblk * ABQ);
+                attn_item<MASKED>(p, w, qblk, head, batch);
+                int first;
+                const int nt = attn_tiles<MASKED>(p, qblk, first);
                 if (nt > 0) mbar_wait(b_qcopied, (uint32_t)(it & 1), abort_flag, flags, 14);
                 for (int j = 0; j < nt; ++j) {
                     const uint32_t gj = g + (uint32_t)j, sb = gj & 1u;
@@ -297,8 +366,9 @@ attn_tc_kernel(const __grid_constant__ AttnTcMaps tm, AttnTcParams p, md_devflag
             int it = 0;
             for (int w; (w = attn_walk(p, it)) >= 0; ++it) {
                 int qblk, head, batch;
-                attn_item(p, w, qblk, head, batch);
-                const int nt = attn_tiles(p, qblk * ABQ);
+                attn_item<MASKED>(p, w, qblk, head, batch);
+                int first;
+                const int nt = attn_tiles<MASKED>(p, qblk, first);
                 for (int j = 0; j < nt; ++j) {
                     const uint32_t gj = g + (uint32_t)j, pb = gj & 1u;
                     mbar_wait(b_vfull + 8 * st, par, abort_flag, flags, 13);
@@ -362,14 +432,20 @@ attn_tc_kernel(const __grid_constant__ AttnTcMaps tm, AttnTcParams p, md_devflag
         if (attn_walk(p, 0) >= 0) copy_q(0);
         for (int w; (w = attn_walk(p, it)) >= 0; ++it) {
             int qblk, head, batch;
-            attn_item(p, w, qblk, head, batch);
-            const int q0 = qblk * ABQ, nt = attn_tiles(p, q0), qi = q0 + row;
+            attn_item<MASKED>(p, w, qblk, head, batch);
+            int first;
+            const int q0 = qblk * ABQ, nt = attn_tiles<MASKED>(p, qblk, first), qi = q0 + row;
             const bool row_ok = qi < p.q_len;
+            // the row's visibility word of the next tile, requested a tile ahead
+            const unsigned long long* words = MASKED ? p.mask_words + (size_t)first * p.q_pad + qi : nullptr;
+            unsigned long long seen_next = MASKED && nt > 0 ? __ldcg(words) : 0ull;
             float m_run = -INFINITY, l_run = 0.f;  // exponent reference (log2 units) and row sum on that reference
 
             for (int j = 0; j < nt; ++j) {
                 const uint32_t gj = g + (uint32_t)j;
-                const int sb = (int)(gj & 1u), key0 = j * ABKV;
+                const int sb = (int)(gj & 1u), key0 = (first + j) * ABKV;
+                const unsigned long long seen = seen_next;
+                if (MASKED && j + 1 < nt) seen_next = __ldcg(words + (size_t)(j + 1) * p.q_pad);
                 mbar_wait(b_sfull + 8 * sb, (gj >> 1) & 1u, abort_flag, flags, 19);
                 tc_fence_after();
                 uint32_t s0[32], s1[32];
@@ -378,9 +454,9 @@ attn_tc_kernel(const __grid_constant__ AttnTcMaps tm, AttnTcParams p, md_devflag
                 tc_wait_ld();
 
                 // tiles wholly inside the valid, visible region (all but the last ones) skip the per-key tests
-                const bool interior = !p.mask && key0 + ABKV <= p.kv_len &&
-                                      (p.causal_pos < 0 || key0 + ABKV - 1 <= p.causal_pos + q0 + quad * 32);
-                if (!interior && !p.mask) {
+                const bool interior = MASKED ? __all_sync(0xffffffffu, seen == ~0ull)
+                                                   : key0 + ABKV <= p.kv_len && (p.causal_pos < 0 || key0 + ABKV - 1 <= p.causal_pos + q0 + quad * 32);
+                if (!MASKED && !interior) {
                     // the visible keys of a row are a prefix of the tile: the first n_vis of its 64
                     int n_vis = p.kv_len - key0;
                     if (p.causal_pos >= 0) n_vis = min(n_vis, p.causal_pos + qi - key0 + 1);
@@ -391,15 +467,11 @@ attn_tc_kernel(const __grid_constant__ AttnTcMaps tm, AttnTcParams p, md_devflag
                         if (e + 32 >= n_vis) s1[e] = 0xff800000u;
                     }
                 } else if (!interior) {
+                    const uint32_t lo = (uint32_t)seen, hi = (uint32_t)(seen >> 32);
 #pragma unroll
-                    for (int e = 0; e < 64; ++e) {
-                        const int key = key0 + e;
-                        bool vis = row_ok && key < p.kv_len;
-                        if (p.causal_pos >= 0) vis = vis && key <= p.causal_pos + qi;
-                        if (vis && p.mask) vis = p.mask[(long long)qi * p.kv_len + key] != 0;
-                        if (!vis) {
-                            if (e < 32) s0[e] = 0xff800000u; else s1[e - 32] = 0xff800000u;  // -inf
-                        }
+                    for (int e = 0; e < 32; ++e) {
+                        if (!(lo >> e & 1u)) s0[e] = 0xff800000u;
+                        if (!(hi >> e & 1u)) s1[e] = 0xff800000u;
                     }
                 }
                 // three-input max (two new values per instruction), eight independent chains of four
@@ -565,10 +637,10 @@ bool plan_map(MapPlan& mp, size_t d, const size_t extent[3], const size_t stride
     return true;
 }
 
-template <int D>
+template <int D, bool MASKED>
 int launch_attn_tc(md_ctx* ctx, const AttnTcMaps& maps, const AttnTcParams& p, dim3 grid) {
-    auto kern = attn_tc_kernel<D>;
-    const uint32_t cfg_bit = 1u << (D == 64 ? 8 : 9);
+    auto kern = attn_tc_kernel<D, MASKED>;
+    const uint32_t cfg_bit = 1u << ((D == 64 ? 8 : 9) + (MASKED ? 8 : 0));
     if (!(ctx->tc_configured & cfg_bit)) {
         MD_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnCfg<D>::SMEM));
         ctx->tc_configured |= cfg_bit;
@@ -630,7 +702,7 @@ int md_launch_sdpa_tc(md_ctx* ctx, const __half* q, const __half* k, const __hal
     AttnTcParams p;
     p.q_len = (int)q_len; p.kv_len = (int)kv_len; p.causal_pos = causal_pos;
     p.scale_log2 = (1.0f / sqrtf((float)d)) * LOG2E_F;
-    p.mask = mask;
+    p.mask_words = nullptr; p.mask_span = nullptr; p.q_pad = 0;
     p.q_dim_row = mq.dim_of[0]; p.q_dim_head = mq.dim_of[1]; p.q_dim_batch = mq.dim_of[2];
     p.kv_dim_row = mk.dim_of[0]; p.kv_dim_head = mk.dim_of[1]; p.kv_dim_batch = mk.dim_of[2];
     p.o_dim_row = mo.dim_of[0]; p.o_dim_head = mo.dim_of[1]; p.o_dim_batch = mo.dim_of[2];
@@ -642,5 +714,20 @@ int md_launch_sdpa_tc(md_ctx* ctx, const __half* q, const __half* k, const __hal
     size_t ctas = n_items;
     if (ctx->attn_ctas_per_sm > 0) ctas = std::min(n_items, (size_t)ctx->attn_ctas_per_sm * (size_t)ctx->sm_count);
     dim3 grid((unsigned)ctas);
-    return d == 64 ? launch_attn_tc<64>(ctx, maps, p, grid) : launch_attn_tc<72>(ctx, maps, p, grid);
+    void* tmp = nullptr;
+    if (mask) {
+        const size_t n_tiles = (kv_len + ABKV - 1) / ABKV, q_pad = (size_t)p.n_qblk * ABQ;
+        const size_t word_bytes = n_tiles * q_pad * sizeof(unsigned long long);
+        MD_TRY(md_temp_alloc(ctx, word_bytes + (size_t)p.n_qblk * MASK_CHUNKS * sizeof(int2), &tmp));
+        unsigned long long* words = (unsigned long long*)tmp;
+        int2* span = reinterpret_cast<int2*>((char*)tmp + word_bytes);
+        p.mask_words = words; p.mask_span = span; p.q_pad = (int)q_pad;
+        const int st = md_launch_ex(ctx, mask_bits_kernel, dim3((unsigned)p.n_qblk, MASK_CHUNKS), dim3(1024), 0, "mask_bits_kernel", mask,
+                                    words, span, (int)q_len, (int)kv_len, (int)q_pad);
+        if (st != MD_OK) { md_temp_free(ctx, tmp); return st; }
+    }
+    if (!mask) return d == 64 ? launch_attn_tc<64, false>(ctx, maps, p, grid) : launch_attn_tc<72, false>(ctx, maps, p, grid);
+    const int st = d == 64 ? launch_attn_tc<64, true>(ctx, maps, p, grid) : launch_attn_tc<72, true>(ctx, maps, p, grid);
+    const int st_free = md_temp_free(ctx, tmp);
+    return st != MD_OK ? st : st_free;
 }

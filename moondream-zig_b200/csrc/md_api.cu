@@ -180,6 +180,25 @@ int md_scratch(md_ctx* ctx, size_t bytes, void** out) {
     return MD_OK;
 }
 
+int md_temp_alloc(md_ctx* ctx, size_t bytes, void** out) {
+    if (!ctx->pool) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = ctx->device;
+        MD_CUDA(ctx, cudaMemPoolCreate(&ctx->pool, &props));
+        uint64_t keep = MD_POOL_KEEP;
+        MD_CUDA(ctx, cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    }
+    MD_CUDA(ctx, cudaMallocFromPoolAsync(out, bytes ? bytes : 1, ctx->pool, ctx->stream));
+    return MD_OK;
+}
+
+int md_temp_free(md_ctx* ctx, void* p) {
+    MD_CUDA(ctx, cudaFreeAsync(p, ctx->stream));
+    return MD_OK;
+}
+
 // Partial tiles and tickets of a split-K GEMM for the stream the context is on.
 int md_splitk_workspace(md_ctx* ctx, size_t bytes, float** part, unsigned** tickets) {
     md_ctx::SplitK* ws = nullptr;
@@ -293,6 +312,7 @@ int md_destroy(md_ctx* ctx) {
         if (w.part) cudaFree(w.part);
         if (w.tickets) cudaFree(w.tickets);
     }
+    if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     if (ctx->counters) cudaFree(ctx->counters);
     if (ctx->rope_tab) cudaFree(ctx->rope_tab);
     if (ctx->flags) cudaFree(ctx->flags);

@@ -40,6 +40,7 @@ struct md_graph {
     cudaGraphExec_t exec = nullptr;
 };
 
+constexpr size_t MD_POOL_KEEP = (size_t)32 << 20;
 constexpr size_t MD_COUNTER_WORDS = 2048;
 constexpr size_t MD_SPLITK_TICKETS = 1024;   // tiles of a split-K GEMM (one arrival ticket each)
 
@@ -67,6 +68,7 @@ struct md_ctx {
     // scratch for kernels that need global memory beyond inputs and outputs
     void* scratch = nullptr;
     size_t scratch_cap = 0;
+    cudaMemPool_t pool = nullptr;   // md_temp_alloc; keeps at most MD_POOL_KEEP bytes between calls
     // per-head arrival counters of the split-KV decode attention (MD_COUNTER_WORDS words): zero between launches
     unsigned int* counters = nullptr;
     // cuTensorMapEncodeTiled resolved through the runtime (no link against libcuda)
@@ -157,6 +159,10 @@ __device__ __forceinline__ void md_pdl_wait() { asm volatile("griddepcontrol.wai
 int md_rope_cached(md_ctx* ctx, size_t rot_dim, float theta, size_t rows, const float** out);
 // Ensure ctx->scratch holds at least `bytes`.
 int md_scratch(md_ctx* ctx, size_t bytes, void** out);
+// Stream-ordered temporary memory for one call: its own for every call, whatever stream the context is on, and an allocation
+// node of the graph when one is being captured.
+int md_temp_alloc(md_ctx* ctx, size_t bytes, void** out);
+int md_temp_free(md_ctx* ctx, void* p);
 int md_splitk_workspace(md_ctx* ctx, size_t bytes, float** part, unsigned** tickets);
 
 // Host-or-device argument resolution for drop-in calls.

@@ -42,6 +42,26 @@ def test_arbitrary_mask(ctx, oracle, forced):
     assert_close_ref(ctx.sdpa_masked(q, k, v, m, 4, 150, 190, 64), oracle.sdpa_masked(q, k, v, m), "random mask")
 
 
+@pytest.mark.parametrize("h,lq,lk,lo,hi", [(2, 129, 65, 64, 65), (3, 65, 300, 70, 131), (2, 200, 640, 0, 64), (1, 256, 1000, 999, 1000),
+                                           (2, 384, 257, 100, 257)])
+def test_mask_whose_tiles_are_partly_unseen(ctx, oracle, forced, h, lq, lk, lo, hi):
+    """Rows see some of the keys lo..hi, one row in every 128 nothing (zeros), the second query block (where there is one)
+    a single key: tiles before, between and after are skipped by the tcgen05 kernel."""
+    rng = np.random.default_rng(lq + lk)
+    q, k, v = f16_normal(rng, (h, lq, 64)), f16_normal(rng, (h, lk, 64)), f16_normal(rng, (h, lk, 64))
+    m = np.zeros((lq, lk), np.uint8)
+    m[:, lo:hi] = rng.integers(0, 256, (lq, hi - lo)) * (rng.random((lq, hi - lo)) > 0.3)
+    m[:, hi - 1] = 7        # any byte but 0 means visible
+    m[128:256] = 0
+    m[128:256, lo] = 1
+    m[5::128] = 0
+    got = ctx.sdpa_masked(q, k, v, m, h, lq, lk, 64)
+    seen = m.any(1)
+    assert (got[:, ~seen] == 0).all()
+    ref = oracle.sdpa_masked(q, k, v, (m != 0).astype(np.uint8))
+    assert_close_ref(got[:, seen], ref[:, seen], "partly unseen")
+
+
 def test_large_scores_stay_finite(ctx, oracle, forced):
     """Scores far from zero: the running-max rescale must keep exp() in range in every tile."""
     rng = np.random.default_rng(5)
