@@ -327,97 +327,149 @@ struct FewShared {       // the shared expert's products; pad 0: none
     float limit;
 };
 
-// act[token][slot * ff_pad + j] = weight * gated(gate_j, up_j); the shared expert's columns follow those of all `slots`
-__global__ void __launch_bounds__(256)
+// The slots' products.  What bounds them is the weights' bytes, and what a stream needs is bytes in flight without gaps: the
+// kernels before these had a block per 16 rows that read its list entry, requested its rows, multiplied and ended, and so asked
+// for nothing during half of its life.  Here the blocks stay (two, or one of twice the size, per SM), and as soon as a piece (32
+// columns of 16 rows) is multiplied its registers take the request of the piece a round later, over the end of an item too.
+// The requests wait in registers and L1 and not in shared memory: with queues there (cp.async, or a ring filled by TMA, which
+// was slower) the GEMVs that follow find L1 shrunk to what the queue left, and lost what these kernels gained.
+// 8 tokens that use 10 or 11 of 16 experts of 2048 x 2368 (205 and 102 MB): 44 and 57 us before, 40 and 24 us now (5.1 and
+// 4.3 TB/s, the wait for the predecessor's result included).
+
+// act[token][slot * ff_pad + j] = weight * gated(gate_j, up_j); the shared expert's columns follow those of all `slots`.
+// An item is 8 gate rows and the 8 up rows beside them of one slot; warp w takes columns 32 w .. of every 256.  U pieces are in
+// flight per lane.  XREG (U = 8, width <= 2048): the tokens' columns of a warp are read once; else they travel with the weights.
+template <int U, bool XREG>
+__global__ void __launch_bounds__(256, 2)
 moe_up_kernel(const __nv_bfloat16* h, const __nv_bfloat16* __restrict__ w_gu, __nv_bfloat16* out, int T, int W, int ff_pad, int act,
               float limit, float alpha, int slots, FewShared sh, Route r) {
-    __shared__ float partial[8][16][8];
+    __shared__ float partial[2][8][16][8];
+    __shared__ int list[MAX_EXPERTS];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    const int slot = blockIdx.y, j = blockIdx.x * 8 + g;
-    md_pdl_launch_dependents();
+    // in this order: when the down products start, the list they read is complete
     md_pdl_wait();
-    // (the three small loads together; entries past n_slots are dropped right after)
-    const bool is_shared = slot == slots;
-    const float* weight = is_shared ? r.shared : r.weight + slot * 8;
-    const int n_slots = __ldcg(r.n_slots), expert = is_shared ? 0 : __ldcg(r.expert + slot);
-    const float mine = __ldcg(weight + g);
-    if (is_shared ? (int)blockIdx.x * 8 >= sh.pad : slot >= n_slots || (int)blockIdx.x * 8 >= ff_pad) return;
-    if (is_shared) limit = sh.limit;
-    const __nv_bfloat16* w = is_shared ? sh.gu : w_gu + (size_t)expert * 2 * ff_pad * W;
-    const __nv_bfloat16* w_lo = w + (size_t)((j / MD_GLU_BLOCK) * (2 * MD_GLU_BLOCK) + j % MD_GLU_BLOCK) * W + t * 8;
-    const __nv_bfloat16* w_hi = w_lo + (size_t)MD_GLU_BLOCK * W;
-    const bool has_x = g < T && mine != 0.f;
-    const __nv_bfloat16* x = h + (size_t)(has_x ? g : 0) * W + t * 8;
+    md_pdl_launch_dependents();
+    const int n_slots = __ldcg(r.n_slots);
+    for (int i = tid; i < slots; i += 256) list[i] = __ldcg(r.expert + i);
     const uint4 zero = make_uint4(0, 0, 0, 0);
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int k0 = warp * 32; k0 < W; k0 += 8 * 256) {
-        uint4 lo[8], hi[8], xv[8];
+    const int at = warp * 32 + t * 8, rounds = (W + U * 256 - 1) / (U * 256);
+    const __nv_bfloat16* x = h + (size_t)(g < T ? g : 0) * W + at;
+    uint4 lo[U], hi[U], xv[U];
+    if (XREG) {
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int k = k0 + u * 256;
-            const bool live = k + t * 8 < W;
-            lo[u] = live ? ldg_stream(w_lo + k) : zero;
-            hi[u] = live ? ldg_stream(w_hi + k) : zero;
-            xv[u] = live && has_x ? ld_act(x + k) : zero;
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) mma_piece(acc, lo[u], hi[u], xv[u]);
+        for (int u = 0; u < U; ++u) xv[u] = g < T && u * 256 + at < W ? ld_act(x + u * 256) : zero;
     }
-    partial[warp][g][2 * t] = acc[0];
-    partial[warp][g][2 * t + 1] = acc[1];
-    partial[warp][g + 8][2 * t] = acc[2];
-    partial[warp][g + 8][2 * t + 1] = acc[3];
     __syncthreads();
-    if (tid < 64) {
-        const int m = tid >> 3, e = tid & 7;
-        if (m < T) {
-            float a = 0.f, b = 0.f;
+    const int tiles = ff_pad / 8, own = n_slots * tiles, items = own + sh.pad / 8;
+    // the request side: item, round and this lane's gate row of the next request
+    int p_item = blockIdx.x, p_round = 0;
+    const __nv_bfloat16* p_w = nullptr;
+    auto locate = [&]() {
+        if (p_item >= items || p_round) return;
+        const int j = (p_item < own ? p_item % tiles : p_item - own) * 8 + g;
+        p_w = (p_item < own ? w_gu + (size_t)list[p_item / tiles] * 2 * ff_pad * W : sh.gu) +
+              (size_t)((j / MD_GLU_BLOCK) * (2 * MD_GLU_BLOCK) + j % MD_GLU_BLOCK) * W + at;
+    };
+    auto request = [&](int u) {
+        const int k = (p_round * U + u) * 256;
+        const bool live = p_item < items && k + at < W;
+        lo[u] = live ? ldg_stream(p_w + k) : zero;
+        hi[u] = live ? ldg_stream(p_w + (size_t)MD_GLU_BLOCK * W + k) : zero;
+        if (!XREG) xv[u] = live && g < T ? ld_act(x + k) : zero;
+    };
+    auto advance = [&]() {
+        if (++p_round == rounds) { p_round = 0; p_item += gridDim.x; }
+    };
+    locate();
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                a += partial[q][e][m];
-                b += partial[q][e + 8][m];
+    for (int u = 0; u < U; ++u) request(u);
+    advance();
+    int buf = 0;
+    for (int item = blockIdx.x; item < items; item += gridDim.x, buf ^= 1) {
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int round = 0; round < rounds; ++round) {
+            locate();
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                mma_piece(acc, lo[u], hi[u], xv[u]);
+                request(u);
             }
-            out[(size_t)m * (slots * ff_pad + sh.pad) + slot * ff_pad + blockIdx.x * 8 + e] =
-                __float2bfloat16_rn(__ldcg(weight + m) * md_gated(act, limit, alpha, a, b));
+            advance();
+        }
+        float (*mine)[16][8] = partial[buf];
+        mine[warp][g][2 * t] = acc[0];
+        mine[warp][g][2 * t + 1] = acc[1];
+        mine[warp][g + 8][2 * t] = acc[2];
+        mine[warp][g + 8][2 * t + 1] = acc[3];
+        __syncthreads();
+        if (tid < 64) {
+            const int m = tid >> 3, e = tid & 7;
+            if (m < T) {
+                const bool routed = item < own;
+                const int slot = routed ? item / tiles : slots, j = (routed ? item % tiles : item - own) * 8 + e;
+                const float weight = __ldcg(routed ? r.weight + slot * 8 + m : r.shared + m);
+                float a = 0.f, b = 0.f;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    a += mine[q][e][m];
+                    b += mine[q][e + 8][m];
+                }
+                // a token that does not use the expert contributes nothing, whatever the product holds
+                out[(size_t)m * (slots * ff_pad + sh.pad) + slot * ff_pad + j] =
+                    __float2bfloat16_rn(weight == 0.f ? 0.f : weight * md_gated(act, routed ? limit : sh.limit, alpha, a, b));
+            }
         }
     }
 }
 
-// y[token][n] = sum over the slots' columns
-__global__ void __launch_bounds__(512, 2)
+// y[token][n] = sum over the slots' columns.  A block owns R <= 16 rows (an equal share for every SM), its warps take the
+// 32-column pieces of all slots in turn.
+__global__ void __launch_bounds__(512, 1)
 moe_down_kernel(const __nv_bfloat16* act, const __nv_bfloat16* __restrict__ w_down, float* y, int T, int W, int ff_pad, int slots,
-                FewShared sh, Route r) {
+                int R, FewShared sh, Route r) {
+    constexpr int U = 6;
     __shared__ float partial[16][16][8];
     __shared__ int list[MAX_EXPERTS];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    const int row0 = blockIdx.x * 16, per = ff_pad / 32, act_stride = slots * ff_pad + sh.pad;
+    const int row0 = blockIdx.x * R, per = ff_pad / 32, act_stride = slots * ff_pad + sh.pad;
     md_pdl_launch_dependents();
-    md_pdl_wait();
+    // the list is older than the up products (which wait for it before they let this kernel start), so the first weights are
+    // requested ahead of the dependency wait
     const int n_slots = __ldcg(r.n_slots), routed = n_slots * per, chunks = routed + sh.pad / 32;
-    if (tid < slots) list[tid] = __ldcg(r.expert + tid);   // what is past n_slots is not used
+    for (int i = tid; i < slots; i += 512) list[i] = __ldcg(r.expert + i);
     __syncthreads();
-    const size_t r_lo = min(row0 + g, W - 1), r_hi = min(row0 + g + 8, W - 1);
+    const bool has_lo = g < R && row0 + g < W, has_hi = g + 8 < R && row0 + g + 8 < W;
+    const size_t r_lo = row0 + g, r_hi = row0 + g + 8;
     const __nv_bfloat16* x = act + (size_t)(g < T ? g : 0) * act_stride + t * 8;
     const uint4 zero = make_uint4(0, 0, 0, 0);
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    constexpr int U = 4;
-    for (int c0 = warp; c0 < chunks; c0 += U * 16) {
-        uint4 lo[U], hi[U], xv[U];
+    uint4 lo[U], hi[U], xv[U];
+    int p_c = warp, p_slot = p_c / per, p_at = p_c - p_slot * per;    // chunk of the next request, its slot and place there
+    auto weights = [&](int u) {
+        const bool own = p_c < routed, live = p_c < chunks;
+        const int pitch = own ? ff_pad : sh.pad;
+        const __nv_bfloat16* w = own ? w_down + (size_t)list[p_slot] * W * ff_pad + p_at * 32 : sh.down + (p_c - routed) * 32;
+        lo[u] = live && has_lo ? ldg_stream(w + r_lo * pitch + t * 8) : zero;
+        hi[u] = live && has_hi ? ldg_stream(w + r_hi * pitch + t * 8) : zero;
+        p_c += 16;
+        p_at += 16;
+        while (p_at >= per) { p_at -= per; ++p_slot; }
+    };
+    auto tokens = [&](int u, int c) {
+        xv[u] = c < chunks && g < T ? ld_act(x + (c < routed ? c * 32 : slots * ff_pad + (c - routed) * 32)) : zero;
+    };
+#pragma unroll
+    for (int u = 0; u < U; ++u) weights(u);
+    md_pdl_wait();
+#pragma unroll
+    for (int u = 0; u < U; ++u) tokens(u, warp + u * 16);
+    for (int c = warp; c < chunks; c += U * 16) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const int c = c0 + u * 16;
-            lo[u] = hi[u] = xv[u] = zero;
-            if (c < chunks) {
-                const bool own = c < routed;
-                const int slot = own ? c / per : 0, pitch = own ? ff_pad : sh.pad;
-                const __nv_bfloat16* w = own ? w_down + (size_t)list[slot] * W * ff_pad + (c - slot * per) * 32 : sh.down + (c - routed) * 32;
-                lo[u] = ldg_stream(w + r_lo * pitch + t * 8);
-                hi[u] = ldg_stream(w + r_hi * pitch + t * 8);
-                if (g < T) xv[u] = ld_act(x + (own ? c * 32 : slots * ff_pad + (c - routed) * 32));
-            }
+            mma_piece(acc, lo[u], hi[u], xv[u]);      // zeros past the end
+            weights(u);
+            tokens(u, c + (U + u) * 16);
         }
-#pragma unroll
-        for (int u = 0; u < U; ++u) mma_piece(acc, lo[u], hi[u], xv[u]);
     }
     partial[warp][g][2 * t] = acc[0];
     partial[warp][g][2 * t + 1] = acc[1];
@@ -426,7 +478,7 @@ moe_down_kernel(const __nv_bfloat16* act, const __nv_bfloat16* __restrict__ w_do
     __syncthreads();
     if (tid < 128) {
         const int m = tid >> 4, e = tid & 15;
-        if (m < T && row0 + e < W) {
+        if (m < T && e < R && row0 + e < W) {
             float v = 0.f;
 #pragma unroll
             for (int w = 0; w < 16; ++w) v += partial[w][e][m];
@@ -445,18 +497,20 @@ int launch_few(md_ctx* ctx, const md_moe& m, const void* h, size_t rows, const m
     r.score = r.shared + 8;
     r.weight = r.score + 8 * (size_t)EA;
     r.expert = reinterpret_cast<int*>(r.weight + 8 * (size_t)EA);
-    const FewShared sh = {reinterpret_cast<const __nv_bfloat16*>(m.shared_gu), reinterpret_cast<const __nv_bfloat16*>(m.shared_down),
-                          m.shared_pad, m.shared_limit};
     const __nv_bfloat16* x = reinterpret_cast<const __nv_bfloat16*>(h);
     __nv_bfloat16* act = reinterpret_cast<__nv_bfloat16*>(b.act);
     MD_TRY(md_launch_ex(ctx, moe_route_kernel, dim3((unsigned)((EA + 15) / 16)), dim3(512), 16 * (size_t)EA * sizeof(float), "moe_route_kernel",
                         x, reinterpret_cast<const __nv_bfloat16*>(m.router), T, m.width, E, EA - E, m.top, m.router_kind, r));
-    MD_TRY(md_launch_ex(ctx, moe_up_kernel, dim3((unsigned)((m.ff_pad > m.shared_pad ? m.ff_pad : m.shared_pad) / 8), (unsigned)(slots + EA - E)),
-                        dim3(256), 0, "moe_up_kernel", x,
-                        reinterpret_cast<const __nv_bfloat16*>(m.w_gu), act, T, m.width, m.ff_pad, m.act, m.limit, m.alpha,
-                        slots, sh, r));
-    return md_launch_ex(ctx, moe_down_kernel, dim3((unsigned)((m.width + 15) / 16)), dim3(512), 0, "moe_down_kernel", act,
-                        reinterpret_cast<const __nv_bfloat16*>(m.w_down), b.y_f32, T, m.width, m.ff_pad, slots, sh, r);
+    const FewShared sh = {reinterpret_cast<const __nv_bfloat16*>(m.shared_gu), reinterpret_cast<const __nv_bfloat16*>(m.shared_down),
+                          m.shared_pad, m.shared_limit};
+    auto up = m.width <= 2048 ? moe_up_kernel<8, true> : moe_up_kernel<4, false>;
+    const int items = (slots * m.ff_pad + m.shared_pad) / 8, most = 2 * ctx->sm_count;
+    MD_TRY(md_launch_ex(ctx, up, dim3((unsigned)(items < most ? items : most)), dim3(256), 0, "moe_up_kernel", x,
+                        reinterpret_cast<const __nv_bfloat16*>(m.w_gu), act, T, m.width, m.ff_pad, m.act, m.limit, m.alpha, slots, sh, r));
+    // as few rounds over the SMs as 16 rows per block allow, in equal shares
+    const int rounds = (m.width + 16 * ctx->sm_count - 1) / (16 * ctx->sm_count), R = (m.width + rounds * ctx->sm_count - 1) / (rounds * ctx->sm_count);
+    return md_launch_ex(ctx, moe_down_kernel, dim3((unsigned)((m.width + R - 1) / R)), dim3(512), 0, "moe_down_kernel", act,
+                        reinterpret_cast<const __nv_bfloat16*>(m.w_down), b.y_f32, T, m.width, m.ff_pad, slots, R, sh, r);
 }
 
 template <class T>

@@ -489,3 +489,13 @@ def test_generate_program(tmp_path):
     assert [ln.size for ln in lines] == [8, 8]
     for t, ln in zip(prompts, lines):
         greedy_ok(cfg, w, t, ln, "bfloat16")
+
+
+@pytest.mark.parametrize("width,ff", [(72, 8), (1984, 264), (2048, 40), (2056, 72), (2376, 96)])
+@pytest.mark.parametrize("n", [1, 3, 8])
+def test_experts_of_a_few_tokens(ctx, mods, width, ff, n):
+    """The decode products of a mixture of experts where their shares of rows and columns are cut: widths around the 2048
+    columns that stay in registers and the 16 rows per SM of one round, hardly any feed-forward columns."""
+    cfg = ku.config(width, 40, 1, [ku.attention(2, 1, 16, 20, 0, ku.moe(9, 2, ff))])
+    w = ref.random_weights(cfg, width + n)
+    compare(ctx, mods, cfg, w, ku.tokens(cfg, n, n), "bfloat16", what=f"width {width}, {n} tokens")
