@@ -8,6 +8,9 @@
 //   stack_glue_any_kernel    widths that are not a multiple of 4 or too wide for the others
 //   stack_parallel_kernel    the same place in a layer whose two sublayers read the same row (md_parallel_glue): both layer
 //                            scales and sums, one norm, two weighted outputs
+#include <algorithm>
+#include <type_traits>
+
 #include "stack.cuh"
 
 namespace {
@@ -302,89 +305,163 @@ stack_glue_step_kernel(const __grid_constant__ md_glue p) {
 }
 
 constexpr int ROWS_THREADS = 512;
+enum { Y_ROWS, Y_F32, Y_ROUTED };     // the sublayer's output: T rows (or none at all), f32 rows, expert-sorted T rows
 
-// GW warps per row, NV vectors of 4 columns per lane: width <= 128 * GW * NV.  Sixteen warps; blocks, halo rows and state as
-// in stack_glue_any_kernel.
-template <class T, int GW, int NV>
-__global__ void __launch_bounds__(ROWS_THREADS, NV <= 4 ? 2 : 1)
+// Rows of a prompt: GW warps per row, NV vectors of 4 columns per lane, width <= 128 * GW * NV; one block per SM with R rows of its
+// own behind the taps - 1 rows ahead of them, which it computes again (those before the prompt are the state's).
+// What bounded the form before this one were the weights: every row read w_post, w_pre and all taps from L2, 48 KB at a width of
+// 2048 for 20 KB of rows.  Here a lane works on the same columns in every row, so the norms' weights stay in registers
+// (NV <= 4); a group's next row is requested before the two sums over the current one; and the convolution runs down the block's
+// rows with a thread's taps and last rows in registers, reading n once from shared memory.
+// 2048 wide, 4 taps, bf16, before -> after: 2048 rows 32 -> 17 us, 231 rows 15 -> 6.5 us.
+template <class T, int GW, int NV, int Y>
+__global__ void __launch_bounds__(ROWS_THREADS, 1)
 stack_glue_rows_kernel(const __grid_constant__ md_glue p, int R) {
-    extern __shared__ __align__(16) float xs[];   // [R + halo][width]
+    extern __shared__ __align__(16) float xs[];   // [R + halo][width]: n of rows t0 - halo ..
     __shared__ float red[2][ROWS_THREADS / 32];
-    constexpr int GROUPS = ROWS_THREADS / 32 / GW;
-    const int W = p.width, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    constexpr int GROUPS = ROWS_THREADS / 32 / GW, MAX_TAPS = 4;
+    constexpr int CHOICES = Y == Y_ROUTED ? 2 : 1;    // experts of a row that are requested ahead; more are read where they are used
+    constexpr bool KEEP = NV <= 4;
+    const int W = p.width, per = W / 4, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int grp = warp / GW, gl = (warp % GW) * 32 + lane;    // this thread's place within its row
-    const int t0 = blockIdx.x * R, own = min(R, p.rows - t0), halo = p.conv ? p.taps - 1 : 0;
-    const bool first = blockIdx.x == 0;
+    const int t0 = blockIdx.x * R, end = min(t0 + R, p.rows), halo = p.conv ? p.taps - 1 : 0, begin = max(t0 - halo, 0);
     md_pdl_launch_dependents();
-    // the weights come from HBM once per pass over the model: on their way to L2 before the wait
-    for (int i = tid * 32; i < W; i += ROWS_THREADS * 32) {
-        prefetch_l2(p.w_pre + i);
-        if (p.w_post) prefetch_l2(p.w_post + i);
-        for (int j = 0; p.conv && j < p.taps; ++j) prefetch_l2(p.conv + (size_t)j * W + i);
-    }
-    md_pdl_wait();
-    auto total = [&](float v, int turn) {
-        v = warp_sum(v);
-        if (GW > 1) {
-            if (lane == 0) red[turn][warp] = v;
-            __syncthreads();
-            v = 0.f;
+    auto vec = [&](int n) { return gl + n * 32 * GW; };         // this thread's n-th vector of a row
+    Vec<4> w_pre[KEEP ? NV : 1], w_post[KEEP ? NV : 1];
+    if (KEEP) {
 #pragma unroll
-            for (int i = 0; i < GW; ++i) v += red[turn][grp * GW + i];
+        for (int n = 0; n < (KEEP ? NV : 1); ++n) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) w_pre[n].f[i] = w_post[n].f[i] = 0.f;
+            if (vec(n) >= per) continue;
+            w_pre[n] = ldv<float, 4>(p.w_pre + vec(n) * 4);
+            if (p.w_post) w_post[n] = ldv<float, 4>(p.w_post + vec(n) * 4);
+        }
+    }
+    // the taps come from HBM once per pass over the model: on their way to L2 before the wait
+    for (int i = tid * 32; i < W; i += ROWS_THREADS * 32)
+        for (int j = 0; p.conv && j < p.taps; ++j) prefetch_l2(p.conv + (size_t)j * W + i);
+    md_pdl_wait();
+
+    // 4 columns as they lie in memory: nothing is done with them before the row's turn, so that the request stays in flight
+    using Raw = typename std::conditional<sizeof(T) == 4 || Y == Y_F32, uint4, uint2>::type;
+    auto value = [](const auto& u) {
+        Vec<4> v;
+        if constexpr (sizeof(u) == 16) {
+            v.f[0] = __uint_as_float(u.x); v.f[1] = __uint_as_float(u.y); v.f[2] = __uint_as_float(u.z); v.f[3] = __uint_as_float(u.w);
+        } else {
+            v.f[0] = __uint_as_float(u.x << 16); v.f[1] = __uint_as_float(u.x & 0xffff0000u);
+            v.f[2] = __uint_as_float(u.y << 16); v.f[3] = __uint_as_float(u.y & 0xffff0000u);
         }
         return v;
     };
-    const int slot = halo ? *p.state_slot[0] : 0;
-    float* state = halo ? p.state[0] : nullptr;
-    if (first && halo)
-        for (int i = tid; i < halo * W; i += ROWS_THREADS) xs[i] = state[slot * halo * W + i];
-    const int lo = first ? halo : 0, hi = halo + own;      // xs[l] = n[t0 - halo + l]
-    for (int l0 = lo; l0 < hi; l0 += GROUPS) {
-        const int l = l0 + grp, t = t0 - halo + l;
-        const bool live = l < hi;
-        Vec<4> x[NV], y[NV];
+    const Raw* yb = reinterpret_cast<const Raw*>(Y == Y_F32 || (sizeof(T) == 4 && p.y_f32) ? (const void*)p.y_f32 : p.y);
+    uint4 rx[NV];
+    Raw ry[NV][CHOICES];
+#pragma unroll
+    for (int n = 0; n < NV; ++n) {
+        rx[n] = make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int k = 0; k < CHOICES; ++k) ry[n][k] = Raw();
+    }
+    [[maybe_unused]] float parts = 0.f, score[CHOICES], score_next[CHOICES];
+    [[maybe_unused]] int slot_next[CHOICES];
+    auto source = [&](int t) { return p.gather ? (size_t)p.gather[t] : (size_t)t; };
+    auto choices = [&](int t) {      // of row t, ahead of request(t)
+        if (Y != Y_ROUTED || t >= end) return;
+        const size_t at = source(t) * p.top;
+#pragma unroll
+        for (int k = 0; k < CHOICES; ++k) {
+            slot_next[k] = k < p.top ? __ldcg(p.slot + at + k) : 0;
+            score_next[k] = k < p.top ? __ldcg(p.score + at + k) : 0.f;
+        }
+    };
+    auto request = [&](int t) {
+        if (t >= end) return;
+        const size_t src = source(t);
+        const T* xe = nullptr;
+        if (p.tokens) {
+            const unsigned long long tok = p.tokens[src];
+            xe = reinterpret_cast<const T*>(p.embed) + (size_t)(tok < (unsigned long long)p.vocab ? tok : 0ull) * W;
+        }
 #pragma unroll
         for (int n = 0; n < NV; ++n) {
+            const int c = vec(n);
+            if (c >= per) continue;
+            if (!xe || sizeof(T) == 4) {
+                rx[n] = __ldcg(reinterpret_cast<const uint4*>(xe ? reinterpret_cast<const float*>(xe) : p.x + src * W) + c);
+            } else {
+                const uint2 u = __ldcg(reinterpret_cast<const uint2*>(xe) + c);     // the first layer
+                rx[n] = make_uint4(u.x << 16, u.x & 0xffff0000u, u.y << 16, u.y & 0xffff0000u);
+            }
+            if (!p.w_post) continue;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) x[n].f[i] = y[n].f[i] = 0.f;
+            for (int k = 0; k < CHOICES; ++k)
+                if (Y != Y_ROUTED || k < p.top) ry[n][k] = __ldcg(yb + (Y == Y_ROUTED ? (size_t)slot_next[k] : src) * per + c);
         }
-        const size_t src = live ? (p.gather ? (size_t)p.gather[t] : t) : 0;
+        if (p.w_post && p.ssq) {     // one value per lane waits for its turn as it is; more parts than lanes are added here
+            parts = lane < p.ssq_parts ? __ldcg(p.ssq + src * p.ssq_parts + lane) : 0.f;
+            for (int i = lane + 32; i < p.ssq_parts; i += 32) parts += __ldcg(p.ssq + src * p.ssq_parts + i);
+        }
+#pragma unroll
+        for (int k = 0; k < CHOICES; ++k) score[k] = score_next[k];
+        choices(t + GROUPS);
+    };
+    int turn = 0;
+    auto total = [&](float v) {      // over the row's warps; the two halves of `red` alternate
+        v = warp_sum(v);
+        if (GW > 1) {
+            if (lane == 0) red[turn][warp] = v;
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(GW * 32) : "memory");
+            v = 0.f;
+#pragma unroll
+            for (int i = 0; i < GW; ++i) v += red[turn][grp * GW + i];
+            turn ^= 1;
+        }
+        return v;
+    };
+    choices(begin + grp);
+    request(begin + grp);
+    const int slot = halo ? *p.state_slot[0] : 0;
+    float* state = halo ? p.state[0] : nullptr;
+    if (t0 < halo)      // rows ahead of the prompt
+        for (int i = tid; i < (halo - t0) * W; i += ROWS_THREADS) xs[i] = state[(size_t)(slot * halo + t0) * W + i];
+    for (int t = begin + grp; t < end; t += GROUPS) {
+        Vec<4> x[NV], y[NV];
         float scale = 1.f;
-        if (live) {
-            if (p.w_post && !p.slot) {
-                const T* yr = reinterpret_cast<const T*>(p.y) + src * W;
+        if (p.w_post && p.ssq) scale = 1.f / sqrtf(warp_sum(parts) / (float)p.ssq_n + p.eps);
+#pragma unroll
+        for (int n = 0; n < NV; ++n) {
+            x[n] = value(rx[n]);
+            if constexpr (Y != Y_ROUTED) {
+                y[n] = value(ry[n][0]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) y[n].f[i] = 0.f;
+#pragma unroll
+                for (int k = 0; k < CHOICES; ++k) {
+                    if (k >= p.top) break;
+                    const Vec<4> e = value(ry[n][k]);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) y[n].f[i] = fmaf(score[k], e.f[i], y[n].f[i]);
+                }
+            }
+        }
+        if constexpr (Y == Y_ROUTED) {
+            for (int k = CHOICES; k < p.top; ++k) {
+                const size_t at = source(t) * p.top + k;
+                const float s = __ldcg(p.score + at);
+                const Raw* row = yb + (size_t)__ldcg(p.slot + at) * per;
 #pragma unroll
                 for (int n = 0; n < NV; ++n) {
-                    const int c = (gl + n * 32 * GW) * 4;
-                    if (c < W) y[n] = p.y_f32 ? ldv<float, 4>(p.y_f32 + src * W + c) : ldv<T, 4>(yr + c);
+                    if (vec(n) >= per) continue;
+                    const Vec<4> e = value(__ldcg(row + vec(n)));
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) y[n].f[i] = fmaf(s, e.f[i], y[n].f[i]);
                 }
             }
-            const T* xe = p.tokens ? reinterpret_cast<const T*>(p.embed) +
-                                         (size_t)(p.tokens[src] < (unsigned long long)p.vocab ? p.tokens[src] : 0ull) * W : nullptr;
-#pragma unroll
-            for (int n = 0; n < NV; ++n) {
-                const int c = (gl + n * 32 * GW) * 4;
-                if (c < W) x[n] = xe ? ldv<T, 4>(xe + c) : ldv<float, 4>(p.x + src * W + c);
-            }
-            if (p.w_post && p.ssq) {
-                float s = 0.f;
-                for (int i = lane; i < p.ssq_parts; i += 32) s += p.ssq[src * p.ssq_parts + i];
-                scale = 1.f / sqrtf(warp_sum(s) / (float)p.ssq_n + p.eps);
-            }
-            if (p.w_post && p.slot)
-                for (int k = 0; k < p.top; ++k) {
-                    const float s = p.score[src * p.top + k];
-                    const T* e = reinterpret_cast<const T*>(p.y) + (size_t)p.slot[src * p.top + k] * W;
-#pragma unroll
-                    for (int n = 0; n < NV; ++n) {
-                        const int c = (gl + n * 32 * GW) * 4;
-                        if (c >= W) continue;
-                        const Vec<4> v = ldv<T, 4>(e + c);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) y[n].f[i] = fmaf(s, v.f[i], y[n].f[i]);
-                    }
-                }
         }
+        request(t + GROUPS);
         if (p.w_post) {
             float ss = 0.f;
 #pragma unroll
@@ -395,46 +472,72 @@ stack_glue_rows_kernel(const __grid_constant__ md_glue p, int R) {
                     ss = fmaf(y[n].f[i], y[n].f[i], ss);
                 }
             }
-            const float inv = p.mult / sqrtf(total(ss, 0) / (float)W + p.eps);
+            const float inv = p.mult / sqrtf(total(ss) / (float)W + p.eps);
 #pragma unroll
             for (int n = 0; n < NV; ++n) {
-                const int c = (gl + n * 32 * GW) * 4;
-                if (c >= W) continue;
-                const Vec<4> w = ldv<float, 4>(p.w_post + c);
+                if (vec(n) >= per) continue;
+                const Vec<4> w = KEEP ? w_post[KEEP ? n : 0] : ldv<float, 4>(p.w_post + vec(n) * 4);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) x[n].f[i] = fmaf(y[n].f[i] * inv, w.f[i], x[n].f[i]);
             }
         }
         float ss = 0.f;
-        const bool store = live && l >= halo && p.x_out;
 #pragma unroll
         for (int n = 0; n < NV; ++n) {
-            const int c = (gl + n * 32 * GW) * 4;
 #pragma unroll
             for (int i = 0; i < 4; ++i) ss = fmaf(x[n].f[i], x[n].f[i], ss);
-            if (store && c < W) stv<float, 4>(p.x_out + (size_t)t * W + c, x[n]);
+            if (p.x_out && t >= t0 && vec(n) < per) stv<float, 4>(p.x_out + (size_t)t * W + vec(n) * 4, x[n]);
         }
-        const float inv2 = 1.f / sqrtf(total(ss, 1) / (float)W + p.eps);
+        const float inv2 = 1.f / sqrtf(total(ss) / (float)W + p.eps);
 #pragma unroll
         for (int n = 0; n < NV; ++n) {
-            const int c = (gl + n * 32 * GW) * 4;
-            if (!live || c >= W) continue;
-            const Vec<4> w = ldv<float, 4>(p.w_pre + c);
+            if (vec(n) >= per) continue;
+            const Vec<4> w = KEEP ? w_pre[KEEP ? n : 0] : ldv<float, 4>(p.w_pre + vec(n) * 4);
             Vec<4> v;
 #pragma unroll
             for (int i = 0; i < 4; ++i) v.f[i] = x[n].f[i] * (inv2 * w.f[i]);
-            stv<float, 4>(xs + (size_t)l * W + c, v);
+            if (p.conv) stv<float, 4>(xs + (size_t)(t - t0 + halo) * W + vec(n) * 4, v);
+            else stv<T, 4>(reinterpret_cast<T*>(p.out) + (size_t)t * W + vec(n) * 4, v);
         }
-        if (GW > 1) __syncthreads();    // `red` is free for the next rows
     }
+    if (!p.conv) return;
     __syncthreads();
     T* out = reinterpret_cast<T*>(p.out) + (size_t)t0 * W;
-    const int per = W / 4;
-    for (int i = tid; i < own * per; i += ROWS_THREADS) {
-        const int r = i / per, c = (i - r * per) * 4;
-        Vec<4> v = lds<4>(xs + (size_t)(r + halo) * W + c);
-        if (p.conv) {
-            Vec<4> s;
+    const int own = end - t0;
+    if (p.taps <= MAX_TAPS) {
+        // a thread takes 4 columns and an equal share of the rows
+        const int shares = per < ROWS_THREADS ? ROWS_THREADS / per : 1, share = per < ROWS_THREADS ? tid / per : 0;
+        const int first = own * share / shares, last = share < shares ? own * (share + 1) / shares : first;
+        for (int c = per < ROWS_THREADS ? tid - share * per : tid; c < per && first < last; c += ROWS_THREADS) {
+            Vec<4> w[MAX_TAPS], win[MAX_TAPS];      // the tap and n, so many rows back
+#pragma unroll
+            for (int d = 0; d < MAX_TAPS; ++d)
+                if (d <= halo) w[d] = ldv<float, 4>(p.conv + (size_t)(halo - d) * W + c * 4);
+#pragma unroll
+            for (int d = 1; d < MAX_TAPS; ++d)
+                if (d <= halo) win[d] = lds<4>(xs + (size_t)(first + halo - d) * W + c * 4);
+            for (int r = first; r < last; ++r) {
+                win[0] = lds<4>(xs + (size_t)(r + halo) * W + c * 4);
+                Vec<4> s, v;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) s.f[i] = 0.f;
+#pragma unroll
+                for (int d = MAX_TAPS - 1; d >= 0; --d) {
+                    if (d > halo) continue;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) s.f[i] = fmaf(w[d].f[i], win[d].f[i], s.f[i]);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v.f[i] = win[0].f[i] + s.f[i];
+                stv<T, 4>(out + (size_t)r * W + c * 4, v);
+#pragma unroll
+                for (int d = MAX_TAPS - 1; d > 0; --d) win[d] = win[d - 1];
+            }
+        }
+    } else {
+        for (int i = tid; i < own * per; i += ROWS_THREADS) {
+            const int r = i / per, c = (i - r * per) * 4;
+            Vec<4> v = lds<4>(xs + (size_t)(r + halo) * W + c), s;
 #pragma unroll
             for (int e = 0; e < 4; ++e) s.f[e] = 0.f;
 #pragma unroll 4
@@ -445,12 +548,17 @@ stack_glue_rows_kernel(const __grid_constant__ md_glue p, int R) {
             }
 #pragma unroll
             for (int e = 0; e < 4; ++e) v.f[e] += s.f[e];
+            stv<T, 4>(out + (size_t)r * W + c, v);
         }
-        stv<T, 4>(out + (size_t)r * W + c, v);
     }
-    if (blockIdx.x + 1 < gridDim.x || !halo) return;
+    if (end < p.rows || !halo) return;
     float* dst = state + (size_t)(p.rows == 1 ? slot : slot ^ 1) * halo * W;
     for (int i = tid; i < halo * W; i += ROWS_THREADS) dst[i] = xs[(size_t)own * W + i];
+}
+
+template <class T, int GW, int NV> void (*rows_kernel(int y))(md_glue, int) {
+    return y == Y_ROUTED ? stack_glue_rows_kernel<T, GW, NV, Y_ROUTED> : y == Y_F32 ? stack_glue_rows_kernel<T, GW, NV, Y_F32>
+                                                                                    : stack_glue_rows_kernel<T, GW, NV, Y_ROWS>;
 }
 
 // rows of f32 logits -> index of the largest (the lowest index of equal ones)
@@ -508,6 +616,21 @@ int launch_glue(md_ctx* ctx, const md_glue& g) {
         return md_launch_ex(ctx, stack_glue_step_kernel<T, 4, 4>, grid, dim3(STEP_THREADS), 0, "stack_glue_step_kernel", g);
     }
     const bool wide = g.rows == 1 || (g.gather && g.rows <= 8);
+    if (v4 && !wide && g.width <= 16384) {
+        // equal shares for the SMs, as far as their rows fit shared memory (any share works; rows ahead of it are computed again)
+        int R = (g.rows + ctx->sm_count - 1) / ctx->sm_count;
+        const int fit = (int)(220 * 1024 / row_bytes) - halo;
+        if (g.conv && R > fit) R = fit;
+        if (fit < std::max(halo, 1)) return md_fail(ctx, MD_ERR_UNSUPPORTED, "a width of %d with %d taps exceeds shared memory", g.width, g.taps);
+        if (g.x && g.x == g.x_out && g.rows > R) return md_fail(ctx, MD_ERR_INVALID_ARG, "md_glue: in-place residual over several blocks");
+        const int y = g.w_post && g.slot ? Y_ROUTED : g.w_post && g.y_f32 && sizeof(T) != 4 ? Y_F32 : Y_ROWS;
+        void (*kern)(md_glue, int) = g.width <= 512 ? rows_kernel<T, 1, 4>(y) : g.width <= 1024 ? rows_kernel<T, 2, 4>(y)
+                                   : g.width <= 2048 ? rows_kernel<T, 4, 4>(y) : g.width <= 4096 ? rows_kernel<T, 8, 4>(y)
+                                   : g.width <= 8192 ? rows_kernel<T, 16, 4>(y) : rows_kernel<T, 16, 8>(y);
+        const size_t smem = g.conv ? (R + halo) * row_bytes : 0;
+        if (smem > 47 * 1024) MD_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+        return md_launch_ex(ctx, kern, dim3((unsigned)((g.rows + R - 1) / R)), dim3(ROWS_THREADS), smem, "stack_glue_rows_kernel", g, R);
+    }
     int R = wide ? 1 : 8 - halo;
     if (!wide && R < halo) R = halo;
     if (R < 1) R = 1;
@@ -515,18 +638,10 @@ int launch_glue(md_ctx* ctx, const md_glue& g) {
     const size_t smem = (R + halo) * row_bytes;
     if (smem > 220 * 1024) return md_fail(ctx, MD_ERR_UNSUPPORTED, "a width of %d with %d taps exceeds shared memory", g.width, g.taps);
     if (g.x && g.x == g.x_out && g.rows > R) return md_fail(ctx, MD_ERR_INVALID_ARG, "md_glue: in-place residual over several blocks");
-    void (*kern)(md_glue, int) = nullptr;
-    const bool rows_form = v4 && !wide && g.width <= 16384;
-    const unsigned threads = wide ? 512 : rows_form ? ROWS_THREADS : 256;
-    if (rows_form)
-        kern = g.width <= 512 ? stack_glue_rows_kernel<T, 1, 4> : g.width <= 1024 ? stack_glue_rows_kernel<T, 2, 4>
-             : g.width <= 2048 ? stack_glue_rows_kernel<T, 4, 4> : g.width <= 4096 ? stack_glue_rows_kernel<T, 8, 4>
-             : g.width <= 8192 ? stack_glue_rows_kernel<T, 16, 4> : stack_glue_rows_kernel<T, 16, 8>;
-    else
-        kern = wide ? (v4 ? stack_glue_any_kernel<T, 4, true> : stack_glue_any_kernel<T, 1, true>)
-                    : (v4 ? stack_glue_any_kernel<T, 4, false> : stack_glue_any_kernel<T, 1, false>);
+    void (*kern)(md_glue, int) = wide ? (v4 ? stack_glue_any_kernel<T, 4, true> : stack_glue_any_kernel<T, 1, true>)
+                                      : (v4 ? stack_glue_any_kernel<T, 4, false> : stack_glue_any_kernel<T, 1, false>);
     if (smem > 47 * 1024) MD_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    return md_launch_ex(ctx, kern, dim3((unsigned)((g.rows + R - 1) / R), (unsigned)g.seqs), dim3(threads), smem,
+    return md_launch_ex(ctx, kern, dim3((unsigned)((g.rows + R - 1) / R), (unsigned)g.seqs), dim3(wide ? 512 : 256), smem,
                         "stack_glue_kernel", g, R);
 }
 

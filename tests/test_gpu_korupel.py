@@ -103,6 +103,21 @@ def test_convolution_and_norms(ctx, mods, taps):
         compare(ctx, mods, cfg, w, ku.tokens(cfg, 45), "float32", cuts, f"{taps} taps, cuts {cuts}")
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("width,taps,rows", [(1100, 4, 700), (2048, 2, 593), (2052, 3, 300), (520, 4, 1190)])
+def test_residual_rows_that_share_a_block(ctx, mods, width, taps, rows, dtype):
+    """More rows than blocks fit on the machine at once (two or three rows to a block, the last one short), portions that start in
+    the middle, routed rows of one expert and of three; one to eight warps per row.
+
+    The mixers' outputs have 96 values or more: with 8, a token's values can nearly cancel, and the norm over them multiplies the
+    rounding of float32 (with one head of 8, row 574 of the first shape was 5.8e-5 to 7.5e-5 from the reference, by the order of
+    the sums alone, the median row 1.6e-6)."""
+    cfg = ku.config(width, 48, taps, [ku.lightning(4, 16, 24, ku.moe(4, 3, 96)), ku.lightning(3, 32, 32, ku.moe(3, 1, 96)),
+                                      ku.lightning(4, 24, 32, ku.dense(160))])
+    w = ref.random_weights(cfg, 9)
+    compare(ctx, mods, cfg, w, ku.tokens(cfg, rows), dtype, (rows - 5, rows - 3))
+
+
 def test_residual_stream_after_every_layer(ctx, mods):
     cfg, w = ku.make("odd")
     toks = ku.tokens(cfg, 21)
