@@ -355,20 +355,18 @@ __device__ __forceinline__ float rope_rotate(const float* x, int dd, int rot_dim
 
 // CLUSTER: the splits of one head form a thread-block cluster (16 CTAs along x); the partial results are
 // merged through distributed shared memory of the cluster's first CTA instead of global scratch, fences
-// and an atomic ticket.
-template <bool CLUSTER>
-__global__ void __launch_bounds__(DEC_WARPS * 32)
-sdpa_decode_kernel(const __grid_constant__ DecodeParams gp) {
+// and an atomic ticket.  A split is WARPS * 32 keys.
+template <bool CLUSTER, int WARPS>
+__device__ __forceinline__ void decode_split(const DecodeParams& gp, int split, int head, int b) {
+    constexpr int KEYS = WARPS * 32;
     // the per-request tables are indexed in the constant bank; the working copy below is only accessed by field
     DecodeParams p = gp;
     __shared__ float cpart[CLUSTER ? 16 : 1][DEC_D + 2];
     __shared__ float q_s[DEC_D], knew_s[DEC_D], vnew_s[DEC_D], raw_s[DEC_D], rawk_s[DEC_D];
-    __shared__ float red_m[DEC_WARPS], red_l[DEC_WARPS], red_o[DEC_WARPS][DEC_D];
+    __shared__ float red_m[WARPS], red_l[WARPS], red_o[WARPS][DEC_D];
     __shared__ int is_last;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int head = blockIdx.y, split = blockIdx.x;
     if (p.batch > 0) {
-        const int b = blockIdx.z;
         p.q += b * p.q_batch_stride;
         p.out += b * p.out_batch_stride;
         p.k = p.k_w = gp.bk[b];
@@ -382,7 +380,7 @@ sdpa_decode_kernel(const __grid_constant__ DecodeParams gp) {
         // context, CTAs beyond the splits this position needs leave at once.
         p.pos = *p.pos_ptr;
         p.kv_cache_len = p.pos;
-        p.splits = max(1, (p.pos + DEC_KEYS - 1) / DEC_KEYS);
+        p.splits = max(1, (p.pos + KEYS - 1) / KEYS);
         if (split >= p.splits) {
             if (CLUSTER) cluster_sync_all();  // the merging CTA waits for every CTA of the cluster
             return;
@@ -397,8 +395,8 @@ sdpa_decode_kernel(const __grid_constant__ DecodeParams gp) {
     asm volatile("griddepcontrol.launch_dependents;");
     const __half* kh = p.k + head * p.k_head_stride;
     const __half* vh = p.v + head * p.k_head_stride;
-    const int key_lo = split * DEC_KEYS + warp * (DEC_KEYS / DEC_WARPS);
-    constexpr int ITER = DEC_KEYS / DEC_WARPS / 4;  // 8 keys per lane group
+    const int key_lo = split * KEYS + warp * 32;
+    constexpr int ITER = 8;  // keys per lane group
 
     uint4 kreg[ITER], vreg[ITER];
     bool valid[ITER];
@@ -525,10 +523,10 @@ sdpa_decode_kernel(const __grid_constant__ DecodeParams gp) {
     float M = -INFINITY, L = 0.f, O = 0.f;
     if (tid < DEC_D) {
 #pragma unroll
-        for (int w = 0; w < DEC_WARPS; ++w) M = fmaxf(M, red_m[w]);
+        for (int w = 0; w < WARPS; ++w) M = fmaxf(M, red_m[w]);
         const float Mu = (M == -INFINITY) ? 0.f : M;
 #pragma unroll
-        for (int w = 0; w < DEC_WARPS; ++w) {
+        for (int w = 0; w < WARPS; ++w) {
             const float f = (red_m[w] == -INFINITY) ? 0.f : expf(red_m[w] - Mu);
             L += red_l[w] * f;
             O += red_o[w][tid] * f;
@@ -616,6 +614,12 @@ sdpa_decode_kernel(const __grid_constant__ DecodeParams gp) {
     if (tid == 0) p.counters[head] = 0;  // ready for the next launch
 }
 
+template <bool CLUSTER>
+__global__ void __launch_bounds__(DEC_WARPS * 32)
+sdpa_decode_kernel(const __grid_constant__ DecodeParams p) {
+    decode_split<CLUSTER, DEC_WARPS>(p, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
 // The same decode attention for a batched step with enough (head, request) pairs to fill the machine by themselves
 // (8 requests x 32 heads = 256 CTAs): ONE CTA per pair walks all of its keys, so nothing is merged across CTAs: no
 // partials in global memory, no fence, no ticket, no last-arriver round.  8 warps; a lane group of 8 lanes x 16 B
@@ -626,12 +630,10 @@ sdpa_decode_kernel(const __grid_constant__ DecodeParams gp) {
 // append to the cache, position from device memory).
 constexpr int LOOP_WARPS = 8, LOOP_ITER = 4, LOOP_KEYS = LOOP_WARPS * 4 * LOOP_ITER;   // 128 keys per turn
 
-__global__ void __launch_bounds__(LOOP_WARPS * 32, 2)
-sdpa_decode_loop_kernel(const __grid_constant__ DecodeParams gp) {
+__device__ __forceinline__ void decode_loop(const DecodeParams& gp, int head, int b) {
     __shared__ float q_s[DEC_D], knew_s[DEC_D], vnew_s[DEC_D], raw_s[DEC_D], rawk_s[DEC_D];
     __shared__ float red_m[LOOP_WARPS * 4], red_l[LOOP_WARPS * 4], red_o[LOOP_WARPS * 4][DEC_D];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int head = blockIdx.x, b = blockIdx.y;
     const bool batched = gp.batch > 0;    // one request: cache and position in the scalar fields
     const __half* qrow = gp.q + (batched ? b * gp.q_batch_stride : 0);
     __half* out = gp.out + (batched ? b * gp.out_batch_stride : 0);
@@ -774,6 +776,153 @@ sdpa_decode_loop_kernel(const __grid_constant__ DecodeParams gp) {
             O += red_o[w][tid] * f;
         }
         out[head * DEC_D + tid] = __float2half_rn(L > 0.f ? O / L : 0.f);
+    }
+}
+
+__global__ void __launch_bounds__(LOOP_WARPS * 32, 2)
+sdpa_decode_loop_kernel(const __grid_constant__ DecodeParams p) {
+    decode_loop(p, blockIdx.x, blockIdx.y);
+}
+
+// One launch for the two things a decode layer does between its first and its last product: the attention over the caches, and
+// fc2, in four parts of its K sum (f32 sums that the last product's epilogue adds).  The attention is a chain of round trips that
+// moves little, fc2 a stream of 33.5 MB, so each fills what the other leaves; and as ONE kernel between two others of the same
+// stream it lets the last product start under it (programmatic dependent launch needs a single predecessor), with all of its
+// weights requested when the attention ends.  The attention's CTAs come first in the grid.
+// One request, 761 keys, behind the products before it: attention alone 4.8 us, fc2 alone 10.2 us, both 10 us.
+// A layer of 101 MB: five to seven kernels in two chains 26.5 us, three in one chain 25.6.
+struct MixParams {
+    DecodeParams a;
+    int attn_ctas, split_ctas;        // split_ctas: CTAs per (head, request), 0: one that walks all keys
+    const __half *x, *w;              // [M][K], [N][K]
+    float* part;                      // [parts][8 * N]
+    int M, N, K, per_part;            // columns per part, a multiple of 32
+};
+
+__device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+constexpr int MIX_WARPS = 8;
+
+// The mapping of gemv_nt_mma_kernel: 16 rows of one part of K.  (CTAs that stay for two to four such units took the same time.)
+__device__ __forceinline__ void mix_product(const MixParams& p, int unit) {
+    constexpr int U = 8;
+    __shared__ float sums[MIX_WARPS][16][8];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int tiles = p.N / 16, part = unit / tiles, row0 = (unit - part * tiles) * 16;
+    const int k0 = part * p.per_part, chunks = min(p.per_part, p.K - k0) / 32;
+    const __half* w_lo = p.w + (size_t)(row0 + g) * p.K + k0 + t * 8;
+    const __half* w_hi = w_lo + (size_t)8 * p.K;
+    const __half* x = p.x + (size_t)(g < p.M ? g : 0) * p.K + k0 + t * 8;
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    bool waited = false;
+    for (int c0 = warp; c0 < chunks || !waited; c0 += U * MIX_WARPS) {
+        uint4 lo[U], hi[U], xv[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int c = c0 + u * MIX_WARPS;
+            lo[u] = c < chunks ? ldg_nc16(w_lo + c * 32) : zero;
+            hi[u] = c < chunks ? ldg_nc16(w_hi + c * 32) : zero;
+        }
+        if (!waited) {
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            asm volatile("griddepcontrol.launch_dependents;");
+        }
+        waited = true;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int c = c0 + u * MIX_WARPS;
+            xv[u] = g < p.M && c < chunks ? __ldcg(reinterpret_cast<const uint4*>(x + c * 32)) : zero;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            mma_f16(acc, lo[u].x, hi[u].x, lo[u].y, hi[u].y, xv[u].x, xv[u].y);
+            mma_f16(acc, lo[u].z, hi[u].z, lo[u].w, hi[u].w, xv[u].z, xv[u].w);
+        }
+    }
+    sums[warp][g][2 * t] = acc[0];
+    sums[warp][g][2 * t + 1] = acc[1];
+    sums[warp][g + 8][2 * t] = acc[2];
+    sums[warp][g + 8][2 * t + 1] = acc[3];
+    __syncthreads();
+    if (tid < 128) {
+        const int m = tid >> 4, r = tid & 15;
+        if (m >= p.M) return;
+        float v = 0.f;
+#pragma unroll
+        for (int q = 0; q < MIX_WARPS; ++q) v += sums[q][r][m];
+        p.part[(size_t)part * 8 * p.N + (size_t)m * p.N + row0 + r] = v;
+    }
+}
+
+__global__ void __launch_bounds__(MIX_WARPS * 32, 2)
+decode_mix_kernel(const __grid_constant__ MixParams p) {
+    const int c = blockIdx.x;
+    if (c >= p.attn_ctas) {
+        mix_product(p, c - p.attn_ctas);
+    } else if (p.split_ctas) {
+        const int pair = c / p.split_ctas;
+        decode_split<false, MIX_WARPS>(p.a, c - pair * p.split_ctas, pair % p.a.n_heads, pair / p.a.n_heads);
+    } else {
+        decode_loop(p.a, c % p.a.n_heads, c / p.a.n_heads);
+    }
+}
+
+// The last product of a decode layer, 16 rows of w_out per CTA: all of their weights are requested before the dependency wait, and
+// what the glue reads beside the activations, so that two round trips are left of it.  As a plain GEMV (which asks for the glue's
+// operands when its sums are done) 4.7 us behind the kernel before it, 3.1 us now.
+// The kernel after it may start when this one has its inputs, not before: its requests (19 MB) ahead of them cost 1.6 us.
+constexpr int OUT_K = 2048;
+
+struct OutParams {
+    const __half *x, *w;      // [M][2048], [N][2048]
+    __half* out;              // [M][N]
+    md_epilogue ep;
+    int M, N;
+};
+
+__global__ void __launch_bounds__(MIX_WARPS * 32)
+decode_out_kernel(const __grid_constant__ OutParams p) {
+    constexpr int PIECES = OUT_K / 32 / MIX_WARPS;
+    __shared__ float sums[MIX_WARPS][16][8];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3, row0 = blockIdx.x * 16;
+    const __half* w_lo = p.w + (size_t)(row0 + g) * OUT_K + warp * 32 + t * 8;
+    uint4 lo[PIECES], hi[PIECES], xv[PIECES];
+#pragma unroll
+    for (int u = 0; u < PIECES; ++u) {
+        lo[u] = ldg_nc16(w_lo + u * MIX_WARPS * 32);
+        hi[u] = ldg_nc16(w_lo + (size_t)8 * OUT_K + u * MIX_WARPS * 32);
+    }
+    if (p.M > 0) asm volatile("griddepcontrol.wait;" ::: "memory");     // always: a branch the requests above do not sink below
+    asm volatile("griddepcontrol.launch_dependents;");
+#pragma unroll
+    for (int u = 0; u < PIECES; ++u)
+        xv[u] = g < p.M ? __ldcg(reinterpret_cast<const uint4*>(p.x + (size_t)g * OUT_K + (warp + u * MIX_WARPS) * 32 + t * 8))
+                        : make_uint4(0, 0, 0, 0);
+    const int o_m = tid >> 4, o_n = row0 + (tid & 15);
+    md_epilogue_ops ops;
+    if (o_m < p.M) ops = md_epilogue_fetch(p.ep, o_m, o_n, p.N);
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int u = 0; u < PIECES; ++u) {
+        mma_f16(acc, lo[u].x, hi[u].x, lo[u].y, hi[u].y, xv[u].x, xv[u].y);
+        mma_f16(acc, lo[u].z, hi[u].z, lo[u].w, hi[u].w, xv[u].z, xv[u].w);
+    }
+    sums[warp][g][2 * t] = acc[0];
+    sums[warp][g][2 * t + 1] = acc[1];
+    sums[warp][g + 8][2 * t] = acc[2];
+    sums[warp][g + 8][2 * t + 1] = acc[3];
+    __syncthreads();
+    if (o_m < p.M) {
+        float v = 0.f;
+#pragma unroll
+        for (int q = 0; q < MIX_WARPS; ++q) v += sums[q][tid & 15][o_m];
+        p.out[(size_t)o_m * p.N + o_n] = __float2half_rn(md_epilogue_apply(p.ep, ops, v));
     }
 }
 
@@ -982,14 +1131,12 @@ int md_launch_sdpa_decode_fused(md_ctx* ctx, const __half* qkv_row, __half* kc, 
 // The decode attention of `batch` requests (1..8) in one launch: request b reads row b of qkv (row stride
 // qkv_stride elements), appends to and reads its own cache kc[b] / vc[b] at the position held in pos_dev[b],
 // and writes row b of out (row stride out_stride).
-int md_launch_sdpa_decode_fused_devpos_batch(md_ctx* ctx, const __half* qkv, size_t qkv_stride, __half* const* kc,
-                                             __half* const* vc, __half* out, size_t out_stride, size_t batch,
-                                             size_t n_heads, size_t d, size_t max_seq, const int* const* pos_dev,
-                                             size_t rot_dim, float theta) {
+static int decode_batch_params(md_ctx* ctx, DecodeParams& p, const __half* qkv, size_t qkv_stride, __half* const* kc, __half* const* vc,
+                               __half* out, size_t out_stride, size_t batch, size_t n_heads, size_t d, size_t max_seq,
+                               const int* const* pos_dev, size_t rot_dim, float theta) {
     if (d != DEC_D || n_heads > 256)
         return md_fail(ctx, MD_ERR_UNSUPPORTED, "decode attention supports head_dim 64 and <= 256 heads");
     if (batch < 1 || batch > 8) return md_fail(ctx, MD_ERR_INVALID_ARG, "decode attention: batch must be 1..8");
-    DecodeParams p{};
     p.q = qkv; p.k = kc[0]; p.v = vc[0]; p.k_w = kc[0]; p.v_w = vc[0]; p.mask = nullptr; p.out = out;
     p.k_head_stride = (long long)max_seq * DEC_D;
     p.n_heads = (int)n_heads; p.fused = 1; p.rot_dim = (int)rot_dim; p.theta = theta;
@@ -1001,6 +1148,15 @@ int md_launch_sdpa_decode_fused_devpos_batch(md_ctx* ctx, const __half* qkv, siz
         p.out_batch_stride = (long long)out_stride;
         for (size_t b = 0; b < batch; ++b) { p.bk[b] = kc[b]; p.bv[b] = vc[b]; p.bpos[b] = pos_dev[b]; }
     }
+    return MD_OK;
+}
+
+int md_launch_sdpa_decode_fused_devpos_batch(md_ctx* ctx, const __half* qkv, size_t qkv_stride, __half* const* kc,
+                                             __half* const* vc, __half* out, size_t out_stride, size_t batch,
+                                             size_t n_heads, size_t d, size_t max_seq, const int* const* pos_dev,
+                                             size_t rot_dim, float theta) {
+    DecodeParams p{};
+    MD_TRY(decode_batch_params(ctx, p, qkv, qkv_stride, kc, vc, out, out_stride, batch, n_heads, d, max_seq, pos_dev, rot_dim, theta));
     if (decode_loop_wanted(ctx, p, batch)) return decode_loop_launch(ctx, p, batch);
     const int max_splits = (int)((max_seq + DEC_KEYS - 1) / DEC_KEYS);
     if (ctx->decode_cluster_ok < 0) {
@@ -1049,6 +1205,41 @@ int md_launch_sdpa_decode_fused_devpos_batch(md_ctx* ctx, const __half* qkv, siz
     if (le != cudaSuccess) return md_fail(ctx, MD_ERR_CUDA, "launch of sdpa_decode_kernel failed: %s", cudaGetErrorString(le));
     MD_LAUNCH_CHECK(ctx, "sdpa_decode_kernel");
     return MD_OK;
+}
+
+bool md_decode_mix_supported(size_t batch, size_t n_heads, size_t d, size_t N, size_t K) {
+    return batch >= 1 && batch <= 8 && d == DEC_D && n_heads * d == OUT_K && N % 16 == 0 && K % 32 == 0 && K > 0;
+}
+
+// What follows the first products of a decode layer: decode_mix_kernel and decode_out_kernel.  out = the glue of ep over
+// attention . w_out[N, 2048]^T; ep.parts = part, which the mix kernel fills with x[batch, K] . w[N, K]^T in `parts` ranges of K.
+int md_launch_decode_mix_out(md_ctx* ctx, const __half* qkv, size_t qkv_stride, __half* const* kc, __half* const* vc, __half* attn,
+                             size_t batch, size_t n_heads, size_t d, size_t max_seq, const int* const* pos_dev, size_t rot_dim, float theta,
+                             const __half* x, const __half* w, float* part, size_t N, size_t K, size_t parts, const __half* w_out,
+                             __half* out, const md_epilogue& ep) {
+    if (!md_decode_mix_supported(batch, n_heads, d, N, K) || rot_dim > DEC_D)
+        return md_fail(ctx, MD_ERR_UNSUPPORTED, "decode_mix_out: unsupported shape");
+    MixParams p{};
+    MD_TRY(decode_batch_params(ctx, p.a, qkv, qkv_stride, kc, vc, attn, OUT_K, batch, n_heads, d, max_seq, pos_dev, rot_dim, theta));
+    const bool loop = decode_loop_wanted(ctx, p.a, batch);
+    const size_t pairs = batch * n_heads;
+    p.split_ctas = loop ? 0 : (int)((max_seq + MIX_WARPS * 32 - 1) / (MIX_WARPS * 32));
+    p.attn_ctas = (int)pairs * (loop ? 1 : p.split_ctas);
+    if (!loop) {
+        void* scratch = nullptr;
+        MD_TRY(md_scratch(ctx, pairs * p.split_ctas * (DEC_D + 2) * sizeof(float), &scratch));
+        p.a.counters = ctx->counters;
+        p.a.partial = reinterpret_cast<float*>(scratch);
+        p.a.splits = p.split_ctas;
+    }
+    p.x = x; p.w = w; p.part = part;
+    p.M = (int)batch; p.N = (int)N; p.K = (int)K;
+    p.per_part = (int)((K / 32 + parts - 1) / parts * 32);
+    MD_TRY(md_launch_ex(ctx, decode_mix_kernel, dim3((unsigned)(p.attn_ctas + N / 16 * parts)), dim3(MIX_WARPS * 32), 0, "decode_mix_kernel", p));
+    OutParams o{};
+    o.x = attn; o.w = w_out; o.out = out; o.ep = ep;
+    o.M = (int)batch; o.N = (int)N;
+    return md_launch_ex(ctx, decode_out_kernel, dim3((unsigned)(N / 16)), dim3(MIX_WARPS * 32), 0, "decode_out_kernel", o);
 }
 
 int md_launch_sdpa_decode_fused_devpos(md_ctx* ctx, const __half* qkv_row, __half* kc, __half* vc, __half* out,

@@ -81,160 +81,181 @@ struct LnDualParams {
     int gelu1;                       // GELU on segment 1 as well (fc1 alone as segment 1)
 };
 
-// MM = compile-time bound on the number of activation rows (1, 2, 4 or 8): keeps the register
-// footprint of the single-stream case small enough for two CTAs per SM.
-template <int MM>
-__global__ void __launch_bounds__(LN_WARPS * 32)
-gemv_ln_dual_kernel(LnDualParams p) {
+// ONE: a single row, normalised by the whole CTA; else up to eight, a warp each.
+//
+// The CTAs stay: two per SM, an equal share of the rows of both matrices each, 16 rows at a time.  A lane's registers always hold
+// the requests of one whole tile (64 KB per CTA); as soon as a piece is multiplied its registers take the request of the same
+// piece of the next tile.  With a CTA per 16 rows a third of a CTA's life went to the LayerNorm, the sum over the warps and the
+// start of the next CTA, with nothing requested: 59 MB (qkv and fc1 in one launch) took 14.2 us, 11.7 now; lm_head (210 MB) 42.7,
+// 32.5 now.  One CTA per SM (64 KB in flight) takes 16 us for the 59 MB.
+template <bool ONE>
+__global__ void __launch_bounds__(LN_WARPS * 32, 2)
+gemv_ln_dual_kernel(LnDualParams p, int R) {
     __shared__ __align__(16) __half xs[8][LN_PITCH];
-    __shared__ float partial[LN_WARPS][16][8];
-    __shared__ float red[LN_WARPS][8];
-    __shared__ float stat[2][8];
+    __shared__ float partial[2][LN_WARPS][16][8];
+    __shared__ float red[2][LN_WARPS];
+    constexpr int PIECES = LN_CHUNKS / LN_WARPS;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    const int row0 = blockIdx.x * 16;
-    const bool seg2 = row0 >= p.n1;
-    const int n_seg = seg2 ? p.n2 : p.n1, r0 = seg2 ? row0 - p.n1 : row0;
-    const __half* W = seg2 ? p.w2 : p.w1;
-    const int r_lo = min(r0 + g, n_seg - 1), r_hi = min(r0 + g + 8, n_seg - 1);
-    const __half* w_lo = W + (size_t)r_lo * LN_K + t * 8;
-    const __half* w_hi = W + (size_t)r_hi * LN_K + t * 8;
+    const int total = p.n1 + p.n2, first = blockIdx.x * R, end = min(first + R, total);
 
     pdl_launch_dependents();
-    // every weight of this CTA is requested before anything else: 16 x 16 bytes per lane
-    uint4 lo[LN_CHUNKS / LN_WARPS], hi[LN_CHUNKS / LN_WARPS];
+    uint4 lo[PIECES], hi[PIECES];
+    const __half *w_lo, *w_hi;
+    bool has_lo, has_hi;
+    float bias = 0.f;                  // of this thread's output row
+    auto locate = [&](int row0) {      // this lane's two rows of a tile
+        const int a = row0 + g, c = a + 8;
+        has_lo = a < end, has_hi = c < end;
+        w_lo = (a < p.n1 ? p.w1 + (size_t)a * LN_K : p.w2 + (size_t)(a - p.n1) * LN_K) + warp * 32 + t * 8;
+        w_hi = (c < p.n1 ? p.w1 + (size_t)c * LN_K : p.w2 + (size_t)(c - p.n1) * LN_K) + warp * 32 + t * 8;
+        const int row = row0 + (tid & 15);
+        if (tid < 128 && row < end) bias = __half2float(row < p.n1 ? p.b1[row] : p.b2[row - p.n1]);
+    };
+    auto request = [&](int u) {
+        lo[u] = has_lo ? ldg_stream(w_lo + u * LN_WARPS * 32) : make_uint4(0, 0, 0, 0);
+        hi[u] = has_hi ? ldg_stream(w_hi + u * LN_WARPS * 32) : make_uint4(0, 0, 0, 0);
+    };
+    locate(first);
 #pragma unroll
-    for (int u = 0; u < LN_CHUNKS / LN_WARPS; ++u) {
-        const int k = (warp + u * LN_WARPS) * 32;
-        lo[u] = ldg_stream(w_lo + k);
-        hi[u] = ldg_stream(w_hi + k);
-    }
-    // LayerNorm parameters are weights too
-    const uint4 gw = ldg_stream(p.ln_w + tid * 8), gb = ldg_stream(p.ln_b + tid * 8);
-    pdl_wait();
+    for (int u = 0; u < PIECES; ++u) request(u);
 
     // ---- LayerNorm of the M rows into shared memory (two-pass f32, one f16 rounding)
-    float v[MM][8];
-    float s[MM];
-#pragma unroll
-    for (int m = 0; m < MM; ++m) {
-        s[m] = 0.f;
-        if (m < p.M) {
-            const uint4 u = ld_act(p.hidden + (size_t)m * LN_K + tid * 8);
-            const __half2* h = reinterpret_cast<const __half2*>(&u);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float2 f = __half22float2(h[i]);
-                v[m][2 * i] = f.x;
-                v[m][2 * i + 1] = f.y;
-                s[m] += f.x + f.y;
-            }
-        }
-    }
-    auto block_sum8 = [&](float (&x)[MM], int slot) {
-#pragma unroll
-        for (int m = 0; m < MM; ++m) {
-#pragma unroll
-            for (int o = 16; o; o >>= 1) x[m] += __shfl_xor_sync(0xffffffffu, x[m], o);
-        }
-        if (lane == 0) {
-#pragma unroll
-            for (int m = 0; m < MM; ++m) red[warp][m] = x[m];
-        }
-        __syncthreads();
-        if (tid < MM) {
-            float a = 0.f;
-#pragma unroll
-            for (int w = 0; w < LN_WARPS; ++w) a += red[w][tid];
-            stat[slot][tid] = a;
-        }
-        __syncthreads();
-    };
-    block_sum8(s, 0);
-    float q[MM];
-#pragma unroll
-    for (int m = 0; m < MM; ++m) {
-        q[m] = 0.f;
-        if (m < p.M) {
-            const float mean = stat[0][m] * (1.0f / LN_K);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float d = v[m][i] - mean;
-                q[m] += d * d;
-            }
-        }
-    }
-    block_sum8(q, 1);
-    {
-        const __half2* wh = reinterpret_cast<const __half2*>(&gw);
-        const __half2* bh = reinterpret_cast<const __half2*>(&gb);
-        float wv[8], bv[8];
+    auto normalised = [&](const float (&v)[8], float mean, float rstd, const uint4& gw, const uint4& gb) {
+        const __half2 *wh = reinterpret_cast<const __half2*>(&gw), *bh = reinterpret_cast<const __half2*>(&gb);
+        const float mean_rstd = mean * rstd;
+        uint4 o;
+        __half2* oh = reinterpret_cast<__half2*>(&o);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const float2 a = __half22float2(wh[i]), b = __half22float2(bh[i]);
-            wv[2 * i] = a.x; wv[2 * i + 1] = a.y;
-            bv[2 * i] = b.x; bv[2 * i + 1] = b.y;
+            oh[i] = __floats2half2_rn((v[2 * i] * rstd - mean_rstd) * a.x + b.x, (v[2 * i + 1] * rstd - mean_rstd) * a.y + b.y);
         }
+        return o;
+    };
+    auto unpack = [](const uint4& u, float (&v)[8]) {
+        const __half2* h = reinterpret_cast<const __half2*>(&u);
 #pragma unroll
-        for (int m = MM; m < 8; ++m) *reinterpret_cast<uint4*>(&xs[m][tid * 8]) = make_uint4(0, 0, 0, 0);
+        for (int i = 0; i < 4; ++i) {
+            const float2 f = __half22float2(h[i]);
+            v[2 * i] = f.x;
+            v[2 * i + 1] = f.y;
+        }
+    };
+    auto warp_sum = [](float x) {
 #pragma unroll
-        for (int m = 0; m < MM; ++m) {
-            uint4 o = make_uint4(0, 0, 0, 0);
-            if (m < p.M) {
-                const float mean = stat[0][m] * (1.0f / LN_K);
-                const float rstd = 1.0f / sqrtf(stat[1][m] * (1.0f / LN_K) + p.eps);
-                const float mean_rstd = mean * rstd;
-                __half2* oh = reinterpret_cast<__half2*>(&o);
+        for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        return x;
+    };
+    if constexpr (ONE) {
+        // LayerNorm parameters are weights too
+        const uint4 gw = ldg_stream(p.ln_w + tid * 8), gb = ldg_stream(p.ln_b + tid * 8);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float y0 = (v[m][2 * i] * rstd - mean_rstd) * wv[2 * i] + bv[2 * i];
-                    const float y1 = (v[m][2 * i + 1] * rstd - mean_rstd) * wv[2 * i + 1] + bv[2 * i + 1];
-                    oh[i] = __floats2half2_rn(y0, y1);
-                }
+        for (int m = 1; m < 8; ++m) *reinterpret_cast<uint4*>(&xs[m][tid * 8]) = make_uint4(0, 0, 0, 0);
+        pdl_wait();
+        auto block_sum = [&](float x, int slot) {
+            x = warp_sum(x);
+            if (lane == 0) red[slot][warp] = x;
+            __syncthreads();
+            x = 0.f;
+#pragma unroll
+            for (int w = 0; w < LN_WARPS; ++w) x += red[slot][w];
+            return x;
+        };
+        float v[8], s = 0.f, q = 0.f;
+        unpack(ld_act(p.hidden + tid * 8), v);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s += v[2 * i] + v[2 * i + 1];
+        const float mean = block_sum(s, 0) * (1.0f / LN_K);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) q += (v[i] - mean) * (v[i] - mean);
+        const float rstd = 1.0f / sqrtf(block_sum(q, 1) * (1.0f / LN_K) + p.eps);
+        *reinterpret_cast<uint4*>(&xs[0][tid * 8]) = normalised(v, mean, rstd, gw, gb);
+    } else {
+        pdl_wait();
+        constexpr int PER = LN_K / 256;      // 16-byte pieces of a row per lane
+        if (warp < p.M) {
+            uint4 row[PER];
+#pragma unroll
+            for (int i = 0; i < PER; ++i) row[i] = ld_act(p.hidden + (size_t)warp * LN_K + (i * 32 + lane) * 8);
+            float s = 0.f, q = 0.f;
+#pragma unroll
+            for (int i = 0; i < PER; ++i) {
+                float v[8];
+                unpack(row[i], v);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) s += v[2 * j] + v[2 * j + 1];
             }
-            *reinterpret_cast<uint4*>(&xs[m][tid * 8]) = o;
+            const float mean = warp_sum(s) * (1.0f / LN_K);
+#pragma unroll
+            for (int i = 0; i < PER; ++i) {
+                float v[8];
+                unpack(row[i], v);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) q += (v[j] - mean) * (v[j] - mean);
+            }
+            const float rstd = 1.0f / sqrtf(warp_sum(q) * (1.0f / LN_K) + p.eps);
+#pragma unroll
+            for (int i = 0; i < PER; ++i) {
+                float v[8];
+                unpack(row[i], v);
+                const int c = (i * 32 + lane) * 8;
+                *reinterpret_cast<uint4*>(&xs[warp][c]) = normalised(v, mean, rstd, ldg_stream(p.ln_w + c), ldg_stream(p.ln_b + c));
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < PER; ++i) *reinterpret_cast<uint4*>(&xs[warp][(i * 32 + lane) * 8]) = make_uint4(0, 0, 0, 0);
         }
     }
     __syncthreads();
+    uint4 xv[PIECES];
+#pragma unroll
+    for (int u = 0; u < PIECES; ++u) xv[u] = *reinterpret_cast<const uint4*>(&xs[g][(warp + u * LN_WARPS) * 32 + t * 8]);  // rows >= M are zeros
 
     // ---- the dot products
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    unsigned long long best = 0ull;
+    int buf = 0;
+    for (int row0 = first; row0 < end; row0 += 16, buf ^= 1) {
+        const float own_bias = bias;
+        locate(row0 + 16);
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int u = 0; u < LN_CHUNKS / LN_WARPS; ++u) {
-        const int k = (warp + u * LN_WARPS) * 32;
-        const uint4 xv = *reinterpret_cast<const uint4*>(&xs[g][k + t * 8]);  // rows >= M are zeros
-        mma_16816(acc, lo[u].x, hi[u].x, lo[u].y, hi[u].y, xv.x, xv.y);
-        mma_16816(acc, lo[u].z, hi[u].z, lo[u].w, hi[u].w, xv.z, xv.w);
+        for (int u = 0; u < PIECES; ++u) {
+            mma_16816(acc, lo[u].x, hi[u].x, lo[u].y, hi[u].y, xv[u].x, xv[u].y);
+            mma_16816(acc, lo[u].z, hi[u].z, lo[u].w, hi[u].w, xv[u].z, xv[u].w);
+            request(u);
+        }
+        float (*mine)[16][8] = partial[buf];
+        mine[warp][g][2 * t] = acc[0];
+        mine[warp][g][2 * t + 1] = acc[1];
+        mine[warp][g + 8][2 * t] = acc[2];
+        mine[warp][g + 8][2 * t + 1] = acc[3];
+        __syncthreads();
+        if (tid >= 128) continue;
+        const int m = tid >> 4, row = row0 + (tid & 15);
+        if (m >= p.M || row >= end) continue;
+        const bool seg2 = row >= p.n1;
+        const int n = seg2 ? row - p.n1 : row, n_seg = seg2 ? p.n2 : p.n1;
+        float sum = 0.f;
+#pragma unroll
+        for (int w = 0; w < LN_WARPS; ++w) sum += mine[w][tid & 15][m];
+        float val = md_round_f16(sum);
+        val = md_round_f16(val + own_bias);
+        if (seg2 || p.gelu1) val = md_round_f16(md_gelu_f32(val));
+        (seg2 ? p.out2 : p.out1)[(size_t)m * n_seg + n] = __float2half_rn(val);
+        // Greedy sampling folded into the lm_head (sampling.zig:257-273: first strict maximum of the f16
+        // logits): a 64-bit key orders by value, then by LOWER index; one atomicMax per CTA and row.
+        const unsigned bits = __float_as_uint(val);
+        const unsigned ordered = (bits & 0x80000000u) ? ~bits : (bits | 0x80000000u);
+        const unsigned long long key = ((unsigned long long)ordered << 32) | (unsigned long long)(0xFFFFFFFFu - (unsigned)n);
+        if (!seg2) best = key > best ? key : best;
     }
-    partial[warp][g][2 * t] = acc[0];
-    partial[warp][g][2 * t + 1] = acc[1];
-    partial[warp][g + 8][2 * t] = acc[2];
-    partial[warp][g + 8][2 * t + 1] = acc[3];
-    __syncthreads();
-    if (tid < 128) {
-        const int m = tid >> 4, r = tid & 15, n = r0 + r;
-        unsigned long long key = 0ull;
-        if (m < p.M && n < n_seg) {
-            float sum = 0.f;
+    if (p.amax && tid < 128) {
 #pragma unroll
-            for (int w = 0; w < LN_WARPS; ++w) sum += partial[w][r][m];
-            float val = md_round_f16(sum);
-            val = md_round_f16(val + __half2float((seg2 ? p.b2 : p.b1)[n]));
-            if (seg2 || p.gelu1) val = md_round_f16(md_gelu_f32(val));
-            (seg2 ? p.out2 : p.out1)[(size_t)m * n_seg + n] = __float2half_rn(val);
-            // Greedy sampling folded into the lm_head (sampling.zig:257-273: first strict maximum of the f16
-            // logits): a 64-bit key orders by value, then by LOWER index; one atomicMax per CTA and row.
-            const unsigned bits = __float_as_uint(val);
-            const unsigned ordered = (bits & 0x80000000u) ? ~bits : (bits | 0x80000000u);
-            key = ((unsigned long long)ordered << 32) | (unsigned long long)(0xFFFFFFFFu - (unsigned)n);
+        for (int o = 8; o; o >>= 1) {
+            const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
+            best = other > best ? other : best;
         }
-        if (p.amax && !seg2) {
-#pragma unroll
-            for (int o = 8; o; o >>= 1) {
-                const unsigned long long other = __shfl_xor_sync(0xffffffffu, key, o);
-                key = other > key ? other : key;
-            }
-            if (r == 0 && m < p.M) atomicMax(p.amax + m, key);
-        }
+        if ((tid & 15) == 0 && (tid >> 4) < p.M) atomicMax(p.amax + (tid >> 4), best);
     }
 }
 
@@ -326,8 +347,8 @@ gemv_dual_k_kernel(DualKParams p) {
     }
 }
 
-template <class Kern, class Params>
-int launch_pdl(md_ctx* ctx, Kern kern, unsigned grid, unsigned block, const Params& p, const char* name) {
+template <class Kern, class Params, class... More>
+int launch_pdl(md_ctx* ctx, Kern kern, unsigned grid, unsigned block, const Params& p, const char* name, More... more) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
@@ -337,7 +358,7 @@ int launch_pdl(md_ctx* ctx, Kern kern, unsigned grid, unsigned block, const Para
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = ctx->pdl ? 1 : 0;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p, more...);
     if (e != cudaSuccess) return md_fail(ctx, MD_ERR_CUDA, "launch of %s failed: %s", name, cudaGetErrorString(e));
     ctx->launches++;
     return MD_OK;
@@ -361,11 +382,11 @@ int md_launch_gemv_ln_dual(md_ctx* ctx, const __half* hidden, const __half* ln_w
     p.n1 = (int)n1; p.n2 = (int)n2; p.M = (int)M;
     p.amax = amax;
     p.gelu1 = gelu1 ? 1 : 0;
-    const unsigned grid = (unsigned)((n1 + n2) / 16);
-    if (M == 1) return launch_pdl(ctx, gemv_ln_dual_kernel<1>, grid, LN_WARPS * 32, p, "gemv_ln_dual_kernel");
-    if (M == 2) return launch_pdl(ctx, gemv_ln_dual_kernel<2>, grid, LN_WARPS * 32, p, "gemv_ln_dual_kernel");
-    if (M <= 4) return launch_pdl(ctx, gemv_ln_dual_kernel<4>, grid, LN_WARPS * 32, p, "gemv_ln_dual_kernel");
-    return launch_pdl(ctx, gemv_ln_dual_kernel<8>, grid, LN_WARPS * 32, p, "gemv_ln_dual_kernel");
+    // an equal share for every CTA that fits at once, in rows (fewer tiles than that: one each)
+    const int total = (int)(n1 + n2), ctas = 2 * ctx->sm_count;
+    const int R = total / 16 < ctas ? 16 : (total + ctas - 1) / ctas;
+    const unsigned grid = (unsigned)((total + R - 1) / R);
+    return launch_pdl(ctx, M == 1 ? gemv_ln_dual_kernel<true> : gemv_ln_dual_kernel<false>, grid, LN_WARPS * 32, p, "gemv_ln_dual_kernel", R);
 }
 
 bool md_gemv_dual_k_supported(size_t M, size_t N, size_t k1, size_t k2) {

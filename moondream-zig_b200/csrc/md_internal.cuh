@@ -101,6 +101,8 @@ struct md_ctx {
     int pdl = 0;             // md_set_option("pdl"): programmatic dependent launch for the GEMV kernels
     int prefill_fork = 1;       // md_set_option("prefill_fork"): prefill layers run the MLP beside the attention
     int decode_split_ln = 5;    // md_set_option("decode_split_ln"): from this many rows on a decode step runs the LayerNorm once
+    int decode_chain = 1;       // md_set_option("decode_chain"): a decode layer runs as three kernels of one chain; setting decode_fork
+                                // or decode_mlp_split turns it off and chooses between the two-chain forms
     int decode_fork = 1;        // md_set_option("decode_fork"): a decode layer runs as two concurrent kernel chains
     int attn_ctas_per_sm = 2;   // md_set_option("attn_ctas_per_sm"): grid of the tcgen05 attention = this many CTAs per SM, each
                                 // walking several (query block, head, batch) items; 0 = one CTA per item
@@ -342,23 +344,35 @@ __device__ __forceinline__ float md_apply_epilogue(float acc, float bias, bool h
 }
 
 // The fused glue for output element (m, n): f16(acc) -> +bias -> gelu -> +residual -> +residual2, one
-// rounding to f16 after every step, exactly where the reference's separate ops round.
-__device__ __forceinline__ float md_epilogue_value(const md_epilogue& ep, float acc, int m, int n, int N) {
-    float v = md_round_f16(acc);
-    if (ep.bias) v = md_round_f16(v + __half2float(ep.bias[n]));
-    if (ep.gelu) v = md_round_f16(md_gelu_f32(v));
+// rounding to f16 after every step, exactly where the reference's separate ops round.  In two halves, so that a kernel can request
+// what the glue reads ahead of its sums.
+struct md_epilogue_ops { float bias, residual, part, bias2, residual2; };
+__device__ __forceinline__ md_epilogue_ops md_epilogue_fetch(const md_epilogue& ep, int m, int n, int N) {
+    md_epilogue_ops o = {0.f, 0.f, 0.f, 0.f, 0.f};
+    if (ep.bias) o.bias = __half2float(ep.bias[n]);
     if (ep.residual) {
         const int rm = ep.residual_rows > 0 ? m % ep.residual_rows : m;
-        v = md_round_f16(v + __half2float(__ldcg(ep.residual + (size_t)rm * N + n)));
+        o.residual = __half2float(__ldcg(ep.residual + (size_t)rm * N + n));
     }
     if (ep.parts) {
-        // the other projection arrives as parts of its K sum: one rounding of the sum, then its bias
-        float r = 0.f;
-        for (int i = 0; i < ep.n_parts; ++i) r += __ldcg(ep.parts + (size_t)i * ep.part_stride + (size_t)m * N + n);
-        r = md_round_f16(md_round_f16(r) + __half2float(ep.bias2[n]));
-        v = md_round_f16(v + r);
+#pragma unroll 4
+        for (int i = 0; i < ep.n_parts; ++i) o.part += __ldcg(ep.parts + (size_t)i * ep.part_stride + (size_t)m * N + n);
+        o.bias2 = __half2float(ep.bias2[n]);
     }
-    if (ep.residual2) v = md_round_f16(v + __half2float(__ldcg(ep.residual2 + (size_t)m * N + n)));
+    if (ep.residual2) o.residual2 = __half2float(__ldcg(ep.residual2 + (size_t)m * N + n));
+    return o;
+}
+__device__ __forceinline__ float md_epilogue_apply(const md_epilogue& ep, const md_epilogue_ops& o, float acc) {
+    float v = md_round_f16(acc);
+    if (ep.bias) v = md_round_f16(v + o.bias);
+    if (ep.gelu) v = md_round_f16(md_gelu_f32(v));
+    if (ep.residual) v = md_round_f16(v + o.residual);
+    // the other projection arrives as parts of its K sum: one rounding of the sum, then its bias
+    if (ep.parts) v = md_round_f16(v + md_round_f16(md_round_f16(o.part) + o.bias2));
+    if (ep.residual2) v = md_round_f16(v + o.residual2);
     return v;
+}
+__device__ __forceinline__ float md_epilogue_value(const md_epilogue& ep, float acc, int m, int n, int N) {
+    return md_epilogue_apply(ep, md_epilogue_fetch(ep, m, n, N), acc);
 }
 #endif

@@ -12,6 +12,11 @@
 
 extern "C" int md_gemm_dispatch(md_ctx* ctx, const __half* a, const __half* b, __half* c, size_t M, size_t N, size_t K,
                                 int b_layout, const md_epilogue& ep);
+bool md_decode_mix_supported(size_t batch, size_t n_heads, size_t d, size_t N, size_t K);
+int md_launch_decode_mix_out(md_ctx* ctx, const __half* qkv, size_t qkv_stride, __half* const* kc, __half* const* vc, __half* attn,
+                             size_t batch, size_t n_heads, size_t d, size_t max_seq, const int* const* pos_dev, size_t rot_dim, float theta,
+                             const __half* x, const __half* w, float* part, size_t N, size_t K, size_t parts, const __half* w_out,
+                             __half* out, const md_epilogue& ep);
 int md_launch_sdpa_decode_fused_devpos_batch(md_ctx* ctx, const __half* qkv, size_t qkv_stride, __half* const* kc,
                                              __half* const* vc, __half* out, size_t out_stride, size_t batch,
                                              size_t n_heads, size_t d, size_t max_seq, const int* const* pos_dev,
@@ -184,6 +189,31 @@ int text_layer(md_text_model* m, size_t layer, const LayerIO& io, size_t rows, b
     // (one CTA per SM instead of two) and L2 reads, so from ctx->decode_split_ln rows on the LayerNorm runs once
     // as its own kernel and plain GEMVs with fused epilogues follow (the generic path below, forked the same way).
     const bool ln_once = ctx->decode_split_ln > 0 && rows >= (size_t)ctx->decode_split_ln;
+    if (decode && ctx->fused_decode && ctx->decode_chain && io.mlp_part && md_gemv_ln_dual_supported(rows, D, 3 * D, F) &&
+        md_decode_mix_supported(rows, w.n_heads, w.head_dim, D, F) && w.rot_dim <= w.head_dim) {
+        // Three kernels in one chain, each started under its predecessor with its first weights requested:
+        //   [LayerNorm + qkv, fc1 + GELU] -> [attention, fc2 in four parts of its K sum] -> [out-proj + bias + the parts + hidden]
+        // Same rounding points as below.
+        constexpr size_t PARTS = 4;
+        MD_TRY(md_launch_gemv_ln_dual(ctx, io.hidden, H(m->ln_w[layer]), H(m->ln_b[layer]), eps_of(w.eps_f16), H(m->wqkv[layer]),
+                                      H(m->bqkv[layer]), io.qkv, 3 * D, H(m->wfc1[layer]), H(m->bfc1[layer]), io.fc1, F, rows, D));
+        __half *kc[8], *vc[8];
+        const int* pos[8];
+        for (size_t b = 0; b < rows; ++b) {
+            kc[b] = reqs[b]->kc[layer];
+            vc[b] = reqs[b]->vc[layer];
+            pos[b] = reqs[b]->pos_dev;
+        }
+        md_epilogue e_out;
+        e_out.bias = H(m->bout[layer]);
+        e_out.parts = io.mlp_part;
+        e_out.n_parts = (int)PARTS;
+        e_out.part_stride = (int)(8 * D);
+        e_out.bias2 = H(m->bfc2[layer]);
+        e_out.residual2 = io.hidden;    // updated in place: every element is read and written by one thread
+        return md_launch_decode_mix_out(ctx, io.qkv, 3 * D, kc, vc, io.attn, rows, w.n_heads, w.head_dim, w.max_seq, pos, w.rot_dim,
+                                        w.rope_theta, io.fc1, H(m->wfc2[layer]), io.mlp_part, D, F, PARTS, H(m->wout[layer]), io.hidden, e_out);
+    }
     if (decode && ctx->fused_decode && !ln_once && md_gemv_ln_dual_supported(rows, D, 3 * D, F) &&
         md_gemv_dual_k_supported(rows, D, D, F)) {
         if (ctx->decode_fork) {
@@ -661,7 +691,7 @@ static int enqueue_decode_step(md_text_model* model, md_text_request* const* req
     // (742 -> 730 us per step at 1 row, 962 -> 942 at 4 rows, 1210 -> 1079 at 6 rows).
     GemvVariantScope gemv_scope(ctx, 3);
     for (size_t l = 0; l < w.n_layers; ++l) MD_TRY(text_layer(model, l, io, batch, true, reqs, 0));
-    const bool fused_head = ctx->fused_decode && !ln_once && md_gemv_ln_dual_supported(batch, w.dim, w.vocab, 0);
+    const bool fused_head = ctx->fused_decode && (!ln_once || ctx->decode_chain) && md_gemv_ln_dual_supported(batch, w.dim, w.vocab, 0);
     if (fused_head) {
         // final LayerNorm + lm_head + greedy argmax in one kernel (text_model.zig:325-345, sampling.zig:257-273)
         MD_TRY(md_launch_gemv_ln_dual(ctx, r0->hidden.as<__half>(), H(w.ln_out_w), H(w.ln_out_b), eps_of(w.eps_f16),

@@ -243,6 +243,39 @@ def test_text_split_mlp_decode_layer_matches_the_single_mlp_chain(ctx, oracle, m
     gpu.close()
 
 
+@pytest.mark.parametrize("hidden", [8192, 1120, 32])
+def test_text_decode_layer_as_one_chain_matches_the_two_chain_layer(ctx, models_mod, hidden):
+    """Option decode_chain (default on): the attention and fc2 in one launch, fc2 in four parts of its K sum (hidden 1120: unequal
+    parts, 32: three empty ones).  Same rounding points as the two-chain layer; positions around the edges of a 256-key split."""
+    w = text_weights(4021, n_layers=2, hidden=hidden, vocab=2048)
+    gpu = models_mod.TextModel(ctx, w, max_seq=1024)
+    rng = np.random.default_rng(21)
+    prompts = [w["wte"][rng.integers(0, 2048, n)] for n in (1, 254, 256, 511, 3, 700, 257, 40)]
+    forced = np.arange(1, 5, dtype=np.uint32) * 43 % 2048
+    rows, tokens = {}, {}
+    try:
+        for chain in (1, 0):
+            ctx.set_option("decode_chain", chain)
+            reqs = [gpu.request() for _ in prompts]
+            firsts = [gpu.forward(r, p)[2] for r, p in zip(reqs, prompts)]
+            rows[chain] = [gpu.generate(r, 7, 4, forced=forced, want_logits=True)[1] for r in reqs]
+            for batch in (2, 5, 8):     # key splits; one CTA per head and request
+                for r, p in zip(reqs[:batch], prompts):
+                    r.reset()
+                    gpu.forward(r, p)
+                tokens[chain, batch] = np.asarray(gpu.generate_batch(reqs[:batch], firsts[:batch], 6))
+            for r in reqs:
+                r.close()
+    finally:
+        ctx.set_option("decode_chain", 1)
+    for a, b in zip(rows[1], rows[0]):
+        for i in range(4):
+            assert_close_ref(a[i], b[i], f"one chain vs two, step {i}", rel=5e-3)
+    for batch in (2, 5, 8):
+        assert (tokens[1, batch] == tokens[0, batch]).mean() >= 0.8      # random weights: near-ties may flip a token
+    gpu.close()
+
+
 @pytest.mark.parametrize("cluster_merge", [1, 0], ids=["cluster_merge", "scratch_merge"])
 def test_text_batched_decode_equals_single_requests(ctx, models_mod, cluster_merge):
     """One attention launch serves the whole batch (grid z = request), each request at its own position; both ways
