@@ -314,6 +314,7 @@ struct DecodeParams {
     int splits;
     const float* rope_tab;  // fused: (cos, sin) table [positions][rot_dim/2][2] (rope.zig:32-128)
     const int* pos_ptr;     // fused + graph replay: position read from device memory, else null
+    int late;               // nothing is read before the dependency wait (the caches may be the predecessor's result)
     // batch > 0: blockIdx.z selects one of up to 8 requests, each with its own cache and position; q and out
     // advance by a row per request, partial and counters by one request's worth
     int batch;
@@ -390,6 +391,7 @@ __device__ __forceinline__ void decode_split(const DecodeParams& gp, int split, 
     const float scale = 0.125f;  // 1/sqrt(64)
 
     const int sub = lane & 7, grp = lane >> 3;  // 8 lanes x 16 B cover one 128-byte key row
+    if (p.late) asm volatile("griddepcontrol.wait;" ::: "memory");
     // ---- request this CTA's keys and values first: the cached prefix was written by earlier steps, so
     //      under programmatic dependent launch these loads overlap the tail of the kernel that produces q
     asm volatile("griddepcontrol.launch_dependents;");
@@ -640,6 +642,7 @@ __device__ __forceinline__ void decode_loop(const DecodeParams& gp, int head, in
     __half* kc = batched ? gp.bk[b] : gp.k_w;
     __half* vc = batched ? gp.bv[b] : gp.v_w;
     const int* pos_ptr = batched ? gp.bpos[b] : gp.pos_ptr;
+    if (gp.late) asm volatile("griddepcontrol.wait;" ::: "memory");
     const int pos = pos_ptr ? *pos_ptr : gp.pos;   // keys 0 .. pos-1 are in the cache, the new token becomes key pos
     const float scale = 0.125f;           // 1/sqrt(64)
     const int sub = lane & 7, grp = lane >> 3;
@@ -1092,6 +1095,7 @@ static int decode_loop_launch(md_ctx* ctx, const DecodeParams& p, size_t batch) 
 }
 
 static int decode_launch(md_ctx* ctx, DecodeParams& p) {
+    p.late = !md_launch_early(ctx);
     if (decode_loop_wanted(ctx, p, 1)) return decode_loop_launch(ctx, p, 1);
     p.splits = (p.kv_cache_len + DEC_KEYS - 1) / DEC_KEYS;
     if (p.splits < 1) p.splits = 1;
@@ -1100,10 +1104,7 @@ static int decode_launch(md_ctx* ctx, DecodeParams& p) {
     MD_TRY(md_scratch(ctx, partial_bytes, &scratch));
     p.counters = ctx->counters;
     p.partial = reinterpret_cast<float*>(scratch);
-    dim3 grid((unsigned)p.splits, (unsigned)p.n_heads);
-    sdpa_decode_kernel<false><<<grid, DEC_WARPS * 32, 0, ctx->stream>>>(p);
-    MD_LAUNCH_CHECK(ctx, "sdpa_decode_kernel");
-    return MD_OK;
+    return md_launch_ex(ctx, sdpa_decode_kernel<false>, dim3((unsigned)p.splits, (unsigned)p.n_heads), dim3(DEC_WARPS * 32), 0, "sdpa_decode_kernel", p);
 }
 
 int md_launch_sdpa_single(md_ctx* ctx, const __half* q, const __half* k, const __half* v, const uint8_t* mask,
@@ -1140,6 +1141,7 @@ static int decode_batch_params(md_ctx* ctx, DecodeParams& p, const __half* qkv, 
     p.q = qkv; p.k = kc[0]; p.v = vc[0]; p.k_w = kc[0]; p.v_w = vc[0]; p.mask = nullptr; p.out = out;
     p.k_head_stride = (long long)max_seq * DEC_D;
     p.n_heads = (int)n_heads; p.fused = 1; p.rot_dim = (int)rot_dim; p.theta = theta;
+    p.late = !md_launch_early(ctx);
     MD_TRY(md_rope_cached(ctx, rot_dim, theta, max_seq, &p.rope_tab));
     p.pos_ptr = pos_dev[0];
     if (batch > 1) {

@@ -43,7 +43,7 @@ constexpr int MAX_SPLITS = 8;          // portable cluster size
 template <bool W_MN_MAJOR, bool BF16>
 __global__ void __launch_bounds__(THREADS, 2)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, __half* C, int M,
-                   int N, int K, int kb_per_split, int splits, md_epilogue ep, md_devflags* flags, md_lin lin) {
+                   int N, int K, int kb_per_split, int splits, int early, md_epilogue ep, md_devflags* flags, md_lin lin) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
@@ -107,6 +107,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             // the first ring of weight tiles does not depend on the predecessor kernel (registered weights are
             // never written on the stream): request it before waiting for the activations' producer
             const int first = min(kbs, STAGES);
+            if (!early) md_pdl_wait();     // the weights may be the predecessor's result
             for (int i = 0; i < first; ++i) load_w(i, kb0 + i);
             md_pdl_wait();
             for (int i = 0; i < first; ++i) load_x(i, kb0 + i);
@@ -282,7 +283,7 @@ bool md_gemm_skinny_supported(const void* a, const void* b, const void* c, size_
 
 namespace {
 
-typedef void (*skinny_fn)(CUtensorMap, CUtensorMap, __half*, int, int, int, int, int, md_epilogue, md_devflags*, md_lin);
+typedef void (*skinny_fn)(CUtensorMap, CUtensorMap, __half*, int, int, int, int, int, int, md_epilogue, md_devflags*, md_lin);
 
 int launch_splits(md_ctx* ctx, skinny_fn kern, uint32_t cfg_bit, const CUtensorMap& tm_w, const CUtensorMap& tm_x, __half* c, size_t M,
                   size_t N, size_t K, const md_epilogue& ep, const md_lin& lin) {
@@ -322,7 +323,7 @@ int launch_splits(md_ctx* ctx, skinny_fn kern, uint32_t cfg_bit, const CUtensorM
     cfg.attrs = attr;
     cfg.numAttrs = na;
     const int Mi = (int)M, Ni = (int)N, Ki = (int)K;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tm_w, tm_x, c, Mi, Ni, Ki, kb_per_split, splits, ep, ctx->flags, lin);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tm_w, tm_x, c, Mi, Ni, Ki, kb_per_split, splits, md_launch_early(ctx), ep, ctx->flags, lin);
     if (e != cudaSuccess) return md_fail(ctx, MD_ERR_CUDA, "launch of gemm_skinny_kernel failed: %s", cudaGetErrorString(e));
     ctx->launches++;
     return MD_OK;

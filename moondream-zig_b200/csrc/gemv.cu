@@ -66,7 +66,7 @@ constexpr int ROWS_PER_CTA = 16;
 template <int WARPS, int UNROLL>
 __global__ void __launch_bounds__(WARPS * 32)
 gemv_nt_mma_kernel(const __half* A, const __half* __restrict__ Bt, __half* C, int M, int N,
-                   int K, int ldb, md_epilogue ep) {
+                   int K, int ldb, int early, md_epilogue ep) {
     __shared__ float partial[WARPS][ROWS_PER_CTA][8];
     __shared__ float cta_sum[ROWS_PER_CTA * 8];   // this CTA's 16 x 8 sums, read by the cluster's first CTA
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -91,7 +91,8 @@ gemv_nt_mma_kernel(const __half* A, const __half* __restrict__ Bt, __half* C, in
     // stream this kernel's first weights (which no earlier kernel writes) before waiting for the kernel
     // that produces the activations.  Without the launch attribute both instructions are no-ops.
     asm volatile("griddepcontrol.launch_dependents;");
-    bool waited = false;
+    bool waited = !early;
+    if (!early) asm volatile("griddepcontrol.wait;" ::: "memory");    // the weights may be the predecessor's result
     for (; ch + (UNROLL - 1) * WARPS < chunks; ch += UNROLL * WARPS) {
         uint4 lo[UNROLL], hi[UNROLL], xv[UNROLL];
 #pragma unroll
@@ -376,7 +377,7 @@ int md_launch_gemv_nt(md_ctx* ctx, const __half* a, const __half* bt, __half* c,
 #define MD_GEMV_CASE(id, W, U)                                                          \
     case id:                                                                            \
         cfg.blockDim = dim3(W * 32);                                                    \
-        le = cudaLaunchKernelEx(&cfg, gemv_nt_mma_kernel<W, U>, a, bt, c, Mi, Ni, Ki, ldbi, ep); \
+        le = cudaLaunchKernelEx(&cfg, gemv_nt_mma_kernel<W, U>, a, bt, c, Mi, Ni, Ki, ldbi, md_launch_early(ctx), ep); \
         break;
     switch (variant) {
         MD_GEMV_CASE(1, 4, 8)

@@ -378,6 +378,8 @@ __global__ void rope_apply_kernel(const __half* __restrict__ x, __half* __restri
 
 // attention.zig:256-281
 __global__ void mask_kernel(uint8_t* __restrict__ mask, size_t pos, size_t seq_len) {
+    md_pdl_launch_dependents();
+    md_pdl_wait();
     const size_t w = pos + seq_len, total = seq_len * w;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -512,9 +514,7 @@ int md_launch_rope_apply(md_ctx* ctx, const __half* x, __half* out, size_t n_hea
 int md_launch_mask(md_ctx* ctx, uint8_t* mask, size_t pos, size_t seq_len) {
     const size_t n = seq_len * (pos + seq_len);
     if (!n) return MD_OK;
-    mask_kernel<<<grid_for(n, 256, ctx->sm_count), 256, 0, ctx->stream>>>(mask, pos, seq_len);
-    MD_LAUNCH_CHECK(ctx, "mask_kernel");
-    return MD_OK;
+    return md_launch_ex(ctx, mask_kernel, dim3((unsigned)grid_for(n, 256, ctx->sm_count)), dim3(256), 0, "mask_kernel", mask, pos, seq_len);
 }
 
 int md_launch_kv_update(md_ctx* ctx, __half* kc, __half* vc, const __half* k, const __half* v, size_t n_heads,

@@ -547,9 +547,26 @@ int md_gemm_dispatch(md_ctx* ctx, const __half* a, const __half* b, __half* c, s
     return md_launch_gemm_simt(ctx, a, b, c, M, N, K, b_layout, ep);
 }
 
+// While alive, the kernels of a product or an attention called by itself are launched dependent on their predecessor: barriers,
+// tensor memory and the start of the grid come under its end, and every one of them waits for it before it reads or writes anything
+// (md_launch_early).  Back to back on one stream: the five products of a decode step 75.8 -> 64.9 us, four of 64
+// rows 58.7 -> 55.8, the attention of an image and of a prompt under its mask, with the mask, 54 -> 46.7.
+// Not while a graph is captured: a captured call keeps plain edges.
+struct CallScope {
+    md_ctx* c;
+    bool on;
+    explicit CallScope(md_ctx* ctx) : c(ctx), on(ctx && !ctx->pdl && !ctx->capturing) {
+        if (on) c->pdl = 1, c->pdl_late = true;
+    }
+    ~CallScope() {
+        if (on) c->pdl = 0, c->pdl_late = false;
+    }
+};
+
 static int hgemm_entry(md_ctx* ctx, const uint16_t* a, const uint16_t* b, uint16_t* c, size_t M, size_t N, size_t K,
                        int b_layout) {
     MD_NEED_CTX(ctx);
+    CallScope call(ctx);
     MD_NEED(ctx, a && b && c, "hgemm: null tensor pointer");
     MD_CUDA(ctx, cudaSetDevice(ctx->device));
     md_arg A, B, Cc;
@@ -577,6 +594,7 @@ int md_hgemm_nt(md_ctx* ctx, const uint16_t* a, const uint16_t* b_t, uint16_t* c
 int md_hgemm_fused(md_ctx* ctx, const uint16_t* a, const uint16_t* b, uint16_t* c, size_t M, size_t N, size_t K,
                    int b_layout, const uint16_t* bias, int gelu, const uint16_t* residual) {
     MD_NEED_CTX(ctx);
+    CallScope call(ctx);
     MD_NEED(ctx, a && b && c, "hgemm_fused: null tensor pointer");
     MD_NEED(ctx, b_layout == 0 || b_layout == 1, "hgemm_fused: b_layout must be 0 or 1");
     md_epilogue ep;
@@ -626,6 +644,7 @@ int md_gather_colblocks(md_ctx* ctx, const uint16_t* gathered, uint16_t* c, size
 int md_sdpa_maskless(md_ctx* ctx, const uint16_t* q, const uint16_t* k, const uint16_t* v, uint16_t* out,
                      size_t n_heads, size_t q_len, size_t kv_len, size_t d) {
     MD_NEED_CTX(ctx);
+    CallScope call(ctx);
     MD_NEED(ctx, q && k && v && out, "sdpa_maskless: null tensor pointer");
     MD_NEED(ctx, n_heads && q_len && kv_len && d, "sdpa_maskless: zero-sized dimension");
     md_arg Q, Kk, V, O;
@@ -641,6 +660,7 @@ int md_sdpa_maskless(md_ctx* ctx, const uint16_t* q, const uint16_t* k, const ui
 
 int md_create_attention_mask(md_ctx* ctx, uint8_t* mask, size_t pos, size_t seq_len) {
     MD_NEED_CTX(ctx);
+    CallScope call(ctx);
     MD_NEED(ctx, mask, "create_attention_mask: null pointer");
     md_arg Mk;
     MD_TRY(md_stage_out(ctx, 0, mask, seq_len * (pos + seq_len), &Mk));
@@ -651,6 +671,7 @@ int md_create_attention_mask(md_ctx* ctx, uint8_t* mask, size_t pos, size_t seq_
 int md_sdpa_masked(md_ctx* ctx, const uint16_t* q, const uint16_t* k, const uint16_t* v, const uint8_t* mask,
                    uint16_t* out, size_t n_heads, size_t q_len, size_t kv_len, size_t d) {
     MD_NEED_CTX(ctx);
+    CallScope call(ctx);
     MD_NEED(ctx, q && k && v && mask && out, "sdpa_masked: null tensor pointer");
     MD_NEED(ctx, n_heads && q_len && kv_len && d, "sdpa_masked: zero-sized dimension");
     md_arg Q, Kk, V, Mk, O;
@@ -668,6 +689,7 @@ int md_sdpa_masked(md_ctx* ctx, const uint16_t* q, const uint16_t* k, const uint
 int md_sdpa_single(md_ctx* ctx, const uint16_t* q, const uint16_t* k, const uint16_t* v, const uint8_t* mask,
                    uint16_t* out, size_t kv_len) {
     MD_NEED_CTX(ctx);
+    CallScope call(ctx);
     MD_NEED(ctx, q && k && v && mask && out, "sdpa_single: null tensor pointer");
     MD_NEED(ctx, kv_len > 0, "sdpa_single: kv_len is 0");
     if (kv_len > 2048) return md_fail(ctx, MD_ERR_SEQUENCE_TOO_LONG, "sdpa_single: kv_len %zu > 2048", kv_len);
@@ -686,6 +708,7 @@ int md_sdpa_decode_fused(md_ctx* ctx, const uint16_t* qkv_row, uint16_t* key_cac
                          uint16_t* out, size_t n_heads, size_t head_dim, size_t max_seq, size_t pos, size_t rot_dim,
                          float theta) {
     MD_NEED_CTX(ctx);
+    CallScope call(ctx);
     MD_NEED(ctx, qkv_row && key_cache && value_cache && out, "sdpa_decode_fused: null tensor pointer");
     if (pos >= max_seq) return md_fail(ctx, MD_ERR_SEQUENCE_TOO_LONG, "decode: position %zu >= cache size %zu", pos, max_seq);
     if (rot_dim > head_dim || (rot_dim & 1)) return md_fail(ctx, MD_ERR_INVALID_ROT_DIM, "decode: rot_dim %zu", rot_dim);
@@ -697,6 +720,7 @@ int md_sdpa_prefill_fused(md_ctx* ctx, const uint16_t* qkv, uint16_t* key_cache,
                           size_t S, size_t n_heads, size_t head_dim, size_t max_seq, size_t pos, size_t rot_dim,
                           float theta) {
     MD_NEED_CTX(ctx);
+    CallScope call(ctx);
     MD_NEED(ctx, qkv && key_cache && value_cache && out, "sdpa_prefill_fused: null tensor pointer");
     MD_NEED(ctx, S > 0, "sdpa_prefill_fused: S is 0");
     if (pos + S > max_seq)
@@ -715,6 +739,7 @@ int md_sdpa_prefill_fused(md_ctx* ctx, const uint16_t* qkv, uint16_t* key_cache,
 int md_sdpa_vit_fused(md_ctx* ctx, const uint16_t* qkv, uint16_t* out, size_t crops, size_t tokens, size_t n_heads,
                       size_t head_dim) {
     MD_NEED_CTX(ctx);
+    CallScope call(ctx);
     MD_NEED(ctx, qkv && out, "sdpa_vit_fused: null tensor pointer");
     MD_NEED(ctx, crops && tokens && n_heads && head_dim, "sdpa_vit_fused: zero-sized dimension");
     const size_t hd = n_heads * head_dim;

@@ -99,6 +99,7 @@ struct md_ctx {
     int stack_trace = 0;     // md_set_option("stack_trace"): md_text_step keeps the residual stream after every layer
     int fused_decode = 1;    // md_set_option("fused_decode"): decode layers as 3 fused kernels
     int pdl = 0;             // md_set_option("pdl"): programmatic dependent launch for the GEMV kernels
+    bool pdl_late = false;   // while pdl is on: no kernel may read anything ahead of its dependency wait (md_launch_early)
     int prefill_fork = 1;       // md_set_option("prefill_fork"): prefill layers run the MLP beside the attention
     int decode_split_ln = 5;    // md_set_option("decode_split_ln"): from this many rows on a decode step runs the LayerNorm once
     int decode_chain = 1;       // md_set_option("decode_chain"): a decode layer runs as three kernels of one chain; setting decode_fork
@@ -114,6 +115,10 @@ struct md_ctx {
     cudaEvent_t ev_fork = nullptr, ev_side = nullptr, ev_mlp[3] = {};
     int attn_tc = -1;        // md_set_option("attn_tc"): -1 auto, 0 mma.sync attention only, 1 tcgen05 attention only
 };
+
+// May a kernel request weights and caches before its dependency wait?  In the model runners, whose weights nothing on the stream
+// writes; not in a call of its own, whose operands may be what the call before it is still writing.
+inline int md_launch_early(const md_ctx* ctx) { return ctx->pdl_late ? 0 : 1; }
 
 int md_fail(md_ctx* ctx, int status, const char* fmt, ...);
 #define MD_CUDA(ctx, expr)                                                                      \

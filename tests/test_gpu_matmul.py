@@ -405,3 +405,39 @@ def test_pinned_host_operands_equal_pageable_ones(ctx, oracle, m, k, n):
         ctx._check(ctx.lib.md_hgemm_nt(ctx.h, C.c_void_p(view.data_ptr()), C.c_void_p(dbt.ptr),
                                        C.c_void_p(out.data_ptr()), sz(m), sz(n), sz(k)))
         np.testing.assert_array_equal(out.numpy(), want, err_msg=f"pinned operands, offset {off}")
+
+
+@pytest.mark.parametrize("rows", [1, 8, 40, 300])
+@pytest.mark.parametrize("layout", ["nt", "nn"])
+def test_back_to_back_calls_whose_weights_are_the_call_before(ctx, rows, layout):
+    """A call may use as weights (or as keys and values) what the call before it on the stream is still writing: every kernel waits
+    for its predecessor before it reads anything.  Against the same calls with a synchronise after each; the weights change from turn
+    to turn, so that a read of the old ones cannot pass."""
+    rng = np.random.default_rng(rows)
+    K, N, big = 1024, 2048, 1536
+    x = ctx.upload(f16_normal(rng, (rows, K)))
+    p, q = [ctx.upload(f16_normal(rng, (2048, big), 0.03)) for _ in range(3)], ctx.upload(f16_normal(rng, (1024, big), 0.03))
+    shape = (N, K) if layout == "nt" else (K, N)
+    outs, keys = {}, {}
+    for wait in (True, False):
+        w, y, s = ctx.alloc(shape), [ctx.alloc((rows, N)) for _ in p], [ctx.alloc((32, 1, 64)) for _ in p]
+        mask = ctx.upload(np.ones(1024, np.uint8))
+        ctx.sync()
+        for i, a in enumerate(p):
+            def step(call, *args, **kw):
+                call(*args, **kw)
+                if wait:
+                    ctx.sync()
+            step(ctx.hgemm_nt, *((a, q) if layout == "nt" else (q, a)), shape[0], shape[1], big, out=w)
+            step(ctx.hgemm_nt if layout == "nt" else ctx.hgemm_nn, x, w, rows, N, K, out=y[i])
+            step(ctx.hgemm_nt, *((a, q) if layout == "nt" else (q, a)), shape[0], shape[1], big, out=w)
+            step(ctx.sdpa_single, x, w, w, mask, 1024, out=s[i]) if rows * K >= 2048 else None
+        outs[wait] = [b.numpy() for b in y]
+        keys[wait] = [b.numpy() for b in s] if rows * K >= 2048 else []
+        for b in [w, mask] + y + s:
+            b.free()
+    for a, b in zip(outs[True] + keys[True], outs[False] + keys[False]):
+        np.testing.assert_array_equal(a, b)
+    assert not np.array_equal(outs[True][0], outs[True][1])
+    for b in [x, q] + p:
+        b.free()
