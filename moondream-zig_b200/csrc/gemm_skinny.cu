@@ -281,6 +281,17 @@ bool md_gemm_skinny_supported(const void* a, const void* b, const void* c, size_
     return N <= (1u << 30) && K <= (1u << 30);
 }
 
+// Against the general kernel's tiles of 64 columns.  That one takes 0.25 us per k-block whatever its bytes (the issuing thread's
+// waits, MMAs and commit) behind 3 us, rounds over the SMs one after the other; this one reads K in parts and pays for adding them up
+// with the rows: 64 rows of 8192 x 2048 take 13.7 us here and 11.4 there, 16 rows 11.1 and 12.5; 64 rows of 12800 x 512 11.6 and 7.4,
+// of 4096 x 2048 10.3 and 11.0, of 2048 x 8192 13.8 and 32.7, of 16384 x 4096 30.8 and 35.4.  The lines are where the two met on 63
+// shapes (9 to 64 rows of nine matrices).
+bool md_gemm_skinny_wanted(const md_ctx* ctx, size_t M, size_t N, size_t K) {
+    if (ctx->skinny_splits >= 0) return true;
+    const size_t tiles = (N + 63) / 64, rounds = (tiles + ctx->sm_count - 1) / ctx->sm_count, kblocks = (K + BLOCK_K - 1) / BLOCK_K;
+    return M < 32 || tiles < 96 || rounds * kblocks > 32;
+}
+
 namespace {
 
 typedef void (*skinny_fn)(CUtensorMap, CUtensorMap, __half*, int, int, int, int, int, int, md_epilogue, md_devflags*, md_lin);

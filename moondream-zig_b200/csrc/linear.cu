@@ -91,7 +91,7 @@ int md_linear(md_ctx* ctx, int dtype, const void* a, const void* w, void* c, siz
             return MD_OK;
         }
         if ((N % 8) == 0 && !ep.out_f32) {
-            if (!ep.tile_expert && ctx->skinny && md_gemm_skinny_supported(a, w, c, M, N, K))
+            if (!ep.tile_expert && ctx->skinny && md_gemm_skinny_supported(a, w, c, M, N, K) && md_gemm_skinny_wanted(ctx, M, N, K))
                 return md_launch_gemm_skinny_lin(ctx, a, w, c, M, N, K, ep);
             return md_launch_gemm_tc_lin(ctx, a, w, c, M, N, K, ep);
         }

@@ -77,7 +77,8 @@ struct md_ctx {
     uint32_t pair_configured = 0;  // the same for the instantiations of gemm_pair_kernel
     uint32_t tc_configured = 0;  // tcgen05 kernels whose dynamic shared memory limit has been raised
     int skinny = 1;          // md_set_option("skinny"): 8 < M <= 64 takes the swapped-operand split-K kernel
-    int skinny_splits = 0;   // md_set_option("skinny_splits"): 0 = automatic, else the number of K splits (tests)
+    int skinny_splits = -1;  // md_set_option("skinny_splits"): -1 = by shape, where the shape wants that kernel; otherwise it is taken
+                             // wherever it can be, with an automatic (0) or this number of K splits
     bool sdpa_mma_configured = false;  // the same for the mma.sync attention kernels
     // (cos, sin) table shared by the fused attention calls: [rope_rows][rope_dim/2][2] f32
     float* rope_tab = nullptr;
@@ -254,6 +255,7 @@ int md_launch_gather_colblocks(md_ctx* ctx, const uint16_t* gathered, uint16_t* 
 
 // gemm_skinny.cu: 8 < M <= 64, weights as the MMA's M side, split-K over a thread-block cluster
 bool md_gemm_skinny_supported(const void* a, const void* b, const void* c, size_t M, size_t N, size_t K);
+bool md_gemm_skinny_wanted(const md_ctx* ctx, size_t M, size_t N, size_t K);   // rather than the general kernel
 int md_launch_gemm_skinny(md_ctx* ctx, const __half* a, const __half* b, __half* c, size_t M, size_t N, size_t K,
                           int b_layout, const md_epilogue& ep);
 

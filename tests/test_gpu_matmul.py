@@ -441,3 +441,16 @@ def test_back_to_back_calls_whose_weights_are_the_call_before(ctx, rows, layout)
     assert not np.array_equal(outs[True][0], outs[True][1])
     for b in [x, q] + p:
         b.free()
+
+
+@pytest.mark.parametrize("m,n,k,general", [(64, 8192, 2048, True), (32, 6152, 2048, True), (31, 8192, 2048, False), (64, 6080, 2048, False),
+                                           (40, 8192, 2056, False), (33, 9480, 1032, False), (48, 9480, 1016, True)])
+def test_few_rows_take_the_faster_of_two_kernels(pkg, oracle, m, n, k, general):
+    """9 to 64 rows: which of the two kernels a shape takes, on both sides of each line, and its result."""
+    ctx = pkg.Context(0)
+    rng = np.random.default_rng(m + n)
+    a, w = f16_normal(rng, (m, k)), f16_normal(rng, (n, k), 0.05)
+    got = ctx.hgemm_nt(a, w, m, n, k)
+    assert (ctx.get_option("last_tc_tile") < 1000) == general
+    assert_close_ref(got, oracle.hgemm_nt(a, w), f"{m}x{n}x{k}")
+    ctx.close()
