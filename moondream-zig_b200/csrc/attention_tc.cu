@@ -640,7 +640,7 @@ bool plan_map(MapPlan& mp, size_t d, const size_t extent[3], const size_t stride
 template <int D, bool MASKED>
 int launch_attn_tc(md_ctx* ctx, const AttnTcMaps& maps, const AttnTcParams& p, dim3 grid) {
     auto kern = attn_tc_kernel<D, MASKED>;
-    const uint32_t cfg_bit = 1u << ((D == 64 ? 8 : 9) + (MASKED ? 8 : 0));
+    const uint32_t cfg_bit = 1u << ((D == 64 ? 8 : 9) + (MASKED ? 16 : 0));   // 16 .. 21, 27 and 28 are gemm_tc.cu's with peers
     if (!(ctx->tc_configured & cfg_bit)) {
         MD_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnCfg<D>::SMEM));
         ctx->tc_configured |= cfg_bit;

@@ -108,3 +108,24 @@ def test_gather_colblocks(ctx):
     ctx._check(ctx.lib.md_gather_colblocks(ctx.h, C.c_void_p(dg.ptr), C.c_void_p(dc.ptr), _sz(world), _sz(M), _sz(n)))
     ctx.sync()
     np.testing.assert_array_equal(dc.numpy(), g.transpose(1, 0, 2).reshape(M, world * n))
+
+
+def test_push_after_masked_attention_in_one_context(pkg, oracle):
+    """Kernels whose shared memory limit has been raised are remembered by one bit each: the masked attention's must not stand for
+    the column-split product's 128 x 256 tile."""
+    ctx = pkg.Context(0)
+    rng = np.random.default_rng(3)
+    q, k, v = (ctx.upload(f16_normal(rng, (2, 96, 64))) for _ in range(3))
+    mask, out = ctx.upload(np.tril(np.ones((96, 96), np.uint8))), ctx.alloc((2, 96, 64))
+    ctx.sdpa_masked(q, k, v, mask, 2, 96, 96, 64, out=out)
+    M, K, N = 256, 128, 512
+    a, b = f16_normal(rng, (M, K)), f16_normal(rng, (N, K), 0.05)
+    cs = [ctx.upload(np.zeros((M, N), np.float16)) for _ in range(2)]
+    da, db = ctx.upload(a), ctx.upload(b)
+    ctx.set_option("tc_block_n", 256)
+    ctx.set_option("tc_pair", 0)
+    _push(ctx, da, db, cs[0], M, N, K, 1, N, 0, [cs[1]])
+    ctx.sync()
+    for c in cs:
+        assert_close_ref(c.numpy(), oracle.hgemm_nt(a, b), "after masked attention")
+    ctx.close()
