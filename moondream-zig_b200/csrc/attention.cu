@@ -908,8 +908,8 @@ decode_out_kernel(const __grid_constant__ OutParams p) {
         xv[u] = g < p.M ? __ldcg(reinterpret_cast<const uint4*>(p.x + (size_t)g * OUT_K + (warp + u * MIX_WARPS) * 32 + t * 8))
                         : make_uint4(0, 0, 0, 0);
     const int o_m = tid >> 4, o_n = row0 + (tid & 15);
-    md_epilogue_ops ops;
-    if (o_m < p.M) ops = md_epilogue_fetch(p.ep, o_m, o_n, p.N);
+    md_end_ops ops;
+    if (o_m < p.M) ops = md_end_fetch(p.ep, o_m, o_n, p.N);
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int u = 0; u < PIECES; ++u) {
@@ -925,7 +925,7 @@ decode_out_kernel(const __grid_constant__ OutParams p) {
         float v = 0.f;
 #pragma unroll
         for (int q = 0; q < MIX_WARPS; ++q) v += sums[q][tid & 15][o_m];
-        p.out[(size_t)o_m * p.N + o_n] = __float2half_rn(md_epilogue_apply(p.ep, ops, v));
+        p.out[(size_t)o_m * p.N + o_n] = __float2half_rn(md_end_apply(ops, v));
     }
 }
 
@@ -1219,7 +1219,8 @@ int md_launch_decode_mix_out(md_ctx* ctx, const __half* qkv, size_t qkv_stride, 
                              size_t batch, size_t n_heads, size_t d, size_t max_seq, const int* const* pos_dev, size_t rot_dim, float theta,
                              const __half* x, const __half* w, float* part, size_t N, size_t K, size_t parts, const __half* w_out,
                              __half* out, const md_epilogue& ep) {
-    if (!md_decode_mix_supported(batch, n_heads, d, N, K) || rot_dim > DEC_D)
+    if (!md_decode_mix_supported(batch, n_heads, d, N, K) || rot_dim > DEC_D || !ep.bias || !ep.parts || !ep.bias2 || !ep.residual2 ||
+        ep.gelu || ep.residual)
         return md_fail(ctx, MD_ERR_UNSUPPORTED, "decode_mix_out: unsupported shape");
     MixParams p{};
     MD_TRY(decode_batch_params(ctx, p.a, qkv, qkv_stride, kc, vc, attn, OUT_K, batch, n_heads, d, max_seq, pos_dev, rot_dim, theta));

@@ -351,35 +351,35 @@ __device__ __forceinline__ float md_apply_epilogue(float acc, float bias, bool h
 }
 
 // The fused glue for output element (m, n): f16(acc) -> +bias -> gelu -> +residual -> +residual2, one
-// rounding to f16 after every step, exactly where the reference's separate ops round.  In two halves, so that a kernel can request
-// what the glue reads ahead of its sums.
-struct md_epilogue_ops { float bias, residual, part, bias2, residual2; };
-__device__ __forceinline__ md_epilogue_ops md_epilogue_fetch(const md_epilogue& ep, int m, int n, int N) {
-    md_epilogue_ops o = {0.f, 0.f, 0.f, 0.f, 0.f};
-    if (ep.bias) o.bias = __half2float(ep.bias[n]);
+// rounding to f16 after every step, exactly where the reference's separate ops round.
+__device__ __forceinline__ float md_epilogue_value(const md_epilogue& ep, float acc, int m, int n, int N) {
+    float v = md_round_f16(acc);
+    if (ep.bias) v = md_round_f16(v + __half2float(ep.bias[n]));
+    if (ep.gelu) v = md_round_f16(md_gelu_f32(v));
     if (ep.residual) {
         const int rm = ep.residual_rows > 0 ? m % ep.residual_rows : m;
-        o.residual = __half2float(__ldcg(ep.residual + (size_t)rm * N + n));
+        v = md_round_f16(v + __half2float(__ldcg(ep.residual + (size_t)rm * N + n)));
     }
     if (ep.parts) {
-#pragma unroll 4
-        for (int i = 0; i < ep.n_parts; ++i) o.part += __ldcg(ep.parts + (size_t)i * ep.part_stride + (size_t)m * N + n);
-        o.bias2 = __half2float(ep.bias2[n]);
+        // the other projection arrives as parts of its K sum: one rounding of the sum, then its bias
+        float r = 0.f;
+        for (int i = 0; i < ep.n_parts; ++i) r += __ldcg(ep.parts + (size_t)i * ep.part_stride + (size_t)m * N + n);
+        r = md_round_f16(md_round_f16(r) + __half2float(ep.bias2[n]));
+        v = md_round_f16(v + r);
     }
-    if (ep.residual2) o.residual2 = __half2float(__ldcg(ep.residual2 + (size_t)m * N + n));
-    return o;
-}
-__device__ __forceinline__ float md_epilogue_apply(const md_epilogue& ep, const md_epilogue_ops& o, float acc) {
-    float v = md_round_f16(acc);
-    if (ep.bias) v = md_round_f16(v + o.bias);
-    if (ep.gelu) v = md_round_f16(md_gelu_f32(v));
-    if (ep.residual) v = md_round_f16(v + o.residual);
-    // the other projection arrives as parts of its K sum: one rounding of the sum, then its bias
-    if (ep.parts) v = md_round_f16(v + md_round_f16(md_round_f16(o.part) + o.bias2));
-    if (ep.residual2) v = md_round_f16(v + o.residual2);
+    if (ep.residual2) v = md_round_f16(v + __half2float(__ldcg(ep.residual2 + (size_t)m * N + n)));
     return v;
 }
-__device__ __forceinline__ float md_epilogue_value(const md_epilogue& ep, float acc, int m, int n, int N) {
-    return md_epilogue_apply(ep, md_epilogue_fetch(ep, m, n, N), acc);
+// The glue of a product that ends a layer (bias, parts, residual2) in two halves, so that what it reads is requested ahead of the sums.
+struct md_end_ops { float bias, part, bias2, residual2; };
+__device__ __forceinline__ md_end_ops md_end_fetch(const md_epilogue& ep, int m, int n, int N) {
+    md_end_ops o = {__half2float(ep.bias[n]), 0.f, __half2float(ep.bias2[n]), __half2float(__ldcg(ep.residual2 + (size_t)m * N + n))};
+#pragma unroll 4
+    for (int i = 0; i < ep.n_parts; ++i) o.part += __ldcg(ep.parts + (size_t)i * ep.part_stride + (size_t)m * N + n);
+    return o;
+}
+__device__ __forceinline__ float md_end_apply(const md_end_ops& o, float acc) {
+    const float v = md_round_f16(md_round_f16(acc) + o.bias), r = md_round_f16(md_round_f16(o.part) + o.bias2);
+    return md_round_f16(md_round_f16(v + r) + o.residual2);
 }
 #endif
