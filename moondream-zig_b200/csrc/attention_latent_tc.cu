@@ -89,7 +89,6 @@ latent_tc_kernel(const __grid_constant__ LatTcMaps tm, const LatTcParams p, md_d
     volatile int* abort_flag = reinterpret_cast<volatile int*>(bars_ptr + 244);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    md_pdl_launch_dependents();
     if (threadIdx.x == 0) {
         tma_prefetch_map(&tm.qn);
         tma_prefetch_map(&tm.qr);
@@ -121,6 +120,7 @@ latent_tc_kernel(const __grid_constant__ LatTcMaps tm, const LatTcParams p, md_d
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    md_pdl_launch_dependents();   // only now that the columns are allocated
     md_pdl_wait();
 
     // Every role walks the same items in the same order.  Ring slots, the S / P buffer of a tile and the wait parities run on

@@ -221,7 +221,6 @@ attn_tc_kernel(const __grid_constant__ AttnTcMaps tm, AttnTcParams p, md_devflag
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-    md_pdl_launch_dependents();
     if (threadIdx.x == 0) {
         // the descriptors are kernel parameters: fetching them does not depend on the predecessor kernel
         tma_prefetch_map(&tm.q);
@@ -263,6 +262,7 @@ attn_tc_kernel(const __grid_constant__ AttnTcMaps tm, AttnTcParams p, md_devflag
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    md_pdl_launch_dependents();   // only now that the columns are allocated
     md_pdl_wait();
 
     // Every role walks the same items in the same order.  Ring slots, the S / P buffer of a tile and the wait

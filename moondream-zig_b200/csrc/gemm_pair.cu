@@ -121,7 +121,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     const int num_kb = (K + BLOCK_K - 1) / BLOCK_K;
     const int tiles_n = num_tiles / tiles_m;
 
-    md_pdl_launch_dependents();
     if (threadIdx.x == 0) {
         tma_prefetch_map(&tm_a);
         tma_prefetch_map(&tm_b);
@@ -151,6 +150,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     cluster_sync_all();   // both CTAs' barriers are initialised before anyone signals them remotely
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    md_pdl_launch_dependents();   // only now that the columns are allocated
     md_pdl_wait();
 
     if (warp == 0) {

@@ -62,7 +62,6 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     const int kb0 = split * kb_per_split;
     const int kbs = max(0, min(kb_per_split, num_kb - kb0));   // 0 for a split past the end of K: it contributes zeros
 
-    md_pdl_launch_dependents();
     if (threadIdx.x == 0) {
         tma_prefetch_map(&tm_w);
         tma_prefetch_map(&tm_x);
@@ -85,6 +84,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    md_pdl_launch_dependents();   // only now that the columns are allocated
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer

@@ -131,9 +131,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     const int kb_per = (num_kb + splits - 1) / splits;
     volatile int* last_flag = reinterpret_cast<volatile int*>(bars_ptr + 16 * STAGES + 40 + 4 * EPI_WARPS);
 
-    // programmatic dependent launch: the successor may start its own set-up now; this kernel sets up its
-    // barriers and tensor memory, then waits for its predecessor before any global access
-    md_pdl_launch_dependents();
+    // programmatic dependent launch: this kernel sets up its barriers and tensor memory, lets its successor start, then
+    // waits for its predecessor before any global access
     if (threadIdx.x == 0) {
         // the descriptors are kernel parameters: fetching them does not depend on the predecessor kernel
         tma_prefetch_map(&tm_a);
@@ -162,6 +161,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    md_pdl_launch_dependents();   // only now that the columns are allocated
     md_pdl_wait();
     const bool grouped = BF16 && MT == 1 && lin.tile_expert != nullptr;
     if (grouped) {

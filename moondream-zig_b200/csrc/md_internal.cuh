@@ -158,6 +158,9 @@ int md_launch_ex(md_ctx* ctx, void (*kern)(KArgs...), dim3 grid, dim3 block, siz
     return MD_OK;
 }
 // Device side of the protocol: let the successor start its prologue, then wait for the predecessor.
+// A kernel that owns tensor memory lets its successor start behind its own allocation, never ahead of it: the successor's CTAs
+// start once every CTA of this grid has said so, and one that took the columns first would hold them until this grid ends, while
+// this grid's allocation waits for them.
 __device__ __forceinline__ void md_pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void md_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 #endif
