@@ -98,7 +98,10 @@ __device__ __forceinline__ int attn_walk(const AttnTcParams& p, int it) {
     const long long w = (long long)it * gridDim.x + c;
     return w < p.n_items ? (int)w : -1;
 }
-// Number of key tiles of a query block, and the first of them.
+// Number of key tiles of a query block, and the first of them.  Never none: a query block whose mask is all zero walks one tile and
+// sees nothing of it.  The roles' waits by parity are only sound while nobody is more than one phase ahead; at an item without
+// tiles nothing would hold the issuer of the S products, whose next wait for Q would pass on the phase before, or hold the softmax
+// warps back for it, whose two phases it would miss.
 template <bool MASKED>
 __device__ __forceinline__ int attn_tiles(const AttnTcParams& p, int qblk, int& first) {
     first = 0;
@@ -110,7 +113,7 @@ __device__ __forceinline__ int attn_tiles(const AttnTcParams& p, int qblk, int& 
             lo = min(lo, s.x);
             hi = max(hi, s.y);
         }
-        if (lo >= hi) return 0;
+        if (lo >= hi) return 1;
         first = lo;
         return hi - lo;
     }
@@ -567,6 +570,7 @@ attn_tc_kernel(const __grid_constant__ AttnTcMaps tm, AttnTcParams p, md_devflag
             if (lane == 0) tma_store_wait_read<0>();   // the previous item's store has read the staging rows
             __syncwarp();
             const float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
+            const bool unseen = MASKED && l_run == 0.f;   // a row that sees no key: zeros, whatever the tile's values hold
 #pragma unroll
             for (int c = 0; c < Cfg::DPAD / 16; ++c) {
 #pragma unroll
@@ -575,8 +579,8 @@ attn_tc_kernel(const __grid_constant__ AttnTcMaps tm, AttnTcParams p, md_devflag
                         uint32_t wv[4];
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
-                            const __half2 h = __floats2half2_rn(__uint_as_float(o[c][h8 * 8 + 2 * e]) * inv,
-                                                                __uint_as_float(o[c][h8 * 8 + 2 * e + 1]) * inv);
+                            const __half2 h = __floats2half2_rn(unseen ? 0.f : __uint_as_float(o[c][h8 * 8 + 2 * e]) * inv,
+                                                                unseen ? 0.f : __uint_as_float(o[c][h8 * 8 + 2 * e + 1]) * inv);
                             wv[e] = *reinterpret_cast<const uint32_t*>(&h);
                         }
                         *reinterpret_cast<uint4*>(stage_row + (c * 16 + h8 * 8) * 2) = make_uint4(wv[0], wv[1], wv[2], wv[3]);

@@ -151,6 +151,45 @@ def test_ctas_that_walk_several_items_give_the_same_result(ctx, oracle, per_sm):
         np.testing.assert_array_equal(got2, _WALK[0][1])
 
 
+_MASKED_WALK: dict = {}
+
+
+@pytest.mark.parametrize("per_sm", [0, 1, 2])
+def test_masked_ctas_that_walk_over_unseen_query_blocks(ctx, oracle, per_sm):
+    """Masked items of one CTA's walk over different spans of keys: whole 128-row blocks that see nothing stand first, last, alone and
+    three in a row.  56 heads of 12 blocks are 672 items, 4 or 5 per CTA (per_sm 1), 2 or 3 (per_sm 2) or one (per_sm 0).  They
+    must not put the roles' barriers out of step: against the oracle, zeros where nothing is seen (the first keys, which only an
+    unseen block's one tile visits, have infinite values), three launches in a row and all three grids bit for bit."""
+    H, lq, lk = 56, 1500, 700
+    rng = np.random.default_rng(31)
+    q, k, v = f16_normal(rng, (H, lq, 64)), f16_normal(rng, (H, lk, 64)), f16_normal(rng, (H, lk, 64))
+    m = (rng.random((lq, lk)) < 0.6).astype(np.uint8)
+    for b in range(12):
+        rows = m[b * 128:(b + 1) * 128]
+        lo = 64 + (b * 61) % 450
+        rows[:, :lo] = 0
+        rows[:, lo + 90 + 20 * b:] = 0
+        rows[:, lo] = 1
+        if b in (0, 3, 4, 5, 8, 11):
+            rows[:] = 0
+    v[:, :64] = np.inf
+    ctx.set_option("attn_tc", 1)
+    ctx.set_option("attn_ctas_per_sm", per_sm)
+    try:
+        got = [ctx.sdpa_masked(q, k, v, m, H, lq, lk, 64) for _ in range(3)]
+    finally:
+        ctx.set_option("attn_ctas_per_sm", 2)
+        ctx.set_option("attn_tc", -1)
+    for again in got[1:]:
+        np.testing.assert_array_equal(again, got[0])
+    seen = m.any(1)
+    assert (got[0][:, ~seen] == 0).all()
+    if not _MASKED_WALK:
+        _MASKED_WALK["ref"] = oracle.sdpa_masked(q, k[:, 64:].copy(), v[:, 64:].copy(), m[:, 64:].copy())[:, seen]
+    assert_close_ref(got[0][:, seen], _MASKED_WALK["ref"], "unseen query blocks")
+    np.testing.assert_array_equal(got[0], _MASKED_WALK.setdefault("first", got[0]))
+
+
 def test_forced_tcgen05_rejects_other_head_dims(ctx, pkg):
     ctx.set_option("attn_tc", 1)
     try:
