@@ -619,7 +619,7 @@ int md_launch_gemm_tc_ex(md_ctx* ctx, const __half* a, const __half* b, __half* 
         return md_fail(ctx, MD_ERR_UNSUPPORTED, "tcgen05 GEMM: the output row stride must be a multiple of 8 and >= N");
     if (ldc != N && (ep.residual || ep.residual2))
         return md_fail(ctx, MD_ERR_UNSUPPORTED, "tcgen05 GEMM: residuals are not supported with a strided output");
-    if (!md_gemm_tc_supported(a, b, c, M, N, K, b_layout))
+    if (!md_gemm_tc_supported(a, b, c, M, N, K, b_layout) || !md_glue_aligned(ep))
         return md_fail(ctx, MD_ERR_UNSUPPORTED, "tcgen05 GEMM needs K %% 8 == 0, N %% 8 == 0 and 16-byte aligned operands");
     // Tile shape.  The kernel is bound by the bytes an SM pulls from L2 per k-block, (rows + columns) x 128,
     // so a tile's time is proportional to its rows + columns: 128 x 64, 128 x 128, 128 x 256, or 256 x 256 (two

@@ -212,6 +212,11 @@ struct md_epilogue {
     const __half* bias2 = nullptr;
 };
 
+// The tcgen05 kernels' epilogue reads bias and residuals eight at a time (N % 8 == 0); the others read them one by one.
+inline bool md_glue_aligned(const md_epilogue& ep) {
+    return ((reinterpret_cast<uintptr_t>(ep.bias) | reinterpret_cast<uintptr_t>(ep.residual) | reinterpret_cast<uintptr_t>(ep.residual2)) & 15) == 0;
+}
+
 // Column-split GEMM: finished C chunks are also stored into the other GPUs' buffers.
 struct md_push {
     int n = 0;                 // number of peers (0 = none)

@@ -454,3 +454,28 @@ def test_few_rows_take_the_faster_of_two_kernels(pkg, oracle, m, n, k, general):
     assert (ctx.get_option("last_tc_tile") < 1000) == general
     assert_close_ref(got, oracle.hgemm_nt(a, w), f"{m}x{n}x{k}")
     ctx.close()
+
+
+@pytest.mark.parametrize("bytes_off", [2, 4, 8, 16])
+@pytest.mark.parametrize("m,n,k", [(7, 512, 256), (40, 512, 256), (64, 8192, 512), (65, 512, 256), (300, 1032, 520)])
+def test_glue_operands_at_any_address(pkg, oracle, m, n, k, bytes_off):
+    """Bias and residual may be slices of larger tensors: at 2, 4, 8 and 16 bytes past a 16-byte boundary, one or both of them, for
+    the row counts of every kernel; the tcgen05 kernels (which read them 16 bytes at a time) must not be given the first three."""
+    ctx = pkg.Context(0)
+    rng = np.random.default_rng(m + n)
+    a, w = f16_normal(rng, (m, k)), f16_normal(rng, (n, k), 0.05)
+    bias, res = f16_normal(rng, (n,), 0.5), f16_normal(rng, (m, n))
+    ref = oracle.add(oracle.bias_add(oracle.hgemm_nt(a, w), bias), res)
+    pad = np.zeros(bytes_off // 2, np.float16)
+    da, dw, out = ctx.upload(a), ctx.upload(w), ctx.alloc((m, n))
+    even = [ctx.upload(x).ptr for x in (bias, res)]
+    moved = [ctx.upload(np.concatenate([pad, x.ravel()])).ptr + bytes_off for x in (bias, res)]
+    for b, r in ((moved[0], even[1]), (even[0], moved[1]), (moved[0], moved[1])):
+        ctx.hgemm_fused(da, dw, out, m, n, k, 1, bias=b, residual=r)
+        ctx.sync()
+        assert_close_ref(out.numpy(), ref, f"{m}x{n}x{k}, {bytes_off} bytes off")
+    if bytes_off < 16 and m > 8:
+        ctx.set_gemm_mode(2)     # the tcgen05 kernel asked for by name: refused, not run
+        with pytest.raises(pkg.MdError):
+            ctx.hgemm_fused(da, dw, out, m, n, k, 1, bias=moved[0])
+    ctx.close()
