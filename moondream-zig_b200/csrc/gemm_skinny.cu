@@ -286,8 +286,10 @@ bool md_gemm_skinny_supported(const void* a, const void* b, const void* c, size_
 // with the rows: 64 rows of 8192 x 2048 take 13.7 us here and 11.4 there, 16 rows 11.1 and 12.5; 64 rows of 12800 x 512 11.6 and 7.4,
 // of 4096 x 2048 10.3 and 11.0, of 2048 x 8192 13.8 and 32.7, of 16384 x 4096 30.8 and 35.4.  The lines are where the two met on 63
 // shapes (9 to 64 rows of nine matrices).
-bool md_gemm_skinny_wanted(const md_ctx* ctx, size_t M, size_t N, size_t K) {
-    if (ctx->skinny_splits >= 0) return true;
+// A fused GELU stays here: this epilogue has tanhf, the general one the hardware's tanh, whose error of 2^-11 is up to 15 places of
+// the f16 result at -2, where tanh is near -1 and the GELU is what is left of it.
+bool md_gemm_skinny_wanted(const md_ctx* ctx, size_t M, size_t N, size_t K, bool gelu) {
+    if (ctx->skinny_splits >= 0 || gelu) return true;
     const size_t tiles = (N + 63) / 64, rounds = (tiles + ctx->sm_count - 1) / ctx->sm_count, kblocks = (K + BLOCK_K - 1) / BLOCK_K;
     return M < 32 || tiles < 96 || rounds * kblocks > 32;
 }

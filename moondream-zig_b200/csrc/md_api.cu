@@ -539,7 +539,7 @@ int md_gemm_dispatch(md_ctx* ctx, const __half* a, const __half* b, __half* c, s
     if (ctx->gemm_mode != 1 && b_layout == 1 && M <= 8 && (K % 8) == 0 && aligned16 && ctx->gemm_mode != 2)
         return md_launch_gemv_nt(ctx, a, b, c, M, N, K, ep);
     const bool glue_ok = md_glue_aligned(ep);
-    if (ctx->gemm_mode == 0 && ctx->skinny && md_gemm_skinny_supported(a, b, c, M, N, K) && (!glue_ok || md_gemm_skinny_wanted(ctx, M, N, K)))
+    if (ctx->gemm_mode == 0 && ctx->skinny && md_gemm_skinny_supported(a, b, c, M, N, K) && (!glue_ok || md_gemm_skinny_wanted(ctx, M, N, K, ep.gelu != 0)))
         return md_launch_gemm_skinny(ctx, a, b, c, M, N, K, b_layout, ep);
     const bool tc_ok = glue_ok && md_gemm_tc_supported(a, b, c, M, N, K, b_layout);
     if (ctx->gemm_mode == 2 && !tc_ok)

@@ -263,7 +263,7 @@ int md_launch_gather_colblocks(md_ctx* ctx, const uint16_t* gathered, uint16_t* 
 
 // gemm_skinny.cu: 8 < M <= 64, weights as the MMA's M side, split-K over a thread-block cluster
 bool md_gemm_skinny_supported(const void* a, const void* b, const void* c, size_t M, size_t N, size_t K);
-bool md_gemm_skinny_wanted(const md_ctx* ctx, size_t M, size_t N, size_t K);   // rather than the general kernel
+bool md_gemm_skinny_wanted(const md_ctx* ctx, size_t M, size_t N, size_t K, bool gelu);   // rather than the general kernel
 int md_launch_gemm_skinny(md_ctx* ctx, const __half* a, const __half* b, __half* c, size_t M, size_t N, size_t K,
                           int b_layout, const md_epilogue& ep);
 

@@ -479,3 +479,31 @@ def test_glue_operands_at_any_address(pkg, oracle, m, n, k, bytes_off):
         with pytest.raises(pkg.MdError):
             ctx.hgemm_fused(da, dw, out, m, n, k, 1, bias=moved[0])
     ctx.close()
+
+
+@pytest.mark.parametrize("layout", [0, 1])
+@pytest.mark.parametrize("m,n,k", [(16, 8192, 2048), (32, 8192, 1024), (64, 8192, 2048), (64, 12800, 512)])
+def test_fused_gelu_of_few_rows_keeps_its_last_places(pkg, m, n, k, layout):
+    """GELU around -2, where 1 + tanh nearly cancels, for up to 64 rows of any shape.  The reference rounds the product and the bias to
+    f16 and then applies the GELU in f32 (ops.zig:1641-1642).  Against 64 bits for the same f16 input: half a place of the f16
+    result (2^-11 of it, 2^-25 below the normal range) and what 32 bits leave of 1 + tanh, two places of tanhf and the roundings
+    around it: 2^-22 over 1 + tanh.  The input itself is taken from the same product without the GELU."""
+    ctx = pkg.Context(0)
+    rng = np.random.default_rng(m + n)
+    a, w = f16_normal(rng, (m, k)), f16_normal(rng, (n, k) if layout else (k, n), 0.05 / np.sqrt(k))
+    bias = (-2.2 + 0.3 * rng.standard_normal(n)).clip(-3, -1).astype(np.float16)
+    da, dw, db, out = ctx.upload(a), ctx.upload(w), ctx.upload(bias), ctx.alloc((m, n))
+    ctx.set_option("skinny_splits", 0)      # one kernel for both calls
+    ctx.hgemm_fused(da, dw, out, m, n, k, layout, bias=db)
+    ctx.sync()
+    x = out.numpy().astype(np.float64)
+    ctx.close()
+    ctx = pkg.Context(0)
+    da, dw, db, out = ctx.upload(a), ctx.upload(w), ctx.upload(bias), ctx.alloc((m, n))
+    ctx.hgemm_fused(da, dw, out, m, n, k, layout, bias=db, gelu=True)
+    ctx.sync()
+    one_plus = 1 + np.tanh(0.7978515625 * (x + 0.044708251953125 * x ** 3))
+    want = 0.5 * x * one_plus
+    err = np.abs(out.numpy().astype(np.float64) - want)
+    assert (err <= np.abs(want) * (2.0 ** -11 + 2.0 ** -22 / one_plus) + 2.0 ** -25).all(), float((err / np.abs(want)).max())
+    ctx.close()
