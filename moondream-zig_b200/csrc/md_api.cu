@@ -538,10 +538,11 @@ int md_gemm_dispatch(md_ctx* ctx, const __half* a, const __half* b, __half* c, s
     const bool aligned16 = ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0;
     if (ctx->gemm_mode != 1 && b_layout == 1 && M <= 8 && (K % 8) == 0 && aligned16 && ctx->gemm_mode != 2)
         return md_launch_gemv_nt(ctx, a, b, c, M, N, K, ep);
-    const bool glue_ok = md_glue_aligned(ep);
-    if (ctx->gemm_mode == 0 && ctx->skinny && md_gemm_skinny_supported(a, b, c, M, N, K) && (!glue_ok || md_gemm_skinny_wanted(ctx, M, N, K, ep.gelu != 0)))
+    const bool tc_ok = md_glue_aligned(ep) && md_gemm_tc_supported(a, b, c, M, N, K, b_layout);
+    // (C and the glue may be aligned well enough for the split-K kernel alone)
+    if (ctx->gemm_mode == 0 && ctx->skinny && md_gemm_skinny_supported(a, b, c, M, N, K) &&
+        (!tc_ok || md_gemm_skinny_wanted(ctx, M, N, K, ep.gelu != 0)))
         return md_launch_gemm_skinny(ctx, a, b, c, M, N, K, b_layout, ep);
-    const bool tc_ok = glue_ok && md_gemm_tc_supported(a, b, c, M, N, K, b_layout);
     if (ctx->gemm_mode == 2 && !tc_ok)
         return md_fail(ctx, MD_ERR_UNSUPPORTED, "tcgen05 GEMM forced but the shape/alignment does not allow it");
     if (ctx->gemm_mode != 1 && tc_ok) return md_launch_gemm_tc(ctx, a, b, c, M, N, K, b_layout, ep);

@@ -507,3 +507,23 @@ def test_fused_gelu_of_few_rows_keeps_its_last_places(pkg, m, n, k, layout):
     err = np.abs(out.numpy().astype(np.float64) - want)
     assert (err <= np.abs(want) * (2.0 ** -11 + 2.0 ** -22 / one_plus) + 2.0 ** -25).all(), float((err / np.abs(want)).max())
     ctx.close()
+
+
+@pytest.mark.parametrize("bytes_off,tile", [(8, 1000), (2, 0), (16, 0)])
+def test_few_rows_into_an_output_of_any_alignment(pkg, oracle, bytes_off, tile):
+    """32 to 64 rows whose general kernel cannot take the output: at 8 bytes past a 16-byte boundary the split-K kernel, and not the
+    one without tensor cores."""
+    ctx = pkg.Context(0)
+    m, n, k = 64, 8192, 1024
+    rng = np.random.default_rng(bytes_off)
+    a, w = f16_normal(rng, (m, k)), f16_normal(rng, (n, k), 0.05)
+    da, dw, out = ctx.upload(a), ctx.upload(w), ctx.upload(np.full(m * n + 16, 7, np.float16))
+    ctx.hgemm_nt(da, dw, m, n, k, out=out.ptr + bytes_off)
+    ctx.sync()
+    if tile:
+        assert ctx.get_option("last_tc_tile") >= tile
+    got = out.numpy()
+    lo = bytes_off // 2
+    assert_close_ref(got[lo:lo + m * n].reshape(m, n), oracle.hgemm_nt(a, w), f"{bytes_off} bytes off")
+    assert (got[:lo] == 7).all() and (got[lo + m * n:] == 7).all()
+    ctx.close()
