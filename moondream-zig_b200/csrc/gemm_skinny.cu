@@ -281,17 +281,21 @@ bool md_gemm_skinny_supported(const void* a, const void* b, const void* c, size_
     return N <= (1u << 30) && K <= (1u << 30);
 }
 
-// Against the general kernel's tiles of 64 columns.  That one takes 0.25 us per k-block whatever its bytes (the issuing thread's
-// waits, MMAs and commit) behind 3 us, rounds over the SMs one after the other; this one reads K in parts and pays for adding them up
-// with the rows: 64 rows of 8192 x 2048 take 13.7 us here and 11.4 there, 16 rows 11.1 and 12.5; 64 rows of 12800 x 512 11.6 and 7.4,
-// of 4096 x 2048 10.3 and 11.0, of 2048 x 8192 13.8 and 32.7, of 16384 x 4096 30.8 and 35.4.  The lines are where the two met on 63
-// shapes (9 to 64 rows of nine matrices).
+// Against the general kernel's tiles of 64 columns, for f16 products.  That one takes 0.2 to 0.25 us per k-block whatever its
+// bytes (the issuing thread's waits, MMAs and commit), rounds over the SMs one after the other, and hardly more for more rows;
+// this one reads K in parts and pays for adding them up with the rows.  So the line is one of rows against rounds * k-blocks.  us here
+// and there, [N, K] weights without glue:
+//   32 rows   8192 x 512: 7.4 and 6.9    x 1024: 9.0 and 9.9                                      16384 x 256: 7.8 and 6.6
+//   48 rows   8192 x 1536: 11.7 and 9.8  x 2560: 14.0 and 13.6  x 4096: 17.7 and 19.6    16384 x 768: 12.4 and 12.0  x 1024: 13.4 and 14.9
+//   64 rows   8192 x 2048: 13.1 and 11.9 x 2560: 14.4 and 13.6  x 3072: 15.5 and 15.7
+// Up to the line (8, 24 and 40 blocks of 32, 48 and 64 rows) the general kernel takes 0.40 to 1.01 of the time here over 5632 to
+// 28416 columns, with bias and residual 0.40 to 1.03.  Narrower matrices stay here: 2048 and 4096 columns meet at 16 and 24 blocks.
 // A fused GELU stays here: this epilogue has tanhf, the general one the hardware's tanh, whose error of 2^-11 is up to 15 places of
 // the f16 result at -2, where tanh is near -1 and the GELU is what is left of it.
 bool md_gemm_skinny_wanted(const md_ctx* ctx, size_t M, size_t N, size_t K, bool gelu) {
     if (ctx->skinny_splits >= 0 || gelu) return true;
     const size_t tiles = (N + 63) / 64, rounds = (tiles + ctx->sm_count - 1) / ctx->sm_count, kblocks = (K + BLOCK_K - 1) / BLOCK_K;
-    return M < 32 || tiles < 96 || rounds * kblocks > 32;
+    return tiles < 96 || rounds * kblocks + 24 > M;
 }
 
 namespace {

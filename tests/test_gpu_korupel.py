@@ -514,3 +514,21 @@ def test_experts_of_a_few_tokens(ctx, mods, width, ff, n):
     cfg = ku.config(width, 40, 1, [ku.attention(2, 1, 16, 20, 0, ku.moe(9, 2, ff))])
     w = ref.random_weights(cfg, width + n)
     compare(ctx, mods, cfg, w, ku.tokens(cfg, n, n), "bfloat16", what=f"width {width}, {n} tokens")
+
+
+def test_prompt_of_few_rows_takes_the_split_k_products(pkg, mods):
+    """bfloat16 products of 9 to 64 rows all take the split-K kernel, wide gated ones with a short K too (the f16 dispatch's line to the
+    general kernel was measured for f16 products): the same logits bit for bit as when it is asked for by name."""
+    cfg = ku.config(512, 40, 1, [ku.attention(4, 2, 32, 40, 0, ku.dense(3200)), ku.lightning(2, 32, 32, ku.dense(4096))])
+    w = ref.random_weights(cfg, 3)
+    toks, got = ku.tokens(cfg, 64), []
+    for asked in (False, True):
+        ctx = pkg.Context(0)
+        if asked:
+            ctx.set_option("skinny_splits", 0)
+        with Model(ctx, mods, cfg, w, "bfloat16") as m:
+            r = m.request()
+            got.append(run(m, r, toks))
+            r.close()
+        ctx.close()
+    np.testing.assert_array_equal(got[0], got[1])

@@ -443,8 +443,9 @@ def test_back_to_back_calls_whose_weights_are_the_call_before(ctx, rows, layout)
         b.free()
 
 
-@pytest.mark.parametrize("m,n,k,general", [(64, 8192, 2048, True), (32, 6152, 2048, True), (31, 8192, 2048, False), (64, 6080, 2048, False),
-                                           (40, 8192, 2056, False), (33, 9480, 1032, False), (48, 9480, 1016, True)])
+@pytest.mark.parametrize("m,n,k,general", [(64, 8192, 2048, True), (64, 8192, 2560, True), (64, 8192, 2568, False), (48, 6152, 1536, True),
+                                           (48, 6152, 1544, False), (32, 6152, 512, True), (32, 6152, 520, False), (31, 6152, 512, False),
+                                           (40, 6080, 512, False), (33, 9480, 256, True), (33, 9480, 264, False)])
 def test_few_rows_take_the_faster_of_two_kernels(pkg, oracle, m, n, k, general):
     """9 to 64 rows: which of the two kernels a shape takes, on both sides of each line, and its result."""
     ctx = pkg.Context(0)
