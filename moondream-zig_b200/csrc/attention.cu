@@ -1095,7 +1095,7 @@ static int decode_loop_launch(md_ctx* ctx, const DecodeParams& p, size_t batch) 
 }
 
 static int decode_launch(md_ctx* ctx, DecodeParams& p) {
-    p.late = !md_launch_early(ctx);
+    p.late = 1;   // a call of its own, whatever "pdl" is set to: keys and values are no weights, and the call before may still write them
     if (decode_loop_wanted(ctx, p, 1)) return decode_loop_launch(ctx, p, 1);
     p.splits = (p.kv_cache_len + DEC_KEYS - 1) / DEC_KEYS;
     if (p.splits < 1) p.splits = 1;

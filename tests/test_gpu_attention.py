@@ -197,3 +197,40 @@ def test_vit_fused_attention(ctx, oracle, crops):
                    for i in range(3)]
         ref = np.ascontiguousarray(oracle.sdpa_maskless(q, k, v).transpose(1, 0, 2)).reshape(T, H * d)
         assert_close_ref(got[c * T:(c + 1) * T], ref, f"vit crop {c}")
+
+
+@pytest.mark.parametrize("loop", [-1, 1], ids=["key splits", "one CTA per head"])
+def test_attention_calls_back_to_back_under_the_pdl_option(pkg, loop):
+    """Option pdl lets products request their weights ahead of the call before them; keys and values are no weights.  Tokens decoded
+    one after the other into one cache (a call reads the key the call before it appends) and sdpa_single over keys that the product
+    before it writes: the same as with a synchronise after each call."""
+    rng = np.random.default_rng(5)
+    H, d, max_seq, start, steps = 32, 64, 1024, 250, 24
+    qkv = f16_normal(rng, (steps, 3 * H * d))
+    kc, vc = f16_normal(rng, (H, max_seq, d)), f16_normal(rng, (H, max_seq, d))
+    w, x = [f16_normal(rng, (2048, 64), 0.3) for _ in range(3)], f16_normal(rng, (4, 64))
+    got = {}
+    for wait in (True, False):
+        ctx = pkg.Context(0)
+        ctx.set_option("pdl", 1)
+        ctx.set_option("decode_loop", loop)
+        rows, dk, dv, out = ctx.upload(qkv), ctx.upload(kc), ctx.upload(vc), ctx.alloc((steps, H * d))
+        dw, dx, q, mask = [ctx.upload(a) for a in w], ctx.upload(x), ctx.upload(qkv[0, :H * d]), ctx.upload(np.ones(4, np.uint8))
+        keys, single = ctx.alloc((4, 2048)), ctx.alloc((steps, H * d))
+        ctx.sync()
+        for i in range(steps):
+            ctx.sdpa_decode_fused(rows.ptr + 2 * i * 3 * H * d, dk, dv, out.ptr + 2 * i * H * d, H, d, max_seq, start + i, 32)
+            if wait:
+                ctx.sync()
+        for i in range(steps):
+            ctx.hgemm_nt(dx, dw[i % 3], 4, 2048, 64, out=keys)
+            if wait:
+                ctx.sync()
+            ctx.sdpa_single(q, keys, keys, mask, 4, out=single.ptr + 2 * i * H * d)
+            if wait:
+                ctx.sync()
+        ctx.sync()
+        got[wait] = out.numpy(), dk.numpy(), single.numpy()
+        ctx.close()
+    for a, b in zip(got[True], got[False]):
+        np.testing.assert_array_equal(a, b)
