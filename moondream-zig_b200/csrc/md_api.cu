@@ -181,15 +181,6 @@ int md_scratch(md_ctx* ctx, size_t bytes, void** out) {
 }
 
 int md_temp_alloc(md_ctx* ctx, size_t bytes, void** out) {
-    if (!ctx->pool) {
-        cudaMemPoolProps props = {};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = ctx->device;
-        MD_CUDA(ctx, cudaMemPoolCreate(&ctx->pool, &props));
-        uint64_t keep = MD_POOL_KEEP;
-        MD_CUDA(ctx, cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep));
-    }
     MD_CUDA(ctx, cudaMallocFromPoolAsync(out, bytes ? bytes : 1, ctx->pool, ctx->stream));
     return MD_OK;
 }
@@ -295,6 +286,14 @@ int md_init(md_ctx** out, int device) {
     if (reset_flags(ctx) != MD_OK) return bail("flag initialisation");
     if (cudaMalloc(&ctx->counters, MD_COUNTER_WORDS * 4) != cudaSuccess) return bail("cudaMalloc counters");
     if (cudaMemset(ctx->counters, 0, MD_COUNTER_WORDS * 4) != cudaSuccess) return bail("cudaMemset counters");
+    // here and not with the first call that wants it, which may come while a stream is captured
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    uint64_t keep = MD_POOL_KEEP;
+    if (cudaMemPoolCreate(&ctx->pool, &props) != cudaSuccess) return bail("cudaMemPoolCreate");
+    if (cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) return bail("cudaMemPoolSetAttribute");
     ctx->scratch_cap = (size_t)16 << 20;
     if (cudaMalloc(&ctx->scratch, ctx->scratch_cap) != cudaSuccess) return bail("cudaMalloc scratch");
     *out = ctx;
@@ -553,11 +552,18 @@ int md_gemm_dispatch(md_ctx* ctx, const __half* a, const __half* b, __half* c, s
 // tensor memory and the start of the grid come under its end, and every one of them waits for it before it reads or writes anything
 // (md_launch_early).  Back to back on one stream: the five products of a decode step 75.8 -> 64.9 us, four of 64
 // rows 58.7 -> 55.8, the attention of an image and of a prompt under its mask, with the mask, 54 -> 46.7.
-// Not while a graph is captured: a captured call keeps plain edges.
+// Not while a graph is captured, by md_graph_begin or by the owner of a stream given to md_set_stream: a captured call keeps plain edges.
 struct CallScope {
     md_ctx* c;
     bool on;
-    explicit CallScope(md_ctx* ctx) : c(ctx), on(ctx && !ctx->pdl && !ctx->capturing) {
+    static bool captured(const md_ctx* ctx) {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        if (ctx->capturing) return true;
+        if (cudaStreamIsCapturing(ctx->stream, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+        cudaGetLastError();   // the legacy stream while another one is captured
+        return true;
+    }
+    explicit CallScope(md_ctx* ctx) : c(ctx), on(ctx && !ctx->pdl && !captured(ctx)) {
         if (on) c->pdl = 1, c->pdl_late = true;
     }
     ~CallScope() {

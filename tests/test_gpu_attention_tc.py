@@ -1,6 +1,8 @@
 """GPU parity of the two multi-query attention kernels, each forced in turn: the tcgen05 kernel
 (option attn_tc = 1) and the mma.sync kernel (attn_tc = 0), against the oracle's
 multiMasklessSDPA / multiMaskedSDPA restatements (attention.zig:125-234, 416-541)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -188,6 +190,94 @@ def test_masked_ctas_that_walk_over_unseen_query_blocks(ctx, oracle, per_sm):
         _MASKED_WALK["ref"] = oracle.sdpa_masked(q, k[:, 64:].copy(), v[:, 64:].copy(), m[:, 64:].copy())[:, seen]
     assert_close_ref(got[0][:, seen], _MASKED_WALK["ref"], "unseen query blocks")
     np.testing.assert_array_equal(got[0], _MASKED_WALK.setdefault("first", got[0]))
+
+
+def _masked_case(rng, h, lq, lk):
+    q, k, v = f16_normal(rng, (h, lq, 64)), f16_normal(rng, (h, lk, 64)), f16_normal(rng, (h, lk, 64))
+    m = (rng.random((lq, lk)) < 0.5).astype(np.uint8)
+    m[:, 0] = 1
+    return q, k, v, m
+
+
+def _plain_edges(graph) -> bool:
+    """Are all edges of a torch-captured graph full dependencies?  (This form of the query refuses edges with data.)"""
+    n = C.c_size_t(64)
+    ends = (C.c_void_p * 64)(), (C.c_void_p * 64)()
+    status = C.CDLL("libcudart.so.12").cudaGraphGetEdges(C.c_void_p(int(graph.raw_cuda_graph())), *ends, C.byref(n))
+    assert status != 0 or n.value > 2
+    return status == 0
+
+
+@pytest.mark.parametrize("owner", ["context", "stream"])
+def test_masked_attention_in_a_captured_graph(pkg, oracle, owner):
+    """The first calls of a context inside a capture, begun by md_graph_begin or by the owner of the stream the context was given (with
+    the strictest capture mode): a product, and the masked attention with its temporary memory, on plain edges, replayed over changed inputs."""
+    import torch
+    rng = np.random.default_rng(4)
+    h, lq, lk = 4, 200, 333
+    ctx, stream = pkg.Context(0), torch.cuda.Stream()
+    bufs = [torch.from_numpy(x).cuda() for x in _masked_case(rng, h, lq, lk)]
+    a, w = torch.randn(16, 256, device="cuda").half(), torch.randn(512, 256, device="cuda").half()
+    out, prod = torch.empty(h, lq, 64, dtype=torch.half, device="cuda"), torch.empty(16, 512, dtype=torch.half, device="cuda")
+    ptr = [b.data_ptr() for b in bufs]
+    ctx.set_stream(stream.cuda_stream)
+    torch.cuda.synchronize()
+
+    def calls():
+        ctx.hgemm_nt(a.data_ptr(), w.data_ptr(), 16, 512, 256, out=prod.data_ptr())
+        ctx.sdpa_masked(*ptr, h, lq, lk, 64, out=out.data_ptr())
+        ctx.sdpa_masked(*ptr, h, lq, lk, 64, out=out.data_ptr())
+
+    if owner == "context":
+        ctx.graph_begin()
+        calls()
+        g = ctx.graph_end()
+        replay = lambda: ctx.graph_launch(g)
+    else:
+        g = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(g, stream=stream, capture_error_mode="global"):
+            calls()
+        assert _plain_edges(g)
+        replay = g.replay
+    for _ in range(3):
+        case = _masked_case(rng, h, lq, lk)
+        for b, x in zip(bufs, case):
+            b.copy_(torch.from_numpy(x))
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            replay()
+            replay()
+        torch.cuda.synchronize()
+        assert_close_ref(out.cpu().numpy(), oracle.sdpa_masked(*case), "replayed")
+        assert_close_ref(prod.cpu().numpy(), (a.float() @ w.float().T).cpu().numpy(), "replayed product")
+    if owner == "context":
+        ctx.graph_destroy(g)
+    else:
+        del g, replay
+    ctx.close()
+
+
+def test_masked_attention_on_two_streams(pkg, oracle):
+    """A context that is moved between two streams: each call's mask words are its own while both are in flight."""
+    import torch
+    rng = np.random.default_rng(6)
+    ctx, streams = pkg.Context(0), [torch.cuda.Stream(), torch.cuda.Stream()]
+    shapes = [(8, 700, 900), (8, 650, 1000)]
+    cases = [_masked_case(rng, *s) for s in shapes]
+    bufs = [[torch.from_numpy(x).cuda() for x in c] for c in cases]
+    outs = [[torch.empty(s[0], s[1], 64, dtype=torch.half, device="cuda") for _ in range(6)] for s in shapes]
+    torch.cuda.synchronize()
+    for i in range(6):
+        for s in (0, 1):
+            ctx.set_stream(streams[s].cuda_stream)
+            ctx.sdpa_masked(*[b.data_ptr() for b in bufs[s]], *shapes[s], 64, out=outs[s][i].data_ptr())
+    torch.cuda.synchronize()
+    for s in (0, 1):
+        ref = oracle.sdpa_masked(*cases[s])
+        for o in outs[s]:
+            assert_close_ref(o.cpu().numpy(), ref, f"stream {s}")
+    ctx.set_stream(None)
+    ctx.close()
 
 
 def test_forced_tcgen05_rejects_other_head_dims(ctx, pkg):
