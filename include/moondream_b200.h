@@ -101,8 +101,8 @@ int md_set_gemm_mode(md_ctx* ctx, int mode);
  *   "skinny"        1 (default) = products with 8 < M <= 64 rows take the swapped-operand split-K kernel (weights on
  *                   the MMA's M side, K split over the CTAs of a thread-block cluster, ~2 CTAs per SM, partials
  *                   added through distributed shared memory)
- *   "skinny_splits" (unset: the kernel is taken by shape) takes it wherever it can be: 0 = automatic, else the number of K
- *                   splits (rounded down to 1, 2, 4 or 8)
+ *   "skinny_splits" -1 (default): that kernel is taken by shape; else it is taken wherever it can be, with an automatic (0) or
+ *                   this number of K splits (rounded down to 1, 2, 4 or 8)
  *   "pdl"           1 = launch the GEMV kernels with programmatic dependent launch: a kernel starts
  *                   streaming its weights while its predecessor on the stream drains.  Only for streams
  *                   on which no earlier kernel writes the weight matrices (registered weights).
@@ -118,8 +118,9 @@ int md_set_gemm_mode(md_ctx* ctx, int mode);
  *                   0 = mma.sync attention only, 1 = tcgen05 only (MD_ERR_UNSUPPORTED otherwise)
  *   "prefill_fork"  1 (default) = a prefill layer runs fc1 -> fc2 as a second kernel chain beside the attention
  *   "decode_chain"  1 (default) = a decode layer runs as three kernels of one chain (LayerNorm + qkv + fc1; attention and
- *                   fc2; out-projection + residuals); 0, or setting one of the next two: the forms they choose
- *   "decode_fork"   1 = the fused decode layer runs as two concurrent kernel chains (q/k/v projection ->
+ *                   fc2; out-projection + residuals).  0, or any of "decode_fork", "decode_mlp_split", "decode_split_ln" and
+ *                   "decode_cluster" away from its default: the forms that those choose between
+ *   "decode_fork"   1 (default) = the fused decode layer runs as two concurrent kernel chains (q/k/v projection ->
  *                   attention -> out-projection | fc1 -> fc2) joined by events, 0 = three kernels in a row
  *   "push_tma"      how md_hgemm_colsplit_push / _fused send a finished tile to the peers: 1 (default) = the epilogue warps issue
  *                   one more TMA store per peer from the shared-memory chunk they have just staged for this GPU's C;
@@ -133,7 +134,7 @@ int md_set_gemm_mode(md_ctx* ctx, int mode);
  *                   (query block, head, batch) items with its barriers, rings and TMEM kept; 0: one CTA per item
  *   "decode_loop"   n: the attention of a batched decode step with at least n (head, request) pairs runs one CTA per
  *                   pair that walks all of its keys (nothing to merge across CTAs); -1 (default) = 128 (four requests of 32 heads), 0 = never
- *   "decode_mlp_split" 2 or 4 = with decode_fork and a single request, the MLP chain runs as that many
+ *   "decode_mlp_split" 2 (default) or 4 = with decode_fork and a single request, the MLP chain runs as that many
  *                   independent chains (a slice of fc1's rows, then that slice of fc2's K sum as f32 partial sums) which
  *                   the out-projection's epilogue adds with the reference's roundings; 0 = one MLP chain */
 int md_set_option(md_ctx* ctx, const char* key, long value);

@@ -415,7 +415,7 @@ int md_set_option(md_ctx* ctx, const char* key, long value) {
     if (!strcmp(key, "stack_trace")) { ctx->stack_trace = value ? 1 : 0; return MD_OK; }
     if (!strcmp(key, "prefill_fork")) { ctx->prefill_fork = value ? 1 : 0; return MD_OK; }
     if (!strcmp(key, "decode_chain")) { ctx->decode_chain = value ? 1 : 0; return MD_OK; }
-    if (!strcmp(key, "decode_fork")) { ctx->decode_fork = value ? 1 : 0; ctx->decode_chain = 0; return MD_OK; }
+    if (!strcmp(key, "decode_fork")) { ctx->decode_fork = value ? 1 : 0; return MD_OK; }
     if (!strcmp(key, "push_tma")) { ctx->push_tma = value ? 1 : 0; return MD_OK; }
     if (!strcmp(key, "tc_splitk")) {
         if (value < -1 || value == 1 || value > 8) return md_fail(ctx, MD_ERR_INVALID_ARG, "tc_splitk must be -1, 0 or 2..8");
@@ -431,12 +431,11 @@ int md_set_option(md_ctx* ctx, const char* key, long value) {
     if (!strcmp(key, "decode_mlp_split")) {
         MD_NEED(ctx, value == 0 || value == 2 || value == 4, "decode_mlp_split must be 0, 2 or 4");
         ctx->decode_mlp_split = (int)value;
-        ctx->decode_chain = 0;
         return MD_OK;
     }
     if (!strcmp(key, "skinny")) { ctx->skinny = value ? 1 : 0; return MD_OK; }
     if (!strcmp(key, "skinny_splits")) {
-        MD_NEED(ctx, value >= 0 && value <= 16, "skinny_splits must be 0 (automatic) or 1..16 (rounded down to 1, 2, 4 or 8)");
+        MD_NEED(ctx, value >= -1 && value <= 16, "skinny_splits must be -1 (by shape), 0 (automatic) or 1..16 (rounded down to 1, 2, 4 or 8)");
         ctx->skinny_splits = (int)value;
         return MD_OK;
     }

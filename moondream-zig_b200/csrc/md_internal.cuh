@@ -40,6 +40,7 @@ struct md_graph {
     cudaGraphExec_t exec = nullptr;
 };
 
+constexpr int MD_DECODE_SPLIT_LN = 5, MD_DECODE_MLP_SPLIT = 2;   // defaults of the options
 constexpr size_t MD_POOL_KEEP = (size_t)32 << 20;
 constexpr size_t MD_COUNTER_WORDS = 2048;
 constexpr size_t MD_SPLITK_TICKETS = 1024;   // tiles of a split-K GEMM (one arrival ticket each)
@@ -102,20 +103,26 @@ struct md_ctx {
     int pdl = 0;             // md_set_option("pdl"): programmatic dependent launch for the GEMV kernels
     bool pdl_late = false;   // while pdl is on: no kernel may read anything ahead of its dependency wait (md_launch_early)
     int prefill_fork = 1;       // md_set_option("prefill_fork"): prefill layers run the MLP beside the attention
-    int decode_split_ln = 5;    // md_set_option("decode_split_ln"): from this many rows on a decode step runs the LayerNorm once
-    int decode_chain = 1;       // md_set_option("decode_chain"): a decode layer runs as three kernels of one chain; setting decode_fork
-                                // or decode_mlp_split turns it off and chooses between the two-chain forms
+    int decode_split_ln = MD_DECODE_SPLIT_LN;   // md_set_option("decode_split_ln"): from this many rows on a decode step runs the LayerNorm once
+    int decode_chain = 1;       // md_set_option("decode_chain"): a decode layer runs as three kernels of one chain (md_decode_chain)
     int decode_fork = 1;        // md_set_option("decode_fork"): a decode layer runs as two concurrent kernel chains
     int attn_ctas_per_sm = 2;   // md_set_option("attn_ctas_per_sm"): grid of the tcgen05 attention = this many CTAs per SM, each
                                 // walking several (query block, head, batch) items; 0 = one CTA per item
     int decode_loop = -1;       // md_set_option("decode_loop"): batched decode attention as one CTA per (head, request) when there
                                 // are at least this many pairs; -1 = 128, 0 = never
-    int decode_mlp_split = 2;   // md_set_option("decode_mlp_split"): single-request decode runs the MLP as 2 or 4 chains (0 = one)
+    int decode_mlp_split = MD_DECODE_MLP_SPLIT;   // md_set_option("decode_mlp_split"): single-request decode runs the MLP as 2 or 4 chains (0 = one)
     cudaStream_t side_stream = nullptr;  // second chain of the forked decode layer
     cudaStream_t mlp_stream[3] = {};     // further chains when the MLP is split (its first part runs on side_stream)
     cudaEvent_t ev_fork = nullptr, ev_side = nullptr, ev_mlp[3] = {};
     int attn_tc = -1;        // md_set_option("attn_tc"): -1 auto, 0 mma.sync attention only, 1 tcgen05 attention only
 };
+
+// Whoever sets one of the options that choose between the older forms of a decode layer gets them; at its default they are not asked
+// for, and the chain is the faster layer (one request: 25.6 against 26.5 us).
+inline bool md_decode_chain(const md_ctx* ctx) {
+    return ctx->decode_chain && ctx->decode_fork == 1 && ctx->decode_mlp_split == MD_DECODE_MLP_SPLIT &&
+           ctx->decode_split_ln == MD_DECODE_SPLIT_LN && ctx->decode_cluster_mode < 0;
+}
 
 // May a kernel request weights and caches before its dependency wait?  In the model runners, whose weights nothing on the stream
 // writes; not in a call of its own, whose operands may be what the call before it is still writing.

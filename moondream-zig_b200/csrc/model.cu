@@ -189,7 +189,7 @@ int text_layer(md_text_model* m, size_t layer, const LayerIO& io, size_t rows, b
     // (one CTA per SM instead of two) and L2 reads, so from ctx->decode_split_ln rows on the LayerNorm runs once
     // as its own kernel and plain GEMVs with fused epilogues follow (the generic path below, forked the same way).
     const bool ln_once = ctx->decode_split_ln > 0 && rows >= (size_t)ctx->decode_split_ln;
-    if (decode && ctx->fused_decode && ctx->decode_chain && io.mlp_part && md_gemv_ln_dual_supported(rows, D, 3 * D, F) &&
+    if (decode && ctx->fused_decode && md_decode_chain(ctx) && io.mlp_part && md_gemv_ln_dual_supported(rows, D, 3 * D, F) &&
         md_decode_mix_supported(rows, w.n_heads, w.head_dim, D, F) && w.rot_dim <= w.head_dim) {
         // Three kernels in one chain, each started under its predecessor with its first weights requested:
         //   [LayerNorm + qkv, fc1 + GELU] -> [attention, fc2 in four parts of its K sum] -> [out-proj + bias + the parts + hidden]
@@ -691,7 +691,7 @@ static int enqueue_decode_step(md_text_model* model, md_text_request* const* req
     // (742 -> 730 us per step at 1 row, 962 -> 942 at 4 rows, 1210 -> 1079 at 6 rows).
     GemvVariantScope gemv_scope(ctx, 3);
     for (size_t l = 0; l < w.n_layers; ++l) MD_TRY(text_layer(model, l, io, batch, true, reqs, 0));
-    const bool fused_head = ctx->fused_decode && (!ln_once || ctx->decode_chain) && md_gemv_ln_dual_supported(batch, w.dim, w.vocab, 0);
+    const bool fused_head = ctx->fused_decode && (!ln_once || md_decode_chain(ctx)) && md_gemv_ln_dual_supported(batch, w.dim, w.vocab, 0);
     if (fused_head) {
         // final LayerNorm + lm_head + greedy argmax in one kernel (text_model.zig:325-345, sampling.zig:257-273)
         MD_TRY(md_launch_gemv_ln_dual(ctx, r0->hidden.as<__half>(), H(w.ln_out_w), H(w.ln_out_b), eps_of(w.eps_f16),

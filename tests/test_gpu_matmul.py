@@ -267,7 +267,7 @@ def test_skinny_gemm(ctx, oracle, m, k, n, layout, splits):
         if splits == 1:
             assert ctx.get_option("last_tc_tile") == 1001
     finally:
-        ctx.set_option("skinny_splits", 0)
+        ctx.set_option("skinny_splits", -1)
     got = out.numpy()
     assert_close_ref(got, ref, f"skinny {m}x{n}x{k} splits {splits}")
     ctx.set_option("skinny", 0)

@@ -128,8 +128,16 @@ def test_text_graphs_are_captured_again_when_the_context_moves_its_buffers(ctx, 
     req.close(); gpu.close()
 
 
+@pytest.fixture
+def without_chain(ctx):
+    """The forms of a decode layer that the chain of three kernels takes the place of."""
+    ctx.set_option("decode_chain", 0)
+    yield
+    ctx.set_option("decode_chain", 1)
+
+
 def test_text_fused_decode_layer_matches_unfused_kernels(ctx, models_mod):
-    """The 3-kernel decode layer (LayerNorm+qkv+fc1, attention, out-proj+fc2+residuals) against the same step
+    """The default decode layer (LayerNorm + qkv + fc1; attention and fc2; out-projection + residuals) against the same step
     run as separate LayerNorm / GEMV kernels: same rounding points, so logits agree to the parity bar."""
     w = text_weights(4006, n_layers=3, hidden=8192, vocab=4096)
     gpu = models_mod.TextModel(ctx, w)
@@ -179,8 +187,8 @@ def test_text_forked_prefill_equals_the_sequential_prefill(ctx, models_mod):
     gpu.close()
 
 
-def test_text_forked_decode_layer_matches_the_three_kernel_layer(ctx, models_mod):
-    """Option decode_fork (default on): attention chain and MLP chain of a layer as concurrent kernel chains.
+def test_text_forked_decode_layer_matches_the_three_kernel_layer(ctx, models_mod, without_chain):
+    """Option decode_fork without decode_chain: attention chain and MLP chain of a layer as concurrent kernel chains.
     Same rounding points as the three-kernel layer; single request and a batch."""
     w = text_weights(4008, n_layers=3, hidden=8192, vocab=4096)
     gpu = models_mod.TextModel(ctx, w)
@@ -209,8 +217,8 @@ def test_text_forked_decode_layer_matches_the_three_kernel_layer(ctx, models_mod
 
 
 @pytest.mark.parametrize("parts", [2, 4])
-def test_text_split_mlp_decode_layer_matches_the_single_mlp_chain(ctx, oracle, models_mod, parts):
-    """Option decode_mlp_split (default 2, single request): the MLP as 2 or 4 independent chains whose f32 partial sums
+def test_text_split_mlp_decode_layer_matches_the_single_mlp_chain(ctx, oracle, models_mod, parts, without_chain):
+    """Option decode_mlp_split without decode_chain (single request): the MLP as 2 or 4 independent chains whose f32 partial sums
     of fc2 meet in the out-projection's epilogue (one rounding of the sum, then the bias, as the reference rounds
     fc2's output once).  Against the single MLP chain (logits within the parity bar) and against the oracle."""
     w = text_weights(4012, n_layers=3, hidden=8192, vocab=4096)
@@ -241,6 +249,45 @@ def test_text_split_mlp_decode_layer_matches_the_single_mlp_chain(ctx, oracle, m
         assert_close_ref(res[1][1][i], res[0][1][i], f"split MLP vs single chain, step {i}", rel=5e-3)
         cur = int(forced[i])
     gpu.close()
+
+
+def test_decode_options_choose_the_older_forms_and_can_be_set_back(pkg, models_mod):
+    """Away from its default, each option that chooses between the forms of a decode layer takes the layer off the chain (seen by the
+    number of kernels); back at its default the chain is back, and skinny_splits -1 gives the choice by shape back."""
+    ctx = pkg.Context(0)
+    w = text_weights(4030, n_layers=2, hidden=512, vocab=2048)
+    gpu = models_mod.TextModel(ctx, w)
+    req = gpu.request()
+
+    def kernels(key, value):
+        ctx.set_option(key, value)
+        req.reset()
+        gpu.forward(req, w["wte"][:5])
+        n0 = ctx.launch_count()
+        gpu.generate(req, 3, 2)
+        return ctx.launch_count() - n0
+
+    chain = kernels("decode_chain", 1)
+    two_chains = kernels("decode_chain", 0)
+    assert two_chains > chain
+    assert kernels("decode_chain", 1) == chain
+    for key, other, default in (("decode_mlp_split", 0, 2), ("decode_mlp_split", 4, 2), ("decode_split_ln", 1, 5), ("decode_cluster", 1, -1)):
+        assert kernels(key, other) > chain, key
+        assert kernels(key, default) == chain, key
+    kernels("decode_fork", 0)                                # three kernels as well
+    assert kernels("decode_mlp_split", 0) == chain           # which "decode_mlp_split" does not change
+    ctx.set_option("decode_mlp_split", 2)
+    assert kernels("decode_fork", 1) == chain
+    a, b, c = ctx.alloc((64, 2048)), ctx.alloc((8192, 2048)), ctx.alloc((64, 8192))
+    for splits, skinny in ((-1, False), (0, True), (4, True), (-1, False)):
+        ctx.set_option("skinny_splits", splits)
+        ctx.hgemm_nt(a, b, 64, 8192, 2048, out=c)
+        assert (ctx.get_option("last_tc_tile") >= 1000) == skinny
+    with pytest.raises(pkg.MdError):
+        ctx.set_option("skinny_splits", -2)
+    req.close()
+    gpu.close()
+    ctx.close()
 
 
 @pytest.mark.parametrize("hidden", [8192, 1120, 32])
@@ -277,9 +324,10 @@ def test_text_decode_layer_as_one_chain_matches_the_two_chain_layer(ctx, models_
 
 
 @pytest.mark.parametrize("cluster_merge", [1, 0], ids=["cluster_merge", "scratch_merge"])
-def test_text_batched_decode_equals_single_requests(ctx, models_mod, cluster_merge):
+def test_text_batched_decode_equals_single_requests(ctx, models_mod, cluster_merge, without_chain):
     """One attention launch serves the whole batch (grid z = request), each request at its own position; both ways
-    of merging the key splits (thread-block cluster, or global scratch + arrival counters) are exercised."""
+    of merging the key splits (thread-block cluster, or global scratch + arrival counters) are exercised, in the layer whose
+    attention is a kernel of its own (decode_chain off)."""
     w = text_weights(4004, n_layers=2, hidden=512, vocab=2048)
     gpu = models_mod.TextModel(ctx, w)
     rng = np.random.default_rng(4)
@@ -341,9 +389,9 @@ def test_text_batched_decode_with_one_cta_per_head_and_request_equals_single_req
 
 
 @pytest.mark.parametrize("split_ln", [0, 2])
-def test_text_batched_decode_with_one_layernorm_kernel_equals_the_fused_kernels(ctx, models_mod, split_ln):
+def test_text_batched_decode_with_one_layernorm_kernel_equals_the_fused_kernels(ctx, models_mod, split_ln, without_chain):
     """From decode_split_ln rows on the LayerNorm runs once as a kernel and plain GEMVs follow; below it every CTA of
-    the fused kernels recomputes it.  Both forms must produce the tokens of the single-request runs."""
+    the fused kernels recomputes it.  Both forms (decode_chain off) must produce the tokens of the single-request runs."""
     w = text_weights(4014, n_layers=2, hidden=512, vocab=2048)
     gpu = models_mod.TextModel(ctx, w)
     rng = np.random.default_rng(14)
