@@ -1045,9 +1045,12 @@ int md_launch_sdpa(md_ctx* ctx, const __half* q, const __half* k, const __half* 
     if (ctx->attn_tc != 0 && q_len > 0 && kv_len > 0 &&
         md_sdpa_tc_supported(q, k, v, out, d, q_row, q_head, q_batch, kv_row, kv_head, kv_batch, o_row, o_head, o_batch,
                              n_heads, batch) &&
-        (ctx->attn_tc == 1 || q_len > 64))
-        return md_launch_sdpa_tc(ctx, q, k, v, mask, out, n_heads, q_len, kv_len, d, q_row, q_head, kv_row, kv_head, o_row,
-                                 o_head, batch, q_batch, kv_batch, o_batch, causal_pos);
+        (ctx->attn_tc == 1 || q_len > 64)) {
+        const int st = md_launch_sdpa_tc(ctx, q, k, v, mask, out, n_heads, q_len, kv_len, d, q_row, q_head, kv_row, kv_head, o_row,
+                                         o_head, batch, q_batch, kv_batch, o_batch, causal_pos);
+        // without memory for the mask's bits (a host may have taken all there is): the kernels below read its bytes
+        if (st != MD_ERR_OOM || ctx->attn_tc == 1) return st;
+    }
     if (ctx->attn_tc == 1) return md_fail(ctx, MD_ERR_UNSUPPORTED, "attn_tc forced but the operands are not addressable");
     if ((d == 64 || d == 72) && vec_ok) {
         dim3 grid((unsigned)((q_len + BQ - 1) / BQ), (unsigned)n_heads, (unsigned)batch);

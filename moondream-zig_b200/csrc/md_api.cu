@@ -181,8 +181,10 @@ int md_scratch(md_ctx* ctx, size_t bytes, void** out) {
 }
 
 int md_temp_alloc(md_ctx* ctx, size_t bytes, void** out) {
-    MD_CUDA(ctx, cudaMallocFromPoolAsync(out, bytes ? bytes : 1, ctx->pool, ctx->stream));
-    return MD_OK;
+    const cudaError_t e = cudaMallocFromPoolAsync(out, bytes ? bytes : 1, ctx->pool, ctx->stream);
+    if (e == cudaSuccess) return MD_OK;
+    cudaGetLastError();
+    return md_fail(ctx, e == cudaErrorMemoryAllocation ? MD_ERR_OOM : MD_ERR_CUDA, "temporary memory: %s", cudaGetErrorString(e));
 }
 
 int md_temp_free(md_ctx* ctx, void* p) {

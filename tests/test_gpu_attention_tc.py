@@ -280,6 +280,38 @@ def test_masked_attention_on_two_streams(pkg, oracle):
     ctx.close()
 
 
+def test_masked_attention_when_no_device_memory_is_left(pkg, oracle):
+    """A host may have taken all of the device's memory before it calls: the masked attention, which wants some for its mask's bits, then
+    takes the kernel that reads the bytes."""
+    rng = np.random.default_rng(8)
+    h, lq, lk = 4, 200, 2100
+    case = _masked_case(rng, h, lq, lk)
+    ctx, taken = pkg.Context(0), []
+    args = [ctx.upload(x) for x in case]
+    out = ctx.alloc((h, lq, 64))
+    ref = oracle.sdpa_masked(*case)
+    small = [ctx.upload(x) for x in _masked_case(rng, h, 8, 64)]
+    ctx.sdpa_masked(*small, h, 8, 64, 64, out=out)          # the kernel that reads bytes, loaded
+    ctx.sync()
+    size = 16 << 30
+    while size >= 1 << 16 and len(taken) < 400:
+        try:
+            taken.append(ctx.alloc((size,), np.uint8))
+        except pkg.MdError:
+            size //= 4
+    try:
+        ctx.sdpa_masked(*args, h, lq, lk, 64, out=out)
+        ctx.sync()
+    finally:
+        for b in taken:
+            ctx.release(b)
+    assert_close_ref(out.numpy(), ref, "no memory left")
+    ctx.sdpa_masked(*args, h, lq, lk, 64, out=out)
+    ctx.sync()
+    assert_close_ref(out.numpy(), ref, "memory again")
+    ctx.close()
+
+
 def test_forced_tcgen05_rejects_other_head_dims(ctx, pkg):
     ctx.set_option("attn_tc", 1)
     try:
