@@ -100,7 +100,8 @@ int md_set_gemm_mode(md_ctx* ctx, int mode);
  *                   0 = single-CTA tiles only.  Same results bit for bit
  *   "skinny"        1 (default) = products with 8 < M <= 64 rows take the swapped-operand split-K kernel (weights on
  *                   the MMA's M side, K split over the CTAs of a thread-block cluster, ~2 CTAs per SM, partials
- *                   added through distributed shared memory)
+ *                   added through distributed shared memory), but for wide f16 ones of 32 rows and more with a short K and
+ *                   no GELU, where the general kernel is the faster one
  *   "skinny_splits" -1 (default): that kernel is taken by shape; else it is taken wherever it can be, with an automatic (0) or
  *                   this number of K splits (rounded down to 1, 2, 4 or 8)
  *   "pdl"           1 = launch the GEMV kernels with programmatic dependent launch: a kernel starts
@@ -178,7 +179,8 @@ int md_check_matmul_shapes(const size_t* a_shape, size_t a_rank, const size_t* b
  * epilogue, keeping the reference's rounding points: c = f16(acc); if bias: c = f16(c + bias[n])
  * (ops.broadcast_add_simd, ops.zig:1780-1953); if gelu: c = gelu(c) (ops.gelu, ops.zig:1635-1774);
  * if residual: c = f16(c + residual[m,n]) (ops.add, ops.zig:312-323).  bias/residual may be NULL.
- * b_layout: 0 = B is [K,N] (hgemm), 1 = B is [N,K] (hgemm_trans).  All pointers device-resident. */
+ * b_layout: 0 = B is [K,N] (hgemm), 1 = B is [N,K] (hgemm_trans).  All pointers device-resident, bias and residual at any
+ * address (more than 64 rows with either off a 16-byte boundary do without the tensor cores). */
 int md_hgemm_fused(md_ctx* ctx, const uint16_t* a, const uint16_t* b, uint16_t* c, size_t M, size_t N, size_t K,
                    int b_layout, const uint16_t* bias, int gelu, const uint16_t* residual);
 
@@ -245,7 +247,8 @@ int md_sdpa_maskless(md_ctx* ctx, const uint16_t* q, const uint16_t* k, const ui
 int md_create_attention_mask(md_ctx* ctx, uint8_t* mask, size_t pos, size_t seq_len);
 
 /* Replaces attention.multiMaskedSDPA(q,k,v,mask,n_heads,head_dim,allocator) — attention.zig:416-541.
- * mask [q_len, kv_len] bytes, 0 = masked out. */
+ * mask [q_len, kv_len] bytes, 0 = masked out.  More than 64 rows take stream-ordered temporary memory, about an eighth of the
+ * mask's size; where there is none to be had, a slower kernel that needs none. */
 int md_sdpa_masked(md_ctx* ctx, const uint16_t* q, const uint16_t* k, const uint16_t* v, const uint8_t* mask,
                    uint16_t* out, size_t n_heads, size_t q_len, size_t kv_len, size_t head_dim);
 

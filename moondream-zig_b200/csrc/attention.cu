@@ -802,13 +802,6 @@ struct MixParams {
     int M, N, K, per_part;            // columns per part, a multiple of 32
 };
 
-__device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
 constexpr int MIX_WARPS = 8;
 
 // The mapping of gemv_nt_mma_kernel: 16 rows of one part of K.  (CTAs that stay for two to four such units took the same time.)
@@ -844,8 +837,8 @@ __device__ __forceinline__ void mix_product(const MixParams& p, int unit) {
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            mma_f16(acc, lo[u].x, hi[u].x, lo[u].y, hi[u].y, xv[u].x, xv[u].y);
-            mma_f16(acc, lo[u].z, hi[u].z, lo[u].w, hi[u].w, xv[u].z, xv[u].w);
+            mma_16816(acc, lo[u].x, hi[u].x, lo[u].y, hi[u].y, xv[u].x, xv[u].y);
+            mma_16816(acc, lo[u].z, hi[u].z, lo[u].w, hi[u].w, xv[u].z, xv[u].w);
         }
     }
     sums[warp][g][2 * t] = acc[0];
@@ -913,8 +906,8 @@ decode_out_kernel(const __grid_constant__ OutParams p) {
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int u = 0; u < PIECES; ++u) {
-        mma_f16(acc, lo[u].x, hi[u].x, lo[u].y, hi[u].y, xv[u].x, xv[u].y);
-        mma_f16(acc, lo[u].z, hi[u].z, lo[u].w, hi[u].w, xv[u].z, xv[u].w);
+        mma_16816(acc, lo[u].x, hi[u].x, lo[u].y, hi[u].y, xv[u].x, xv[u].y);
+        mma_16816(acc, lo[u].z, hi[u].z, lo[u].w, hi[u].w, xv[u].z, xv[u].w);
     }
     sums[warp][g][2 * t] = acc[0];
     sums[warp][g][2 * t + 1] = acc[1];

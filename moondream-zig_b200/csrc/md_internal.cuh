@@ -343,8 +343,8 @@ __device__ __forceinline__ float md_gelu_f32(float v) {
 }
 
 // The same GELU with the hardware tanh (tanh.approx.f32, one special-function op; absolute error about 5e-4 on the
-// tanh, i.e. at most 0.5 * |x| * 5e-4 on the result, a fraction of the f16 spacing at |x| and far inside the parity
-// bar), for the GEMM epilogues where tanhf, or an exp and a divide, would cost more than the tile's MMAs: with the
+// tanh, i.e. at most 0.5 * |x| * 5e-4 on the result: a fraction of the f16 spacing of the result for x > 0, but up to 15 places
+// of it at -2, where the result is small; against the largest value of a tensor far inside the parity bar), for the GEMM epilogues where tanhf, or an exp and a divide, would cost more than the tile's MMAs: with the
 // exp / divide form the bias + GELU epilogue of a 128 x 256 tile took longer than its 18 k-blocks of MMAs.
 __device__ __forceinline__ float md_gelu_fast_f32(float v) {
     const float c = 0.7978515625f, a = 0.044708251953125f;

@@ -185,9 +185,8 @@ int text_layer(md_text_model* m, size_t layer, const LayerIO& io, size_t rows, b
     md_ctx* ctx = m->ctx;
     const md_text_weights& w = m->w;
     const size_t D = w.dim, F = w.hidden;
-    // The fused kernels recompute the LayerNorm of all rows in every CTA; with many rows that costs registers
-    // (one CTA per SM instead of two) and L2 reads, so from ctx->decode_split_ln rows on the LayerNorm runs once
-    // as its own kernel and plain GEMVs with fused epilogues follow (the generic path below, forked the same way).
+    // Off the chain: the first products recompute the LayerNorm of all rows in every CTA, so from ctx->decode_split_ln rows on
+    // it runs once as its own kernel and plain GEMVs with fused epilogues follow (the generic path below, forked the same way).
     const bool ln_once = ctx->decode_split_ln > 0 && rows >= (size_t)ctx->decode_split_ln;
     if (decode && ctx->fused_decode && md_decode_chain(ctx) && io.mlp_part && md_gemv_ln_dual_supported(rows, D, 3 * D, F) &&
         md_decode_mix_supported(rows, w.n_heads, w.head_dim, D, F) && w.rot_dim <= w.head_dim) {
@@ -686,9 +685,9 @@ static int enqueue_decode_step(md_text_model* model, md_text_request* const* req
     // hidden already holds the embeddings of the current tokens (generate_impl / the previous advance_kernel)
     const LayerIO io = io_of(r0);
     const bool ln_once = ctx->decode_split_ln > 0 && batch >= (size_t)ctx->decode_split_ln;
-    // The automatic GEMV variant is tuned for isolated calls; inside the decode step, where two kernel chains share
-    // the SMs, 8 warps with 8 loads in flight per lane measured best for every GEMV and every batch size
-    // (742 -> 730 us per step at 1 row, 962 -> 942 at 4 rows, 1210 -> 1079 at 6 rows).
+    // The automatic GEMV variant is tuned for isolated calls; inside the layer of two kernel chains, which share the SMs, 8 warps
+    // with 8 loads in flight per lane measured best for every GEMV and every batch size (742 -> 730 us per step at 1 row,
+    // 962 -> 942 at 4 rows, 1210 -> 1079 at 6 rows).  The chain's layers have no plain GEMV.
     GemvVariantScope gemv_scope(ctx, 3);
     for (size_t l = 0; l < w.n_layers; ++l) MD_TRY(text_layer(model, l, io, batch, true, reqs, 0));
     const bool fused_head = ctx->fused_decode && (!ln_once || md_decode_chain(ctx)) && md_gemv_ln_dual_supported(batch, w.dim, w.vocab, 0);
