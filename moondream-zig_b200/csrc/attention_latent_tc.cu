@@ -127,7 +127,7 @@ latent_tc_kernel(const __grid_constant__ LatTcMaps tm, const LatTcParams p, md_d
     // over the items: `g` counts the key tiles this CTA has handled before the current item.
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t kst = 0, vst = 0;       // ring slots
             uint32_t gk = 0, gv = 0;         // K and V tiles loaded so far
             int it = 0;
@@ -169,7 +169,7 @@ latent_tc_kernel(const __grid_constant__ LatTcMaps tm, const LatTcParams p, md_d
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ issuer of the S products
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc_s = idesc_format<true>() | (1u << 4) | ((uint32_t)(LBK >> 3) << 17) | ((uint32_t)(LBQ >> 4) << 24);
             const uint32_t hi128 = desc_hi(1024, 2), k_lo0 = desc_lo(sm_k, 16), stage16 = k_bytes >> 4;
             uint32_t st = 0, par = 0;        // ring slot and parity of the next S product
@@ -211,7 +211,7 @@ latent_tc_kernel(const __grid_constant__ LatTcMaps tm, const LatTcParams p, md_d
         }
     } else if (warp == 6) {
         // ------------------------------------------------------------------ issuer of the PV products
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc_pv =
                 idesc_format<true>() | (1u << 4) | (1u << 16) | ((uint32_t)(p.v_cols >> 3) << 17) | ((uint32_t)(LBQ >> 4) << 24);
             // V: MN-major, 64 dims contiguous per key; the next atom along the dims lies K_ATOM further

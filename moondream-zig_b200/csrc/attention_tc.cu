@@ -272,7 +272,7 @@ attn_tc_kernel(const __grid_constant__ AttnTcMaps tm, AttnTcParams p, md_devflag
     // parities run on over the items: `g` counts the key tiles this CTA has handled before the current item.
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t kst = 0, kpar = 1, vst = 0, vpar = 1;  // ring slots and the parities that say "slot free"
             int ck[4] = {0, 0, 0, 0}, first = 0;
             auto load_k = [&](int j) {
@@ -320,7 +320,7 @@ attn_tc_kernel(const __grid_constant__ AttnTcMaps tm, AttnTcParams p, md_devflag
         // 16; only K and V are read from shared memory.  Issuing a tile's nine MMAs and four commits from one thread
         // took longer than the softmax of the tile, so the two products have a thread each; what orders them across
         // the two threads are the barriers (S(j) waits for PV(j-2), whose P it overwrites; PV(j) waits for P(j)).
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc_s = (1u << 4) | ((uint32_t)(ABKV >> 3) << 17) | ((uint32_t)(ABQ >> 4) << 24);
             // descriptors as 32-bit halves (tc_common.cuh): constant high words, low words advanced by adds; ring
             // slots and their wait parities are running counters
@@ -357,7 +357,7 @@ attn_tc_kernel(const __grid_constant__ AttnTcMaps tm, AttnTcParams p, md_devflag
         }
     } else if (warp == 6) {
         // ------------------------------------------------------------------ issuer of the PV products
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc_pv =
                 (1u << 4) | (1u << 16) | ((uint32_t)(Cfg::DPAD >> 3) << 17) | ((uint32_t)(ABQ >> 4) << 24);
             const uint32_t hi128 = desc_hi(1024, 2);

@@ -155,7 +155,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer (both CTAs)
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0;
             uint32_t phase = 0;
             const uint32_t leader_full = map_to(bar_full, 0);
@@ -190,7 +190,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer (leader only)
-        if (lane == 0 && rank == 0) {
+        if (rank == 0 && elect_one()) {
             // M = 256 over the pair (128 rows per CTA), N = 256, f32 accumulators
             const uint32_t idesc = (1u << 4) | idesc_format<BF16>() | ((B_MN_MAJOR ? 1u : 0u) << 16) | ((uint32_t)(BLOCK_N >> 3) << 17) |
                                    ((uint32_t)((2 * BLOCK_M) >> 4) << 24);

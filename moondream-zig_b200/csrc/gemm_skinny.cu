@@ -88,7 +88,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             auto load_w = [&](int stage, int kb) {
                 const uint32_t full = bar_full + 8 * stage;
                 mbar_expect_tx(full, STAGE_BYTES);
@@ -127,7 +127,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
         md_pdl_wait();
-        if (lane == 0) {
+        if (elect_one()) {
             // D[128 weight rows, 64 activation rows] (f32), A = weights (K-major, or MN-major for the [K,N] layout),
             // B = activations (K-major)
             const uint32_t idesc = (1u << 4) | idesc_format<BF16>() | ((W_MN_MAJOR ? 1u : 0u) << 15) | ((uint32_t)(XN >> 3) << 17) |
