@@ -412,10 +412,10 @@ int md_make_map_2d(md_ctx* ctx, CUtensorMap* map, const void* ptr, uint64_t inne
 // 16-byte aligned pointers, C with row stride ldc); the caller decides when the shape is large enough to pay for the
 // pairing.  push.n > 0: the column-split form (every tile also stored into the peers' C).
 int md_launch_gemm_pair(md_ctx* ctx, const __half* a, const __half* b, __half* c, size_t M, size_t N, size_t K, int b_layout,
-                        const md_epilogue& ep, size_t ldc, const md_push& push) {
+                        const md_epilogue& ep, size_t ldc, const md_push& push, size_t lda) {
     const bool mn = (b_layout == 0), with_push = push.n > 0;
     CUtensorMap tm_a, tm_b, tm_c;
-    MD_TRY(md_make_map_2d(ctx, &tm_a, a, K, M, BLOCK_K, BLOCK_M, 0));
+    MD_TRY(md_make_map_2d(ctx, &tm_a, a, K, M, BLOCK_K, BLOCK_M, lda));
     if (mn) MD_TRY(md_make_map_2d(ctx, &tm_b, b, N, K, 64, BLOCK_K, 0));
     else MD_TRY(md_make_map_2d(ctx, &tm_b, b, K, N, BLOCK_K, HALF_N, 0));
     MD_TRY(md_make_map_2d(ctx, &tm_c, c, N, M, 64, 32, ldc));

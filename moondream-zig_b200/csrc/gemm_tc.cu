@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(PUSH ? NUM_THREADS_PUSH : NUM_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                const __grid_constant__ CUtensorMap tm_c, int M, int N, int K, int tiles_m, int num_tiles,
                md_epilogue ep, md_push push, md_devflags* flags, int splits_arg, float* part, unsigned* tickets,
-               const __grid_constant__ md_peer_maps pm, md_lin lin) {
+               const __grid_constant__ md_peer_maps pm, md_lin lin, int early) {
     const int splits = SPLITK ? splits_arg : 1;
     // splits > 1 (MT == 1, no peers): a work unit is one of `splits` ranges of k-blocks of a tile.  Every unit leaves
     // its f32 accumulators in `part` ([unit][column][row]); the unit that arrives last at the tile's ticket adds the
@@ -131,6 +131,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     const int kb_per = (num_kb + splits - 1) / splits;
     volatile int* last_flag = reinterpret_cast<volatile int*>(bars_ptr + 16 * STAGES + 40 + 4 * EPI_WARPS);
 
+    auto load_b = [&](int stage, int k, int n) {
+        const uint32_t full = bar_full + 8 * stage, dst = smem_b + stage * B_STAGE_BYTES;
+        if (B_MN_MAJOR) {
+#pragma unroll
+            for (int j = 0; j < BLOCK_N / 64; ++j) tma_load_2d(dst + j * (64 * BLOCK_K * 2), &tm_b, full, n + j * 64, k);
+        } else {
+            tma_load_2d(dst, &tm_b, full, k, n);
+        }
+    };
+
     // programmatic dependent launch: this kernel sets up its barriers and tensor memory, lets its successor start, then
     // waits for its predecessor before any global access
     if (threadIdx.x == 0) {
@@ -162,6 +172,22 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     md_pdl_launch_dependents();   // only now that the columns are allocated
+    // The first ring of B does not wait for the kernel before this one if it is a weight that nothing on the stream writes (early):
+    // the producer requests it here, and the A tiles that complete those stages behind the wait.
+    int ahead = 0;
+    if (early && warp == 0 && blockIdx.x < num_units) {
+        const int tile = blockIdx.x / splits, kb0 = (blockIdx.x - tile * splits) * kb_per;
+        ahead = min(STAGES, min(num_kb, kb0 + kb_per) - kb0);
+        if (elect_one()) {
+            int tm, tn;
+            tile_coords(tile, tiles_m, tiles_n, tm, tn);
+            for (int i = 0; i < ahead; ++i) {
+                mbar_expect_tx(bar_full + 8 * i, STAGE_BYTES);
+                load_b(i, (kb0 + i) * BLOCK_K, tn * BLOCK_N);
+            }
+        }
+        __syncwarp();
+    }
     md_pdl_wait();
     const bool grouped = BF16 && MT == 1 && lin.tile_expert != nullptr;
     if (grouped) {
@@ -172,7 +198,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
         if (elect_one()) {
-            int stage = 0;
+            int stage = 0, requested = ahead;
             uint32_t phase = 0;
             for (int unit = blockIdx.x; unit < num_units; unit += gridDim.x) {
                 const int tile = unit / splits, kb0 = (unit - tile * splits) * kb_per, kb1 = min(num_kb, kb0 + kb_per);
@@ -180,21 +206,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                 tile_coords(tile, tiles_m, tiles_n, tm, tn);
                 const int m0 = tm * TILE_M, n0 = tn * BLOCK_N + (grouped ? lin.tile_expert[tm] * N : 0);
                 for (int kb = kb0; kb < kb1; ++kb) {
-                    mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag, flags, 1);
                     const uint32_t full = bar_full + 8 * stage;
-                    mbar_expect_tx(full, STAGE_BYTES);
+                    if (requested > 0) {
+                        --requested;     // the stage's first use: free, announced, B under way
+                    } else {
+                        mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag, flags, 1);
+                        mbar_expect_tx(full, STAGE_BYTES);
+                        load_b(stage, kb * BLOCK_K, n0);
+                    }
 #pragma unroll
                     for (int mt = 0; mt < MT; ++mt)
                         tma_load_2d(smem_a + stage * A_TILE_BYTES + mt * A_STAGE_BYTES, &tm_a, full, kb * BLOCK_K,
                                     m0 + mt * BLOCK_M);
-                    if (B_MN_MAJOR) {
-#pragma unroll
-                        for (int j = 0; j < BLOCK_N / 64; ++j)
-                            tma_load_2d(smem_b + stage * B_STAGE_BYTES + j * (64 * BLOCK_K * 2), &tm_b, full,
-                                        n0 + j * 64, kb * BLOCK_K);
-                    } else {
-                        tma_load_2d(smem_b + stage * B_STAGE_BYTES, &tm_b, full, kb * BLOCK_K, n0);
-                    }
                     if (++stage == STAGES) { stage = 0; phase ^= 1u; }
                 }
             }
@@ -489,9 +512,9 @@ int make_map_2d(md_ctx* ctx, CUtensorMap* map, const void* ptr, uint64_t inner, 
 
 template <int BLOCK_N, bool B_MN_MAJOR, int MT, bool PUSH>
 int launch_as(md_ctx* ctx, const __half* a, const __half* b, __half* c, size_t M, size_t N, size_t K,
-           const md_epilogue& ep, size_t ldc, const md_push& push, int splits = 1) {
+           const md_epilogue& ep, size_t ldc, const md_push& push, size_t lda, int splits = 1) {
     CUtensorMap tm_a, tm_b, tm_c;
-    MD_TRY(make_map_2d(ctx, &tm_a, a, K, M, BLOCK_K, BLOCK_M));
+    MD_TRY(make_map_2d(ctx, &tm_a, a, K, M, BLOCK_K, BLOCK_M, lda));
     if (B_MN_MAJOR) MD_TRY(make_map_2d(ctx, &tm_b, b, N, K, 64, BLOCK_K));
     else MD_TRY(make_map_2d(ctx, &tm_b, b, K, N, BLOCK_K, BLOCK_N));
     MD_TRY(make_map_2d(ctx, &tm_c, c, N, M, 64, 32, ldc));
@@ -512,6 +535,7 @@ int launch_as(md_ctx* ctx, const __half* a, const __half* b, __half* c, size_t M
     memset(&pm, 0, sizeof(pm));
     if (PUSH && push.tma)
         for (int i = 0; i < push.n; ++i) MD_TRY(make_map_2d(ctx, &pm.m[i], push.base[i], N, M, 64, 32, ldc));
+    const int early = ctx->pdl && md_launch_early(ctx) && !PUSH;
     const int units = num_tiles * splits;
     const int grid = units < ctx->sm_count ? units : ctx->sm_count;
     // the split-K instantiation exists for single 128-row tiles of 256 columns without peers only
@@ -531,7 +555,7 @@ int launch_as(md_ctx* ctx, const __half* a, const __half* b, __half* c, size_t M
     ctx->last_tc_tile = (MT == 2 ? 512 : BLOCK_N) + (splits > 1 ? 10000 * splits : 0);   // 30256 = 128 x 256 tiles, K in 3
     return md_launch_ex(ctx, kern, dim3((unsigned)grid), dim3(PUSH ? NUM_THREADS_PUSH : NUM_THREADS), smem,
                         "gemm_tc_kernel", tm_a, tm_b, tm_c, (int)M, (int)N, (int)K, tiles_m, num_tiles, ep, push, ctx->flags,
-                        splits, part, tickets, pm, md_lin());
+                        splits, part, tickets, pm, md_lin(), early);
 }
 
 // The bfloat16 form: C[M, N] (N / 2 columns for a gated product) = md_lin of A[M, K] and B[N, K].
@@ -545,6 +569,7 @@ int launch_lin(md_ctx* ctx, const void* a, const void* b, void* c, size_t M, siz
     else MD_TRY(make_map_2d(ctx, &tm_c, c, N, M, 64, 32, 0, true));
     const int tiles_m = (int)((M + MT * BLOCK_M - 1) / (MT * BLOCK_M)), tiles_n = (int)((N + BLOCK_N - 1) / BLOCK_N);
     const int num_tiles = tiles_m * tiles_n, grid = num_tiles < ctx->sm_count ? num_tiles : ctx->sm_count;
+    const int early = ctx->pdl && md_launch_early(ctx) && !lin.tile_expert;
     auto kern = gemm_tc_kernel<BLOCK_N, false, MT, false, false, true>;
     constexpr int smem = smem_bytes(BLOCK_N, MT);
     const uint32_t bit = 1u << (MT == 2 ? 3 : BLOCK_N == 256 ? 0 : BLOCK_N == 128 ? 1 : 2);
@@ -556,14 +581,14 @@ int launch_lin(md_ctx* ctx, const void* a, const void* b, void* c, size_t M, siz
     memset(&pm, 0, sizeof(pm));
     ctx->last_tc_tile = MT == 2 ? 512 : BLOCK_N;
     return md_launch_ex(ctx, kern, dim3((unsigned)grid), dim3(NUM_THREADS), smem, "gemm_tc_kernel", tm_a, tm_b, tm_c, (int)M, (int)N,
-                        (int)K, tiles_m, num_tiles, md_epilogue(), md_push(), ctx->flags, 1, (float*)nullptr, (unsigned*)nullptr, pm, lin);
+                        (int)K, tiles_m, num_tiles, md_epilogue(), md_push(), ctx->flags, 1, (float*)nullptr, (unsigned*)nullptr, pm, lin, early);
 }
 
 template <int BLOCK_N, bool B_MN_MAJOR, int MT = 1>
 int launch(md_ctx* ctx, const __half* a, const __half* b, __half* c, size_t M, size_t N, size_t K,
-           const md_epilogue& ep, size_t ldc, const md_push& push, int splits = 1) {
-    if (push.n > 0) return launch_as<BLOCK_N, B_MN_MAJOR, MT, true>(ctx, a, b, c, M, N, K, ep, ldc, push);
-    return launch_as<BLOCK_N, B_MN_MAJOR, MT, false>(ctx, a, b, c, M, N, K, ep, ldc, push, splits);
+           const md_epilogue& ep, size_t ldc, const md_push& push, size_t lda, int splits = 1) {
+    if (push.n > 0) return launch_as<BLOCK_N, B_MN_MAJOR, MT, true>(ctx, a, b, c, M, N, K, ep, ldc, push, lda);
+    return launch_as<BLOCK_N, B_MN_MAJOR, MT, false>(ctx, a, b, c, M, N, K, ep, ldc, push, lda, splits);
 }
 
 }  // namespace
@@ -614,9 +639,11 @@ int md_launch_gemm_tc_lin(md_ctx* ctx, const void* a, const void* b, void* c, si
 }
 
 int md_launch_gemm_tc_ex(md_ctx* ctx, const __half* a, const __half* b, __half* c, size_t M, size_t N, size_t K,
-                         int b_layout, const md_epilogue& ep, size_t ldc, const md_push& push) {
+                         int b_layout, const md_epilogue& ep, size_t ldc, const md_push& push, size_t lda) {
     if ((ldc % 8) != 0 || ldc < N)
         return md_fail(ctx, MD_ERR_UNSUPPORTED, "tcgen05 GEMM: the output row stride must be a multiple of 8 and >= N");
+    if (lda != 0 && (lda % 8 != 0 || lda < K))
+        return md_fail(ctx, MD_ERR_UNSUPPORTED, "tcgen05 GEMM: A's row stride must be a multiple of 8 and >= K");
     if (ldc != N && (ep.residual || ep.residual2))
         return md_fail(ctx, MD_ERR_UNSUPPORTED, "tcgen05 GEMM: residuals are not supported with a strided output");
     if (!md_gemm_tc_supported(a, b, c, M, N, K, b_layout) || !md_glue_aligned(ep))
@@ -690,8 +717,8 @@ int md_launch_gemm_tc_ex(md_ctx* ctx, const __half* a, const __half* b, __half* 
         }
     }
     if (splits > 1) {
-        if (b_layout == 0) return launch<256, true>(ctx, a, b, c, M, N, K, ep, ldc, push, splits);
-        return launch<256, false>(ctx, a, b, c, M, N, K, ep, ldc, push, splits);
+        if (b_layout == 0) return launch<256, true>(ctx, a, b, c, M, N, K, ep, ldc, push, lda, splits);
+        return launch<256, false>(ctx, a, b, c, M, N, K, ep, ldc, push, lda, splits);
     }
     // CTA pairs (gemm_pair.cu): where the single-CTA choice is the 128 x 256 tile and there are rows for both CTAs of
     // a pair, the pair's 256 x 256 tile does the same work per SM with a third less traffic from L2 and measured
@@ -699,22 +726,22 @@ int md_launch_gemm_tc_ex(md_ctx* ctx, const __half* a, const __half* b, __half* 
     // choices it lost.  md_set_option("tc_pair"): 1 = always, 0 = never.
     if (!ctx->tc_block_n &&
         (ctx->tc_pair == 1 || (ctx->tc_pair < 0 && bn == 256 && mt == 1 && M > 256)))
-        return md_launch_gemm_pair(ctx, a, b, c, M, N, K, b_layout, ep, ldc, push);
+        return md_launch_gemm_pair(ctx, a, b, c, M, N, K, b_layout, ep, ldc, push, lda);
     if (ctx->tc_block_n) {  // forced: 512 = the 256 x 256 tile
         bn = ctx->tc_block_n == 512 ? 256 : ctx->tc_block_n;
         mt = ctx->tc_block_n == 512 ? 2 : 1;
     }
     const bool mn = (b_layout == 0);
     if (mn) {
-        if (mt == 2) return launch<256, true, 2>(ctx, a, b, c, M, N, K, ep, ldc, push);
-        if (bn == 256) return launch<256, true>(ctx, a, b, c, M, N, K, ep, ldc, push);
-        if (bn == 128) return launch<128, true>(ctx, a, b, c, M, N, K, ep, ldc, push);
-        return launch<64, true>(ctx, a, b, c, M, N, K, ep, ldc, push);
+        if (mt == 2) return launch<256, true, 2>(ctx, a, b, c, M, N, K, ep, ldc, push, lda);
+        if (bn == 256) return launch<256, true>(ctx, a, b, c, M, N, K, ep, ldc, push, lda);
+        if (bn == 128) return launch<128, true>(ctx, a, b, c, M, N, K, ep, ldc, push, lda);
+        return launch<64, true>(ctx, a, b, c, M, N, K, ep, ldc, push, lda);
     }
-    if (mt == 2) return launch<256, false, 2>(ctx, a, b, c, M, N, K, ep, ldc, push);
-    if (bn == 256) return launch<256, false>(ctx, a, b, c, M, N, K, ep, ldc, push);
-    if (bn == 128) return launch<128, false>(ctx, a, b, c, M, N, K, ep, ldc, push);
-    return launch<64, false>(ctx, a, b, c, M, N, K, ep, ldc, push);
+    if (mt == 2) return launch<256, false, 2>(ctx, a, b, c, M, N, K, ep, ldc, push, lda);
+    if (bn == 256) return launch<256, false>(ctx, a, b, c, M, N, K, ep, ldc, push, lda);
+    if (bn == 128) return launch<128, false>(ctx, a, b, c, M, N, K, ep, ldc, push, lda);
+    return launch<64, false>(ctx, a, b, c, M, N, K, ep, ldc, push, lda);
 }
 
 // 2-D f16 tensor map with 128-byte swizzle for other translation units (the attention kernel).

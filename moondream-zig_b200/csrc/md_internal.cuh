@@ -263,7 +263,7 @@ int md_launch_gemm_tc(md_ctx* ctx, const __half* a, const __half* b, __half* c, 
                       int b_layout, const md_epilogue& ep);
 // as above with an output row stride ldc >= N (C is a column block of a wider matrix) and peer pushes
 int md_launch_gemm_tc_ex(md_ctx* ctx, const __half* a, const __half* b, __half* c, size_t M, size_t N, size_t K,
-                         int b_layout, const md_epilogue& ep, size_t ldc, const md_push& push);
+                         int b_layout, const md_epilogue& ep, size_t ldc, const md_push& push, size_t lda = 0);   // lda: A's row stride (0 = K)
 
 // comm.cu: gathered [world][M][n_local] -> c [M][world * n_local] (n_local % 8 == 0, 16-byte aligned)
 int md_launch_gather_colblocks(md_ctx* ctx, const uint16_t* gathered, uint16_t* c, size_t world, size_t M, size_t n_local);
@@ -276,7 +276,7 @@ int md_launch_gemm_skinny(md_ctx* ctx, const __half* a, const __half* b, __half*
 
 // gemm_pair.cu: 256 x 256 tiles on CTA pairs (tcgen05 cta_group::2); same operand rules as md_launch_gemm_tc
 int md_launch_gemm_pair(md_ctx* ctx, const __half* a, const __half* b, __half* c, size_t M, size_t N, size_t K, int b_layout,
-                        const md_epilogue& ep, size_t ldc, const md_push& push);
+                        const md_epilogue& ep, size_t ldc, const md_push& push, size_t lda = 0);
 
 // gemm_tc.cu: a kernel whose bounded wait runs out on purpose (md_selftest_bounded_wait)
 int md_launch_selftest_wait(md_ctx* ctx, unsigned limit_ms);
