@@ -232,6 +232,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         const int half = (warp - 2) >> 2;
         const uint32_t my_epi = smem_epi + (uint32_t)(warp - 2) * EPI_BUF_BYTES;
         uint8_t* my_epi_ptr = epi_ptr + (warp - 2) * EPI_BUF_BYTES;
+        constexpr bool AHEAD = !BF16 && !PUSH;     // (the push warps leave no registers for it)
         const bool any_glue = ep.bias || ep.residual || ep.residual2 || ep.gelu;
         const uint32_t leader_tempty = map_to(bar_tempty, 0);
         constexpr int CHUNKS = BLOCK_N / 64;
@@ -242,6 +243,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             const int m0 = tm * (2 * BLOCK_M) + (int)rank * BLOCK_M, n0 = tn * BLOCK_N;
             const int buf = local & 1;
             const uint32_t acc_phase = (uint32_t)(local >> 1) & 1u;
+            GlueOperands now, next;      // the glue's operands, 32 columns ahead of the accumulators they meet
+            if (AHEAD && any_glue) fetch_glue(now, ep, m0 + quad * 32 + lane, M, n0 + half * 64, N);
             mbar_wait(bar_tfull + 8 * buf, acc_phase, abort_flag, flags, 24);
             tc_fence_after();
 #pragma unroll 1
@@ -268,6 +271,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     if (glu) break;
+                    if (AHEAD && any_glue) {
+                        const int nc = h == 0 ? c : c + 2;
+                        if (nc < CHUNKS) fetch_glue(next, ep, row, M, n0 + nc * 64 + (h ^ 1) * 32, N);
+                    }
                     uint32_t r[32];
                     tc_ld_32x32(t_row + (uint32_t)(c * 64 + h * 32), r);
                     tc_wait_ld();
@@ -276,11 +283,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                     for (int q = 0; q < 4; ++q) {
                         const int cq = col0 + 8 * q;
                         uint32_t pk[4];
-                        if constexpr (BF16) lin_glue8(r + 8 * q, lin, cq, N, pk);
-                        else epilogue_glue8(r + 8 * q, ep, row, cq, N, any_glue && row < M && cq < N, pk);
+                        if constexpr (BF16) {
+                            lin_glue8(r + 8 * q, lin, cq, N, pk);
+                        } else if constexpr (AHEAD) {
+                            epilogue_glue8(r + 8 * q, ep, now, q, any_glue && row < M && cq < N, pk);
+                        } else {
+                            GlueOperands here;
+                            if (any_glue) fetch_glue8(here, q, ep, row, M, cq, N);
+                            epilogue_glue8(r + 8 * q, ep, here, q, any_glue && row < M && cq < N, pk);
+                        }
                         const int chunk = (h * 4 + q) ^ (lane & 7);  // 128-byte swizzle, matches the store map
                         *reinterpret_cast<uint4*>(out_row + chunk * 16) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
                     }
+                    if (AHEAD) now = next;
                 }
                 if (c + 2 >= CHUNKS) {
                     // all of this warp's TMEM reads of the tile are done: hand the buffer back to the leader

@@ -102,6 +102,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     // tile i+1); MT == 2: the two sub-tiles fill all 512 columns, one buffer
     constexpr int NBUF = MT == 1 ? 2 : 1;
     constexpr uint32_t TMEM_COLS = 2 * BLOCK_N;  // 128, 256 or 512: a power of two >= 32
+    constexpr bool NARROW = BLOCK_N == 64 && !PUSH;
     constexpr int TILE_M = MT * BLOCK_M, CHUNKS_N = BLOCK_N / 64, CHUNKS = MT * CHUNKS_N;
     static_assert(BLOCK_N == 64 || BLOCK_N == 128 || BLOCK_N == 256, "BLOCK_N");
     static_assert(MT == 1 || (MT == 2 && BLOCK_N == 256), "two sub-tiles only with 256-wide tiles");
@@ -281,6 +282,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
         const int half = (warp - 2) >> 2;
         const uint32_t my_epi = smem_epi + (uint32_t)(warp - 2) * EPI_BUF_BYTES;
         uint8_t* my_epi_ptr = epi_ptr + (warp - 2) * EPI_BUF_BYTES;
+        constexpr bool AHEAD = !BF16 && !PUSH;     // (the push warps leave no registers for it)
         const bool any_glue = ep.bias || ep.residual || ep.residual2 || ep.gelu;
         int local = 0;
         for (int unit = blockIdx.x; unit < num_units; unit += gridDim.x, ++local) {
@@ -290,6 +292,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
             const int m0 = tm * TILE_M, n0 = tn * BLOCK_N;
             const int buf = local % NBUF;
             const uint32_t acc_phase = (uint32_t)(local / NBUF) & 1u;
+            const bool glu = BF16 && lin.glu;
+            const bool narrow = NARROW && !glu;      // 32 columns per warp instead of 64 for every other one
+            const int first_cc = narrow ? 0 : half, first_h = narrow ? half : 0;
+            // the glue's operands, 32 columns ahead of the accumulators they meet
+            GlueOperands now, next;
+            if (AHEAD && any_glue && first_cc < CHUNKS)
+                fetch_glue(now, ep, m0 + (first_cc / CHUNKS_N) * BLOCK_M + quad * 32 + lane, M, n0 + (first_cc % CHUNKS_N) * 64 + first_h * 32, N);
             mbar_wait(bar_tfull + 8 * buf, acc_phase, abort_flag, flags, 4);
             tc_fence_after();
             const bool from_part = SPLITK && splits > 1;
@@ -325,7 +334,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
             }
             const float* parts = part + (size_t)tile * splits * (BLOCK_M * BLOCK_N) + quad * 32 + lane;
 #pragma unroll 1
-            for (int cc = half; cc < CHUNKS; cc += 2) {
+            for (int cc = first_cc; cc < CHUNKS; cc += 2) {
                 // chunk cc = 64 columns c of sub-tile mt
                 const int mt = cc / CHUNKS_N, c = cc % CHUNKS_N;
                 const int mrow0 = m0 + mt * BLOCK_M + quad * 32, row = mrow0 + lane;
@@ -333,8 +342,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                 // the staging buffer must have been read by this warp's previous TMA store
                 if (lane == 0) tma_store_wait_read<0>();
                 __syncwarp();
-                uint8_t* out_row = my_epi_ptr + lane * 128;
-                const bool glu = BF16 && lin.glu;
+                uint8_t* out_row = my_epi_ptr + lane * (narrow ? 64 : 128);
                 if (glu) {
                     uint32_t g[32], u[32];
                     tc_ld_32x32(t_row + (uint32_t)(c * 64), g);
@@ -350,7 +358,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                 }
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    if (glu) break;
+                    if (glu || (narrow && h != half)) continue;
+                    if (AHEAD && any_glue) {
+                        const int nc = h == 0 ? cc : cc + 2, nh = h ^ 1;
+                        if (!narrow && nc < CHUNKS)
+                            fetch_glue(next, ep, m0 + (nc / CHUNKS_N) * BLOCK_M + quad * 32 + lane, M, n0 + (nc % CHUNKS_N) * 64 + nh * 32, N);
+                    }
                     uint32_t r[32];
                     if (from_part) {
                         // the k ranges added up in their order, whichever unit got here last; a range's 32 loads are
@@ -380,11 +393,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                     for (int q = 0; q < 4; ++q) {
                         const int cq = col0 + 8 * q;
                         uint32_t pk[4];
-                        if constexpr (BF16) lin_glue8(r + 8 * q, lin, cq, N, pk);
-                        else epilogue_glue8(r + 8 * q, ep, row, cq, N, any_glue && row < M && cq < N, pk);
-                        const int chunk = (h * 4 + q) ^ (lane & 7);  // 128-byte swizzle, matches the store map
+                        if constexpr (BF16) {
+                            lin_glue8(r + 8 * q, lin, cq, N, pk);
+                        } else if constexpr (AHEAD) {
+                            epilogue_glue8(r + 8 * q, ep, now, q, any_glue && row < M && cq < N, pk);
+                        } else {
+                            GlueOperands here;
+                            if (any_glue) fetch_glue8(here, q, ep, row, M, cq, N);
+                            epilogue_glue8(r + 8 * q, ep, here, q, any_glue && row < M && cq < N, pk);
+                        }
+                        // 128-byte or 64-byte swizzle, as the store map says
+                        const int chunk = narrow ? q ^ ((lane >> 1) & 3) : (h * 4 + q) ^ (lane & 7);
                         *reinterpret_cast<uint4*>(out_row + chunk * 16) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
                     }
+                    if (AHEAD) now = next;
                 }
                 if (cc + 2 >= CHUNKS && !from_part) {
                     // all of this warp's TMEM reads of the tile are done: hand the buffer back
@@ -395,7 +417,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                 fence_async_smem();
                 __syncwarp();
                 if (lane == 0) {
-                    tma_store_2d(&tm_c, my_epi, glu ? (n0 + c * 64) / 2 : n0 + c * 64, mrow0);
+                    tma_store_2d(&tm_c, my_epi, glu ? (n0 + c * 64) / 2 : narrow ? n0 + half * 32 : n0 + c * 64, mrow0);
                     if (PUSH && push.tma) {
                         // the same staged chunk into every peer's C, starting with a different peer in every CTA;
                         // the staging buffer is reused once all of these stores have read it
@@ -408,7 +430,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                     tma_store_commit();
                 }
             }
-            if (half >= CHUNKS && !from_part) {
+            if (first_cc >= CHUNKS && !from_part) {
                 // a warp without a chunk (tile narrower than its share) still releases the accumulator
                 tc_fence_before();
                 __syncwarp();
@@ -517,7 +539,8 @@ int launch_as(md_ctx* ctx, const __half* a, const __half* b, __half* c, size_t M
     MD_TRY(make_map_2d(ctx, &tm_a, a, K, M, BLOCK_K, BLOCK_M, lda));
     if (B_MN_MAJOR) MD_TRY(make_map_2d(ctx, &tm_b, b, N, K, 64, BLOCK_K));
     else MD_TRY(make_map_2d(ctx, &tm_b, b, K, N, BLOCK_K, BLOCK_N));
-    MD_TRY(make_map_2d(ctx, &tm_c, c, N, M, 64, 32, ldc));
+    constexpr bool NARROW = BLOCK_N == 64 && !PUSH;    // the epilogue's warps then store 32 columns each
+    MD_TRY(make_map_2d(ctx, &tm_c, c, N, M, NARROW ? 32 : 64, 32, ldc, false, NARROW));
     const int tiles_m = (int)((M + MT * BLOCK_M - 1) / (MT * BLOCK_M)), tiles_n = (int)((N + BLOCK_N - 1) / BLOCK_N);
     const int num_tiles = tiles_m * tiles_n;
     float* part = nullptr;
@@ -566,7 +589,7 @@ int launch_lin(md_ctx* ctx, const void* a, const void* b, void* c, size_t M, siz
     MD_TRY(make_map_2d(ctx, &tm_a, a, K, M, BLOCK_K, BLOCK_M, 0, true));
     MD_TRY(make_map_2d(ctx, &tm_b, b, K, b_rows, BLOCK_K, BLOCK_N, 0, true));
     if (lin.glu) MD_TRY(make_map_2d(ctx, &tm_c, c, N / 2, M, 32, 32, 0, true, true));
-    else MD_TRY(make_map_2d(ctx, &tm_c, c, N, M, 64, 32, 0, true));
+    else MD_TRY(make_map_2d(ctx, &tm_c, c, N, M, BLOCK_N == 64 ? 32 : 64, 32, 0, true, BLOCK_N == 64));
     const int tiles_m = (int)((M + MT * BLOCK_M - 1) / (MT * BLOCK_M)), tiles_n = (int)((N + BLOCK_N - 1) / BLOCK_N);
     const int num_tiles = tiles_m * tiles_n, grid = num_tiles < ctx->sm_count ? num_tiles : ctx->sm_count;
     const int early = ctx->pdl && md_launch_early(ctx) && !lin.tile_expert;

@@ -244,23 +244,39 @@ __device__ __forceinline__ void load8(const __half* p, float (&f)[8]) {
     }
 }
 
-// The fused glue of a GEMM epilogue on 8 consecutive output columns of one row: f32 accumulators in, four packed
-// half2 out.  Every step keeps the reference's rounding point (one rounding to f16 after the product, after the
+// What the fused glue reads beside the accumulators, for 32 consecutive output columns of one row.  Requested ahead of the
+// accumulators: as loads between their arrival and the stores they were a round trip to L2 for every 32 columns.
+struct GlueOperands { uint4 bias[4], residual[4], residual2[4]; };
+__device__ __forceinline__ void fetch_glue8(GlueOperands& o, int q, const md_epilogue& ep, int row, int M, int cq, int N) {
+    if (row >= M || cq >= N) return;
+    if (ep.bias) o.bias[q] = *reinterpret_cast<const uint4*>(ep.bias + cq);
+    if (ep.residual) {
+        const int rm = ep.residual_rows > 0 ? row % ep.residual_rows : row;
+        o.residual[q] = *reinterpret_cast<const uint4*>(ep.residual + (size_t)rm * N + cq);
+    }
+    if (ep.residual2) o.residual2[q] = *reinterpret_cast<const uint4*>(ep.residual2 + (size_t)row * N + cq);
+}
+__device__ __forceinline__ void fetch_glue(GlueOperands& o, const md_epilogue& ep, int row, int M, int col0, int N) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) fetch_glue8(o, q, ep, row, M, col0 + 8 * q, N);
+}
+// The fused glue of a GEMM epilogue on 8 consecutive output columns of one row (piece q of its operands): f32 accumulators in, four
+// packed half2 out.  Every step keeps the reference's rounding point (one rounding to f16 after the product, after the
 // bias, after the GELU, after each residual).  Sums of two f16 values are formed with packed f16 adds: an f16 + f16
 // sum is exact in f32, so f16(f32(a) + f32(b)) and the correctly rounded f16 add are the same number; only the GELU
-// needs f32 arithmetic.  (cq, row) is the position of the first column; N % 8 == 0 and 16-byte aligned operands.
-__device__ __forceinline__ void epilogue_glue8(const uint32_t* acc_bits, const md_epilogue& ep, int row, int cq, int N,
-                                               bool apply, uint32_t (&pk)[4]) {
+// needs f32 arithmetic.  N % 8 == 0 and 16-byte aligned operands; apply = the columns lie inside the matrix.
+__device__ __forceinline__ void epilogue_glue8(const uint32_t* acc_bits, const md_epilogue& ep, const GlueOperands& o, int q, bool apply,
+                                               uint32_t (&pk)[4]) {
     __half2 h[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) h[j] = __floats2half2_rn(__uint_as_float(acc_bits[2 * j]), __uint_as_float(acc_bits[2 * j + 1]));
     if (apply) {
-        if (ep.bias) {
-            const uint4 u = *reinterpret_cast<const uint4*>(ep.bias + cq);
+        auto add = [&](const uint4& u) {
             const __half2* b = reinterpret_cast<const __half2*>(&u);
 #pragma unroll
             for (int j = 0; j < 4; ++j) h[j] = __hadd2(h[j], b[j]);
-        }
+        };
+        if (ep.bias) add(o.bias[q]);
         if (ep.gelu) {
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -268,19 +284,8 @@ __device__ __forceinline__ void epilogue_glue8(const uint32_t* acc_bits, const m
                 h[j] = __floats2half2_rn(md_gelu_fast_f32(x.x), md_gelu_fast_f32(x.y));
             }
         }
-        if (ep.residual) {
-            const int rm = ep.residual_rows > 0 ? row % ep.residual_rows : row;
-            const uint4 u = *reinterpret_cast<const uint4*>(ep.residual + (size_t)rm * N + cq);
-            const __half2* b = reinterpret_cast<const __half2*>(&u);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) h[j] = __hadd2(h[j], b[j]);
-        }
-        if (ep.residual2) {
-            const uint4 u = *reinterpret_cast<const uint4*>(ep.residual2 + (size_t)row * N + cq);
-            const __half2* b = reinterpret_cast<const __half2*>(&u);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) h[j] = __hadd2(h[j], b[j]);
-        }
+        if (ep.residual) add(o.residual[q]);
+        if (ep.residual2) add(o.residual2[q]);
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) pk[j] = *reinterpret_cast<uint32_t*>(&h[j]);
