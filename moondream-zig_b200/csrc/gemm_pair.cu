@@ -236,86 +236,108 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         const bool any_glue = ep.bias || ep.residual || ep.residual2 || ep.gelu;
         const uint32_t leader_tempty = map_to(bar_tempty, 0);
         constexpr int CHUNKS = BLOCK_N / 64;
-        int local = 0;
+        int local = 0, stage_buf = 0;
         for (int tile = pair; tile < num_tiles; tile += num_pairs, ++local) {
             int tm, tn;
             pair_tile_coords(tile, tiles_m, tiles_n, tm, tn);
             const int m0 = tm * (2 * BLOCK_M) + (int)rank * BLOCK_M, n0 = tn * BLOCK_N;
             const int buf = local & 1;
             const uint32_t acc_phase = (uint32_t)(local >> 1) & 1u;
-            GlueOperands now, next;      // the glue's operands, 32 columns ahead of the accumulators they meet
-            if (AHEAD && any_glue) fetch_glue(now, ep, m0 + quad * 32 + lane, M, n0 + half * 64, N);
+            const bool glu = BF16 && lin.glu;
+            const int n_units = PUSH || glu ? CHUNKS : 2 * CHUNKS;   // as in the single-CTA kernel: 32 output columns at a time
+            const int mrow0 = m0 + quad * 32, row = mrow0 + lane;
+            const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * BLOCK_N);
+            GlueOperands now, next;      // the glue's operands, a unit ahead of the accumulators they meet
+            if (AHEAD && any_glue) fetch_glue(now, ep, row, M, n0 + half * 32, N);
             mbar_wait(bar_tfull + 8 * buf, acc_phase, abort_flag, flags, 24);
             tc_fence_after();
-#pragma unroll 1
-            for (int c = half; c < CHUNKS; c += 2) {
-                const int mrow0 = m0 + quad * 32, row = mrow0 + lane;
-                const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * BLOCK_N);
-                if (lane == 0) tma_store_wait_read<0>();
+            auto hand_back = [&]() {     // all of this warp's TMEM reads of the tile are done: the buffer is the leader's again
+                tc_fence_before();
                 __syncwarp();
-                uint8_t* out_row = my_epi_ptr + lane * 128;
-                const bool glu = BF16 && lin.glu;
-                if (glu) {
-                    uint32_t g[32], u[32];
-                    tc_ld_32x32(t_row + (uint32_t)(c * 64), g);
-                    tc_ld_32x32(t_row + (uint32_t)(c * 64 + 32), u);
-                    tc_wait_ld();
+                if (lane == 0) mbar_arrive_cluster(leader_tempty + 8 * buf);
+            };
+            if constexpr (PUSH) {
+#pragma unroll 1
+                for (int c = half; c < CHUNKS; c += 2) {
+                    if (lane == 0) tma_store_wait_read<0>();
+                    __syncwarp();
+                    uint8_t* out_row = my_epi_ptr + lane * 128;
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        uint32_t pk[4];
-                        glu_glue8(g + 8 * q, u + 8 * q, lin, pk);
-                        const int chunk = q ^ ((lane >> 1) & 3);   // 64-byte swizzle
-                        *reinterpret_cast<uint4*>(my_epi_ptr + lane * 64 + chunk * 16) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                    }
-                }
+                    for (int h = 0; h < 2; ++h) {
+                        uint32_t r[32];
+                        tc_ld_32x32(t_row + (uint32_t)(c * 64 + h * 32), r);
+                        tc_wait_ld();
+                        const int col0 = n0 + c * 64 + h * 32;
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    if (glu) break;
-                    if (AHEAD && any_glue) {
-                        const int nc = h == 0 ? c : c + 2;
-                        if (nc < CHUNKS) fetch_glue(next, ep, row, M, n0 + nc * 64 + (h ^ 1) * 32, N);
-                    }
-                    uint32_t r[32];
-                    tc_ld_32x32(t_row + (uint32_t)(c * 64 + h * 32), r);
-                    tc_wait_ld();
-                    const int col0 = n0 + c * 64 + h * 32;
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const int cq = col0 + 8 * q;
-                        uint32_t pk[4];
-                        if constexpr (BF16) {
-                            lin_glue8(r + 8 * q, lin, cq, N, pk);
-                        } else if constexpr (AHEAD) {
-                            epilogue_glue8(r + 8 * q, ep, now, q, any_glue && row < M && cq < N, pk);
-                        } else {
+                        for (int q = 0; q < 4; ++q) {
+                            const int cq = col0 + 8 * q;
+                            uint32_t pk[4];
                             GlueOperands here;
                             if (any_glue) fetch_glue8(here, q, ep, row, M, cq, N);
                             epilogue_glue8(r + 8 * q, ep, here, q, any_glue && row < M && cq < N, pk);
+                            const int chunk = (h * 4 + q) ^ (lane & 7);  // 128-byte swizzle, matches the store map
+                            *reinterpret_cast<uint4*>(out_row + chunk * 16) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
                         }
-                        const int chunk = (h * 4 + q) ^ (lane & 7);  // 128-byte swizzle, matches the store map
-                        *reinterpret_cast<uint4*>(out_row + chunk * 16) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
                     }
-                    if (AHEAD) now = next;
-                }
-                if (c + 2 >= CHUNKS) {
-                    // all of this warp's TMEM reads of the tile are done: hand the buffer back to the leader
-                    tc_fence_before();
+                    if (c + 2 >= CHUNKS) hand_back();
+                    fence_async_smem();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive_cluster(leader_tempty + 8 * buf);
-                }
-                fence_async_smem();
-                __syncwarp();
-                if (lane == 0) {
-                    tma_store_2d(&tm_c, my_epi, glu ? (n0 + c * 64) / 2 : n0 + c * 64, mrow0);
-                    if (PUSH && push.tma) {
-                        // the same staged chunk into every peer's C, starting with a different peer in every CTA
-                        for (int pi = 0; pi < push.n; ++pi) {
-                            int peer = pi + (int)blockIdx.x;
-                            peer -= (peer / push.n) * push.n;
-                            tma_store_2d(&pm.m[peer], my_epi, n0 + c * 64, mrow0);
+                    if (lane == 0) {
+                        tma_store_2d(&tm_c, my_epi, n0 + c * 64, mrow0);
+                        if (push.tma) {
+                            // the same staged chunk into every peer's C, starting with a different peer in every CTA
+                            for (int pi = 0; pi < push.n; ++pi) {
+                                int peer = pi + (int)blockIdx.x;
+                                peer -= (peer / push.n) * push.n;
+                                tma_store_2d(&pm.m[peer], my_epi, n0 + c * 64, mrow0);
+                            }
                         }
+                        tma_store_commit();
                     }
-                    tma_store_commit();
+                }
+            } else {
+#pragma unroll 1
+                for (int u = half; u < n_units; u += 2) {
+                    const int acc_col = u * (glu ? 64 : 32), out_col = glu ? (n0 + acc_col) / 2 : n0 + acc_col;
+                    if (lane == 0) tma_store_wait_read<1>();     // two staging buffers a warp
+                    __syncwarp();
+                    uint8_t* out_row = my_epi_ptr + stage_buf * (EPI_BUF_BYTES / 2) + lane * 64;
+                    auto put = [&](int q, const uint32_t(&pk)[4]) {     // 64-byte swizzle
+                        *reinterpret_cast<uint4*>(out_row + ((q ^ ((lane >> 1) & 3)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                    };
+                    uint32_t r[32];
+                    tc_ld_32x32(t_row + (uint32_t)acc_col, r);
+                    if (glu) {
+                        uint32_t up[32];
+                        tc_ld_32x32(t_row + (uint32_t)acc_col + 32u, up);
+                        tc_wait_ld();
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            uint32_t pk[4];
+                            glu_glue8(r + 8 * q, up + 8 * q, lin, pk);
+                            put(q, pk);
+                        }
+                    } else {
+                        if (AHEAD && any_glue && u + 2 < n_units) fetch_glue(next, ep, row, M, out_col + 64, N);
+                        tc_wait_ld();
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const int cq = out_col + 8 * q;
+                            uint32_t pk[4];
+                            if constexpr (BF16) lin_glue8(r + 8 * q, lin, cq, N, pk);
+                            else epilogue_glue8(r + 8 * q, ep, now, q, any_glue && row < M && cq < N, pk);
+                            put(q, pk);
+                        }
+                        if (AHEAD) now = next;
+                    }
+                    if (u + 2 >= n_units) hand_back();
+                    fence_async_smem();
+                    __syncwarp();
+                    if (lane == 0) {
+                        tma_store_2d(&tm_c, my_epi + (uint32_t)(stage_buf * (EPI_BUF_BYTES / 2)), out_col, mrow0);
+                        tma_store_commit();
+                    }
+                    stage_buf ^= 1;
                 }
             }
             if (PUSH && !push.tma && lane == 0) {
@@ -421,7 +443,7 @@ int launch_pairs(md_ctx* ctx, pair_fn kern, uint32_t cfg_bit, const CUtensorMap&
 }  // namespace
 
 int md_make_map_2d(md_ctx* ctx, CUtensorMap* map, const void* ptr, uint64_t inner, uint64_t outer, uint32_t box_inner,
-                   uint32_t box_outer, uint64_t ld);
+                   uint32_t box_outer, uint64_t ld, bool swizzle_64 = false);
 
 // C[M,N] = A . B (+ fused glue) on CTA pairs.  Same operand rules as the single-CTA kernel (K % 8 == 0, N % 8 == 0,
 // 16-byte aligned pointers, C with row stride ldc); the caller decides when the shape is large enough to pay for the
@@ -433,7 +455,7 @@ int md_launch_gemm_pair(md_ctx* ctx, const __half* a, const __half* b, __half* c
     MD_TRY(md_make_map_2d(ctx, &tm_a, a, K, M, BLOCK_K, BLOCK_M, lda));
     if (mn) MD_TRY(md_make_map_2d(ctx, &tm_b, b, N, K, 64, BLOCK_K, 0));
     else MD_TRY(md_make_map_2d(ctx, &tm_b, b, K, N, BLOCK_K, HALF_N, 0));
-    MD_TRY(md_make_map_2d(ctx, &tm_c, c, N, M, 64, 32, ldc));
+    MD_TRY(md_make_map_2d(ctx, &tm_c, c, N, M, with_push ? 64 : 32, 32, ldc, !with_push));
     md_peer_maps pm;
     memset(&pm, 0, sizeof(pm));
     if (with_push && push.tma)
@@ -449,8 +471,7 @@ int md_launch_gemm_pair_lin(md_ctx* ctx, const void* a, const void* b, void* c, 
     CUtensorMap tm_a, tm_b, tm_c;
     MD_TRY(md_make_map_2d_bf16(ctx, &tm_a, a, K, M, BLOCK_K, BLOCK_M, false));
     MD_TRY(md_make_map_2d_bf16(ctx, &tm_b, b, K, N, BLOCK_K, HALF_N, false));
-    if (lin.glu) MD_TRY(md_make_map_2d_bf16(ctx, &tm_c, c, N / 2, M, 32, 32, true));
-    else MD_TRY(md_make_map_2d_bf16(ctx, &tm_c, c, N, M, 64, 32, false));
+    MD_TRY(md_make_map_2d_bf16(ctx, &tm_c, c, lin.glu ? N / 2 : N, M, 32, 32, true));
     md_peer_maps pm;
     memset(&pm, 0, sizeof(pm));
     return launch_pairs(ctx, gemm_pair_kernel<false, false, true>, 1u << 4, tm_a, tm_b, tm_c, M, N, K, md_epilogue(), md_push(), pm, lin);

@@ -271,7 +271,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
 }  // namespace
 
 int md_make_map_2d(md_ctx* ctx, CUtensorMap* map, const void* ptr, uint64_t inner, uint64_t outer, uint32_t box_inner,
-                   uint32_t box_outer, uint64_t ld);
+                   uint32_t box_outer, uint64_t ld, bool swizzle_64 = false);
 
 bool md_gemm_skinny_supported(const void* a, const void* b, const void* c, size_t M, size_t N, size_t K) {
     if (M <= 8 || M > (size_t)XN || N == 0 || K == 0) return false;

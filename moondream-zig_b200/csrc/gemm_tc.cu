@@ -102,7 +102,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     // tile i+1); MT == 2: the two sub-tiles fill all 512 columns, one buffer
     constexpr int NBUF = MT == 1 ? 2 : 1;
     constexpr uint32_t TMEM_COLS = 2 * BLOCK_N;  // 128, 256 or 512: a power of two >= 32
-    constexpr bool NARROW = BLOCK_N == 64 && !PUSH;
     constexpr int TILE_M = MT * BLOCK_M, CHUNKS_N = BLOCK_N / 64, CHUNKS = MT * CHUNKS_N;
     static_assert(BLOCK_N == 64 || BLOCK_N == 128 || BLOCK_N == 256, "BLOCK_N");
     static_assert(MT == 1 || (MT == 2 && BLOCK_N == 256), "two sub-tiles only with 256-wide tiles");
@@ -284,7 +283,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
         uint8_t* my_epi_ptr = epi_ptr + (warp - 2) * EPI_BUF_BYTES;
         constexpr bool AHEAD = !BF16 && !PUSH;     // (the push warps leave no registers for it)
         const bool any_glue = ep.bias || ep.residual || ep.residual2 || ep.gelu;
-        int local = 0;
+        int local = 0, stage_buf = 0;
         for (int unit = blockIdx.x; unit < num_units; unit += gridDim.x, ++local) {
             const int tile = unit / splits;
             int tm, tn;
@@ -293,12 +292,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
             const int buf = local % NBUF;
             const uint32_t acc_phase = (uint32_t)(local / NBUF) & 1u;
             const bool glu = BF16 && lin.glu;
-            const bool narrow = NARROW && !glu;      // 32 columns per warp instead of 64 for every other one
-            const int first_cc = narrow ? 0 : half, first_h = narrow ? half : 0;
-            // the glue's operands, 32 columns ahead of the accumulators they meet
-            GlueOperands now, next;
-            if (AHEAD && any_glue && first_cc < CHUNKS)
-                fetch_glue(now, ep, m0 + (first_cc / CHUNKS_N) * BLOCK_M + quad * 32 + lane, M, n0 + (first_cc % CHUNKS_N) * 64 + first_h * 32, N);
+            // 32 output columns at a time, in turn by the two warps of a lane quadrant (a gated product's come from 64)
+            const int n_units = PUSH || glu ? CHUNKS : 2 * CHUNKS;
+            GlueOperands now, next;   // the glue's operands, a unit ahead of the accumulators they meet
+            auto fetch_unit = [&](GlueOperands& o, int u) {
+                fetch_glue(o, ep, m0 + u / (2 * CHUNKS_N) * BLOCK_M + quad * 32 + lane, M, n0 + u % (2 * CHUNKS_N) * 32, N);
+            };
+            if (AHEAD && any_glue && half < n_units) fetch_unit(now, half);
             mbar_wait(bar_tfull + 8 * buf, acc_phase, abort_flag, flags, 4);
             tc_fence_after();
             const bool from_part = SPLITK && splits > 1;
@@ -333,105 +333,136 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                 __threadfence();
             }
             const float* parts = part + (size_t)tile * splits * (BLOCK_M * BLOCK_N) + quad * 32 + lane;
+            if constexpr (PUSH) {
 #pragma unroll 1
-            for (int cc = first_cc; cc < CHUNKS; cc += 2) {
-                // chunk cc = 64 columns c of sub-tile mt
-                const int mt = cc / CHUNKS_N, c = cc % CHUNKS_N;
-                const int mrow0 = m0 + mt * BLOCK_M + quad * 32, row = mrow0 + lane;
-                const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * BLOCK_N + mt * 256);
-                // the staging buffer must have been read by this warp's previous TMA store
-                if (lane == 0) tma_store_wait_read<0>();
-                __syncwarp();
-                uint8_t* out_row = my_epi_ptr + lane * (narrow ? 64 : 128);
-                if (glu) {
-                    uint32_t g[32], u[32];
-                    tc_ld_32x32(t_row + (uint32_t)(c * 64), g);
-                    tc_ld_32x32(t_row + (uint32_t)(c * 64 + 32), u);
-                    tc_wait_ld();
+                for (int cc = half; cc < CHUNKS; cc += 2) {
+                    // chunk cc = 64 columns c of sub-tile mt
+                    const int mt = cc / CHUNKS_N, c = cc % CHUNKS_N;
+                    const int mrow0 = m0 + mt * BLOCK_M + quad * 32, row = mrow0 + lane;
+                    const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * BLOCK_N + mt * 256);
+                    // the staging buffer must have been read by this warp's previous TMA stores
+                    if (lane == 0) tma_store_wait_read<0>();
+                    __syncwarp();
+                    uint8_t* out_row = my_epi_ptr + lane * 128;
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        uint32_t pk[4];
-                        glu_glue8(g + 8 * q, u + 8 * q, lin, pk);
-                        const int chunk = q ^ ((lane >> 1) & 3);   // 64-byte swizzle: 16-byte piece ^ address bits 7-8
-                        *reinterpret_cast<uint4*>(my_epi_ptr + lane * 64 + chunk * 16) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                    }
-                }
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    if (glu || (narrow && h != half)) continue;
-                    if (AHEAD && any_glue) {
-                        const int nc = h == 0 ? cc : cc + 2, nh = h ^ 1;
-                        if (!narrow && nc < CHUNKS)
-                            fetch_glue(next, ep, m0 + (nc / CHUNKS_N) * BLOCK_M + quad * 32 + lane, M, n0 + (nc % CHUNKS_N) * 64 + nh * 32, N);
-                    }
-                    uint32_t r[32];
-                    if (from_part) {
-                        // the k ranges added up in their order, whichever unit got here last; a range's 32 loads are
-                        // independent of one another and all in flight before the first add
-                        const float* src = parts + (size_t)(c * 64 + h * 32) * BLOCK_M;
-                        float acc[32];
-#pragma unroll
-                        for (int e = 0; e < 32; ++e) acc[e] = __ldcg(src + e * BLOCK_M);
-                        for (int sp = 1; sp < splits; ++sp) {
-                            src += BLOCK_M * BLOCK_N;
-                            float nxt[32];
-#pragma unroll
-                            for (int e = 0; e < 32; ++e) nxt[e] = __ldcg(src + e * BLOCK_M);
-#pragma unroll
-                            for (int e = 0; e < 32; ++e) acc[e] += nxt[e];
-                        }
-#pragma unroll
-                        for (int e = 0; e < 32; ++e) r[e] = __float_as_uint(acc[e]);
-                    } else {
+                    for (int h = 0; h < 2; ++h) {
+                        uint32_t r[32];
                         tc_ld_32x32(t_row + (uint32_t)(c * 64 + h * 32), r);
                         tc_wait_ld();
-                    }
-                    const int col0 = n0 + c * 64 + h * 32;
-                    // Glue per group of 8 columns (N % 8 == 0, so a group is entirely inside or outside
-                    // the matrix): bias, residual and residual2 arrive as single 16-byte loads.
+                        const int col0 = n0 + c * 64 + h * 32;
+                        // Glue per group of 8 columns (N % 8 == 0, so a group is entirely inside or outside the matrix)
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const int cq = col0 + 8 * q;
-                        uint32_t pk[4];
-                        if constexpr (BF16) {
-                            lin_glue8(r + 8 * q, lin, cq, N, pk);
-                        } else if constexpr (AHEAD) {
-                            epilogue_glue8(r + 8 * q, ep, now, q, any_glue && row < M && cq < N, pk);
-                        } else {
+                        for (int q = 0; q < 4; ++q) {
+                            const int cq = col0 + 8 * q;
+                            uint32_t pk[4];
                             GlueOperands here;
                             if (any_glue) fetch_glue8(here, q, ep, row, M, cq, N);
                             epilogue_glue8(r + 8 * q, ep, here, q, any_glue && row < M && cq < N, pk);
+                            const int chunk = (h * 4 + q) ^ (lane & 7);  // 128-byte swizzle, matches the store map
+                            *reinterpret_cast<uint4*>(out_row + chunk * 16) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
                         }
-                        // 128-byte or 64-byte swizzle, as the store map says
-                        const int chunk = narrow ? q ^ ((lane >> 1) & 3) : (h * 4 + q) ^ (lane & 7);
-                        *reinterpret_cast<uint4*>(out_row + chunk * 16) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
                     }
-                    if (AHEAD) now = next;
-                }
-                if (cc + 2 >= CHUNKS && !from_part) {
-                    // all of this warp's TMEM reads of the tile are done: hand the buffer back
-                    tc_fence_before();
+                    if (cc + 2 >= CHUNKS) {
+                        // all of this warp's TMEM reads of the tile are done: hand the buffer back
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar_tempty + 8 * buf);
+                    }
+                    fence_async_smem();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(bar_tempty + 8 * buf);
-                }
-                fence_async_smem();
-                __syncwarp();
-                if (lane == 0) {
-                    tma_store_2d(&tm_c, my_epi, glu ? (n0 + c * 64) / 2 : narrow ? n0 + half * 32 : n0 + c * 64, mrow0);
-                    if (PUSH && push.tma) {
-                        // the same staged chunk into every peer's C, starting with a different peer in every CTA;
-                        // the staging buffer is reused once all of these stores have read it
-                        for (int pi = 0; pi < push.n; ++pi) {
-                            int peer = pi + (int)blockIdx.x;
-                            peer -= (peer / push.n) * push.n;
-                            tma_store_2d(&pm.m[peer], my_epi, n0 + c * 64, mrow0);
+                    if (lane == 0) {
+                        tma_store_2d(&tm_c, my_epi, n0 + c * 64, mrow0);
+                        if (push.tma) {
+                            // the same staged chunk into every peer's C, starting with a different peer in every CTA;
+                            // the staging buffer is reused once all of these stores have read it
+                            for (int pi = 0; pi < push.n; ++pi) {
+                                int peer = pi + (int)blockIdx.x;
+                                peer -= (peer / push.n) * push.n;
+                                tma_store_2d(&pm.m[peer], my_epi, n0 + c * 64, mrow0);
+                            }
                         }
+                        tma_store_commit();
                     }
-                    tma_store_commit();
+                }
+            } else {
+#pragma unroll 1
+                for (int u = half; u < n_units; u += 2) {
+                    const bool last = CHUNKS == 1 || u + 2 >= n_units;
+                    const int mt = glu ? u / CHUNKS_N : u / (2 * CHUNKS_N);
+                    const int acc_col = glu ? u % CHUNKS_N * 64 : u % (2 * CHUNKS_N) * 32, out_col = glu ? (n0 + acc_col) / 2 : n0 + acc_col;
+                    const int mrow0 = m0 + mt * BLOCK_M + quad * 32, row = mrow0 + lane;
+                    const uint32_t t_acc = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * BLOCK_N + mt * 256 + acc_col);
+                    // two staging buffers a warp: the store of the unit before the last must have read its own.  (With one, every
+                    // 32 columns waited for the store before them: 0.8 us each.)
+                    if (lane == 0) tma_store_wait_read<1>();
+                    __syncwarp();
+                    uint8_t* out_row = my_epi_ptr + stage_buf * (EPI_BUF_BYTES / 2) + lane * 64;
+                    auto put = [&](int q, const uint32_t(&pk)[4]) {     // 64-byte swizzle: 16-byte piece ^ address bits 7-8
+                        *reinterpret_cast<uint4*>(out_row + ((q ^ ((lane >> 1) & 3)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                    };
+                    if (glu) {
+                        uint32_t g[32], up[32];
+                        tc_ld_32x32(t_acc, g);
+                        tc_ld_32x32(t_acc + 32u, up);
+                        tc_wait_ld();
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            uint32_t pk[4];
+                            glu_glue8(g + 8 * q, up + 8 * q, lin, pk);
+                            put(q, pk);
+                        }
+                    } else {
+                        if (AHEAD && any_glue && !last) fetch_unit(next, u + 2);
+                        uint32_t r[32];
+                        if (from_part) {
+                            // the k ranges added up in their order, whichever unit got here last; a range's 32 loads are
+                            // independent of one another and all in flight before the first add
+                            const float* src = parts + (size_t)acc_col * BLOCK_M;
+                            float acc[32];
+#pragma unroll
+                            for (int e = 0; e < 32; ++e) acc[e] = __ldcg(src + e * BLOCK_M);
+                            for (int sp = 1; sp < splits; ++sp) {
+                                src += BLOCK_M * BLOCK_N;
+                                float more[32];
+#pragma unroll
+                                for (int e = 0; e < 32; ++e) more[e] = __ldcg(src + e * BLOCK_M);
+#pragma unroll
+                                for (int e = 0; e < 32; ++e) acc[e] += more[e];
+                            }
+#pragma unroll
+                            for (int e = 0; e < 32; ++e) r[e] = __float_as_uint(acc[e]);
+                        } else {
+                            tc_ld_32x32(t_acc, r);
+                            tc_wait_ld();
+                        }
+                        // Glue per group of 8 columns (N % 8 == 0, so a group is entirely inside or outside the matrix)
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const int cq = out_col + 8 * q;
+                            uint32_t pk[4];
+                            if constexpr (BF16) lin_glue8(r + 8 * q, lin, cq, N, pk);
+                            else epilogue_glue8(r + 8 * q, ep, now, q, any_glue && row < M && cq < N, pk);
+                            put(q, pk);
+                        }
+                        if (AHEAD && CHUNKS > 1) now = next;
+                    }
+                    if (last && !from_part) {
+                        // all of this warp's TMEM reads of the tile are done: hand the buffer back
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar_tempty + 8 * buf);
+                    }
+                    fence_async_smem();
+                    __syncwarp();
+                    if (lane == 0) {
+                        tma_store_2d(&tm_c, my_epi + (uint32_t)(stage_buf * (EPI_BUF_BYTES / 2)), out_col, mrow0);
+                        tma_store_commit();
+                    }
+                    stage_buf ^= 1;
                 }
             }
-            if (first_cc >= CHUNKS && !from_part) {
-                // a warp without a chunk (tile narrower than its share) still releases the accumulator
+            if (half >= n_units && !from_part) {
+                // a warp without a unit (tile narrower than its share) still releases the accumulator
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar_tempty + 8 * buf);
@@ -539,8 +570,7 @@ int launch_as(md_ctx* ctx, const __half* a, const __half* b, __half* c, size_t M
     MD_TRY(make_map_2d(ctx, &tm_a, a, K, M, BLOCK_K, BLOCK_M, lda));
     if (B_MN_MAJOR) MD_TRY(make_map_2d(ctx, &tm_b, b, N, K, 64, BLOCK_K));
     else MD_TRY(make_map_2d(ctx, &tm_b, b, K, N, BLOCK_K, BLOCK_N));
-    constexpr bool NARROW = BLOCK_N == 64 && !PUSH;    // the epilogue's warps then store 32 columns each
-    MD_TRY(make_map_2d(ctx, &tm_c, c, N, M, NARROW ? 32 : 64, 32, ldc, false, NARROW));
+    MD_TRY(make_map_2d(ctx, &tm_c, c, N, M, PUSH ? 64 : 32, 32, ldc, false, !PUSH));
     const int tiles_m = (int)((M + MT * BLOCK_M - 1) / (MT * BLOCK_M)), tiles_n = (int)((N + BLOCK_N - 1) / BLOCK_N);
     const int num_tiles = tiles_m * tiles_n;
     float* part = nullptr;
@@ -588,8 +618,7 @@ int launch_lin(md_ctx* ctx, const void* a, const void* b, void* c, size_t M, siz
     const size_t b_rows = lin.tile_expert ? N * (size_t)lin.n_experts : N;
     MD_TRY(make_map_2d(ctx, &tm_a, a, K, M, BLOCK_K, BLOCK_M, 0, true));
     MD_TRY(make_map_2d(ctx, &tm_b, b, K, b_rows, BLOCK_K, BLOCK_N, 0, true));
-    if (lin.glu) MD_TRY(make_map_2d(ctx, &tm_c, c, N / 2, M, 32, 32, 0, true, true));
-    else MD_TRY(make_map_2d(ctx, &tm_c, c, N, M, BLOCK_N == 64 ? 32 : 64, 32, 0, true, BLOCK_N == 64));
+    MD_TRY(make_map_2d(ctx, &tm_c, c, lin.glu ? N / 2 : N, M, 32, 32, 0, true, true));
     const int tiles_m = (int)((M + MT * BLOCK_M - 1) / (MT * BLOCK_M)), tiles_n = (int)((N + BLOCK_N - 1) / BLOCK_N);
     const int num_tiles = tiles_m * tiles_n, grid = num_tiles < ctx->sm_count ? num_tiles : ctx->sm_count;
     const int early = ctx->pdl && md_launch_early(ctx) && !lin.tile_expert;
@@ -614,6 +643,69 @@ int launch(md_ctx* ctx, const __half* a, const __half* b, __half* c, size_t M, s
     return launch_as<BLOCK_N, B_MN_MAJOR, MT, false>(ctx, a, b, c, M, N, K, ep, ldc, push, lda, splits);
 }
 
+struct TileChoice { int bn = 64, mt = 1; bool pair = false; };
+
+// The tile of a product that covers the machine many times over: the bytes an SM pulls from L2 per k-block, (rows + columns) x 128,
+// decide (there the clock under the power cap follows them too).  Cost = (waves over the SMs) x (rows + columns); the 256 x 256 tile
+// moves ~42 B per cycle against ~55 for the 128-row tiles (three ring stages), hence the factor 1.3, and its epilogue is not hidden
+// behind the next tile's main loop (one accumulator buffer): a fixed cost per tile, larger with glue.  128 x 256 tiles of more than
+// 256 rows run on CTA pairs: the same work per SM with a third less traffic (9477 x 1152 x 4304: 91.1 -> 84.7 us).
+// pushing > 0: the block also has to cross NVLink to that many peers.
+TileChoice choose_tile_large(const md_ctx* ctx, size_t M, size_t N, size_t K, bool glue, int pushing) {
+    const int cand_n[4] = {256, 256, 128, 64}, cand_mt[4] = {2, 1, 1, 1};
+    const double kblocks = (double)((K + BLOCK_K - 1) / BLOCK_K);
+    TileChoice c;
+    double best = -1.0;
+    for (int i = 0; i < 4; ++i) {
+        const size_t rows = (size_t)cand_mt[i] * BLOCK_M;
+        const size_t t = ((M + rows - 1) / rows) * ((N + cand_n[i] - 1) / cand_n[i]);
+        const size_t waves = (t + ctx->sm_count - 1) / ctx->sm_count;
+        const double tile = (double)(rows + cand_n[i]) * kblocks * (cand_mt[i] == 2 ? 1.3 : 1.0) +
+                            (cand_mt[i] == 2 ? (glue ? 7000.0 : 2500.0) : 0.0);
+        double cost = (double)waves * tile;
+        if (pushing > 0) {
+            // ~770 GB/s per direction: in the units of `tile`, 128 bytes pulled from L2 = ~2.5 cycles, about 1000 bytes of link time.
+            // The pushes can start when the first tile is done, and the last wave's tiles are pushed after the math.
+            const double per_byte = 1.0 / 1000.0;
+            const double total_push = (double)M * (double)N * 2.0 * pushing * per_byte;
+            const size_t last_wave = t - (waves - 1) * (size_t)ctx->sm_count;
+            const double tail_push = (double)last_wave * (double)(rows * cand_n[i]) * 2.0 * pushing * per_byte;
+            const double through = tile + total_push;
+            cost = cost + tail_push > through ? cost + tail_push : through;
+        }
+        if (best < 0.0 || cost < best) { best = cost; c.bn = cand_n[i]; c.mt = cand_mt[i]; }
+    }
+    c.pair = c.bn == 256 && c.mt == 1 && M > 256;
+    return c;
+}
+
+// The tile of a product of few waves, from what each tile takes on its own (us): a fixed part (start, first loads, the last
+// epilogue), per wave the k-blocks and what the next tile's main loop does not hide, and for all of them together what L2 delivers
+// (about 20 TB/s).  Measured back to back with cold weights (us; 64 and 128 columns, 128 x 256, pair of 256 x 256):
+//   729 x 3456 x 1152 bias 11.4, 11.2, 11.8, 12.9     761 x 2048 x 2048 residuals 12.3, 11.3, 18.4, 19.1
+//   729 x 1152 x 1152 residual 5.9, 7.5, 12.4, 13.7   761 x 8192 x 2048 GELU 33.1, 26.3, 29.4, 28.8
+//   1458 x 4304 x 1152 GELU 21.1, 17.7, 20.9, 19.2    300 x 9536 x 2048 21.0, 17.0, 16.1, 24.3
+//   2048 x 2048 x 4768 67.8, 46.9, 38.2, 33.0         300 x 2048 x 4768 15.0, 18.8, 30.7, 27.4
+// Above 300 tiles of 128 x 256 the rule above holds.
+TileChoice choose_tile(const md_ctx* ctx, size_t M, size_t N, size_t K, bool glue) {
+    if (((M + BLOCK_M - 1) / BLOCK_M) * ((N + 255) / 256) > 2 * (size_t)ctx->sm_count) return choose_tile_large(ctx, M, N, K, glue, 0);
+    struct Tile { int bn, mt; bool pair; double kb, fixed, wave, with_glue; };
+    static const Tile tiles[5] = {{64, 1, false, 0.14, 2.9, 0.15, 0.3}, {128, 1, false, 0.165, 3.7, 0.4, 0.6}, {256, 1, false, 0.28, 5.1, 0.3, 1.2},
+                                  {256, 1, true, 0.29, 5.1, 0.3, 1.2}, {256, 2, false, 0.55, 5.8, 4.2, 2.0}};
+    const double kblocks = (double)((K + BLOCK_K - 1) / BLOCK_K);
+    TileChoice c;
+    double best = -1.0;
+    for (const Tile& t : tiles) {
+        if (t.pair && (M <= BLOCK_M || ctx->tc_pair == 0)) continue;
+        const size_t rows = (t.pair ? 2 : t.mt) * BLOCK_M, at_once = t.pair ? ctx->sm_count / 2 : ctx->sm_count;
+        const size_t n = ((M + rows - 1) / rows) * ((N + t.bn - 1) / t.bn), waves = (n + at_once - 1) / at_once;
+        const double l2 = (double)n * kblocks * (double)(rows + t.bn) * BLOCK_K * 2 / 20e6, sm = (double)waves * (kblocks * t.kb + t.wave);
+        const double cost = t.fixed + (glue ? t.with_glue : 0.0) + (l2 > sm ? l2 : sm);
+        if (best < 0.0 || cost < best) { best = cost; c.bn = t.bn; c.mt = t.mt; c.pair = t.pair; }
+    }
+    return c;
+}
+
 }  // namespace
 
 bool md_gemm_tc_supported(const void* a, const void* b, const void* c, size_t M, size_t N, size_t K, int b_layout) {
@@ -635,26 +727,17 @@ int md_launch_gemm_tc(md_ctx* ctx, const __half* a, const __half* b, __half* c, 
 int md_launch_gemm_tc_lin(md_ctx* ctx, const void* a, const void* b, void* c, size_t M, size_t N, size_t K, const md_lin& lin) {
     if (!md_gemm_tc_supported(a, b, c, M, N, K, 1) || lin.out_f32)
         return md_fail(ctx, MD_ERR_UNSUPPORTED, "tcgen05 GEMM needs K %% 8 == 0, N %% 8 == 0, 16-byte aligned operands and a 16-bit output");
-    int bn = 64, mt = 1;
     if (lin.tile_expert) {
         // the number of row blocks is only known on the device: enough of them to fill the machine with wide tiles, or narrow ones
         const size_t blocks = (M + BLOCK_M - 1) / BLOCK_M;
-        bn = blocks * ((N + 255) / 256) >= 2 * (size_t)ctx->sm_count ? 256 : blocks * ((N + 127) / 128) >= (size_t)ctx->sm_count ? 128 : 64;
-    } else {
-        // the same cost as for f16 operands (see md_launch_gemm_tc_ex)
-        const int cand_n[4] = {256, 256, 128, 64}, cand_mt[4] = {2, 1, 1, 1};
-        double best = -1.0;
-        for (int i = 0; i < 4; ++i) {
-            const size_t rows = (size_t)cand_mt[i] * BLOCK_M;
-            const size_t t = ((M + rows - 1) / rows) * ((N + cand_n[i] - 1) / cand_n[i]);
-            const size_t waves = (t + ctx->sm_count - 1) / ctx->sm_count;
-            const double kblocks = (double)((K + BLOCK_K - 1) / BLOCK_K);
-            const double cost = (double)waves * ((double)(rows + cand_n[i]) * kblocks * (cand_mt[i] == 2 ? 1.3 : 1.0) +
-                                                 (cand_mt[i] == 2 ? 7000.0 : 0.0));
-            if (best < 0.0 || cost < best) { best = cost; bn = cand_n[i]; mt = cand_mt[i]; }
-        }
-        if (bn == 256 && mt == 1 && M > 256 && ctx->tc_pair != 0) return md_launch_gemm_pair_lin(ctx, a, b, c, M, N, K, lin);
+        const int bn = blocks * ((N + 255) / 256) >= 2 * (size_t)ctx->sm_count ? 256 : blocks * ((N + 127) / 128) >= (size_t)ctx->sm_count ? 128 : 64;
+        if (bn == 256) return launch_lin<256, 1>(ctx, a, b, c, M, N, K, lin);
+        if (bn == 128) return launch_lin<128, 1>(ctx, a, b, c, M, N, K, lin);
+        return launch_lin<64, 1>(ctx, a, b, c, M, N, K, lin);
     }
+    const TileChoice t = choose_tile(ctx, M, N, K, lin.bias || lin.glu || lin.silu_cols || lin.sigmoid_from < (int)N);
+    if (t.pair && ctx->tc_pair != 0) return md_launch_gemm_pair_lin(ctx, a, b, c, M, N, K, lin);
+    const int bn = t.bn, mt = t.mt;
     if (mt == 2) return launch_lin<256, 2>(ctx, a, b, c, M, N, K, lin);
     if (bn == 256) return launch_lin<256, 1>(ctx, a, b, c, M, N, K, lin);
     if (bn == 128) return launch_lin<128, 1>(ctx, a, b, c, M, N, K, lin);
@@ -671,45 +754,16 @@ int md_launch_gemm_tc_ex(md_ctx* ctx, const __half* a, const __half* b, __half* 
         return md_fail(ctx, MD_ERR_UNSUPPORTED, "tcgen05 GEMM: residuals are not supported with a strided output");
     if (!md_gemm_tc_supported(a, b, c, M, N, K, b_layout) || !md_glue_aligned(ep))
         return md_fail(ctx, MD_ERR_UNSUPPORTED, "tcgen05 GEMM needs K %% 8 == 0, N %% 8 == 0 and 16-byte aligned operands");
-    // Tile shape.  The kernel is bound by the bytes an SM pulls from L2 per k-block, (rows + columns) x 128,
-    // so a tile's time is proportional to its rows + columns: 128 x 64, 128 x 128, 128 x 256, or 256 x 256 (two
-    // 128-row sub-tiles sharing one B tile).  Cost = (waves over the SMs) x (rows + columns).  Skinny problems
-    // (M <= 64) are HBM-bound and take the narrowest tile to get many CTAs streaming B.
-    int bn = 64, mt = 1;
-    if (M > 64) {
-        const int cand_n[4] = {256, 256, 128, 64}, cand_mt[4] = {2, 1, 1, 1};
-        double best = -1.0;
-        for (int i = 0; i < 4; ++i) {
-            const size_t rows = (size_t)cand_mt[i] * BLOCK_M;
-            const size_t t = ((M + rows - 1) / rows) * ((N + cand_n[i] - 1) / cand_n[i]);
-            const size_t waves = (t + ctx->sm_count - 1) / ctx->sm_count;
-            // per tile: (rows + columns) per k-block; measured, the 256 x 256 tile moves ~42 B per cycle against
-            // ~55 for the 128-row tiles (three ring stages), hence the factor 1.3, and its epilogue is not hidden
-            // behind the next tile's main loop (one accumulator buffer): a fixed cost per tile, larger with glue
-            const double kblocks = (double)((K + BLOCK_K - 1) / BLOCK_K);
-            const bool glue = ep.bias || ep.gelu || ep.residual || ep.residual2;
-            const double tile = (double)(rows + cand_n[i]) * kblocks * (cand_mt[i] == 2 ? 1.3 : 1.0) +
-                                (cand_mt[i] == 2 ? (glue ? 7000.0 : 2500.0) : 0.0);
-            double cost = (double)waves * tile;
-            if (push.n > 0) {
-                // Column-split GEMM: the block also has to cross NVLink to every peer (~770 GB/s per direction: in
-                // the units of `tile`, 128 bytes pulled from L2 = ~2.5 cycles, about 1000 bytes of link time).  The
-                // pushes can start when the first tile is done, and the last wave's tiles are pushed after the math.
-                const double per_byte = 1.0 / 1000.0;
-                const double total_push = (double)M * (double)N * 2.0 * push.n * per_byte;
-                const size_t last_wave = t - (waves - 1) * (size_t)ctx->sm_count;
-                const double tail_push = (double)last_wave * (double)(rows * cand_n[i]) * 2.0 * push.n * per_byte;
-                const double through = tile + total_push;
-                cost = cost + tail_push > through ? cost + tail_push : through;
-            }
-            if (best < 0.0 || cost < best) { best = cost; bn = cand_n[i]; mt = cand_mt[i]; }
-        }
-    }
+    // Skinny problems (M <= 64) are HBM-bound and take the narrowest tile to get many CTAs streaming B.
+    const bool glue = ep.bias || ep.gelu || ep.residual || ep.residual2;
+    TileChoice t;
+    if (M > 64) t = push.n > 0 ? choose_tile_large(ctx, M, N, K, glue, push.n) : choose_tile(ctx, M, N, K, glue);
+    int bn = t.bn, mt = t.mt;
     // Column-split products with rows for both CTAs of a pair and at least one 256-wide tile take the pair kernel
     // whatever the search above found: measured at 8 GPUs (8192 x 1024 x 8192 per rank, seven peers) 265 us on pairs
     // against 289-292 us on 128 x 128, 128 x 256 or 256 x 256 single-CTA tiles; at 2 and 4 GPUs the search picks the
     // 128 x 256 tile, and with it the pairs, by itself.
-    if (push.n > 0 && M > 256 && N >= 256 && !ctx->tc_block_n && ctx->tc_pair < 0) { bn = 256; mt = 1; }
+    if (push.n > 0 && M > 256 && N >= 256 && !ctx->tc_block_n && ctx->tc_pair < 0) { bn = 256; mt = 1; t.pair = true; }
     // Split K (md_set_option("tc_splitk"), off by default: inside the forked prefill layer the other chain's kernels
     // already use the SMs such a product leaves idle, and the whole prefill measured 3.13 ms without against 3.27 ms
     // with it).  With fewer 128 x 256 tiles than SMs and a long K (the 2048-wide outputs of a 761-row prefill, the
@@ -743,12 +797,8 @@ int md_launch_gemm_tc_ex(md_ctx* ctx, const __half* a, const __half* b, __half* 
         if (b_layout == 0) return launch<256, true>(ctx, a, b, c, M, N, K, ep, ldc, push, lda, splits);
         return launch<256, false>(ctx, a, b, c, M, N, K, ep, ldc, push, lda, splits);
     }
-    // CTA pairs (gemm_pair.cu): where the single-CTA choice is the 128 x 256 tile and there are rows for both CTAs of
-    // a pair, the pair's 256 x 256 tile does the same work per SM with a third less traffic from L2 and measured
-    // 1 to 12 % faster (761 x 8192 x 2048: 34.8 -> 31.2 us; 9477 x 1152 x 4304: 91.1 -> 84.7 us); with the other
-    // choices it lost.  md_set_option("tc_pair"): 1 = always, 0 = never.
-    if (!ctx->tc_block_n &&
-        (ctx->tc_pair == 1 || (ctx->tc_pair < 0 && bn == 256 && mt == 1 && M > 256)))
+    // md_set_option("tc_pair"): 1 = CTA pairs always, 0 = never
+    if (!ctx->tc_block_n && (ctx->tc_pair == 1 || (ctx->tc_pair < 0 && t.pair)))
         return md_launch_gemm_pair(ctx, a, b, c, M, N, K, b_layout, ep, ldc, push, lda);
     if (ctx->tc_block_n) {  // forced: 512 = the 256 x 256 tile
         bn = ctx->tc_block_n == 512 ? 256 : ctx->tc_block_n;
@@ -767,10 +817,10 @@ int md_launch_gemm_tc_ex(md_ctx* ctx, const __half* a, const __half* b, __half* 
     return launch<64, false>(ctx, a, b, c, M, N, K, ep, ldc, push, lda);
 }
 
-// 2-D f16 tensor map with 128-byte swizzle for other translation units (the attention kernel).
+// 2-D f16 tensor map with 128-byte (or 64-byte) swizzle for other translation units.
 int md_make_map_2d(md_ctx* ctx, CUtensorMap* map, const void* ptr, uint64_t inner, uint64_t outer, uint32_t box_inner,
-                   uint32_t box_outer, uint64_t ld) {
-    return make_map_2d(ctx, map, ptr, inner, outer, box_inner, box_outer, ld);
+                   uint32_t box_outer, uint64_t ld, bool swizzle_64) {
+    return make_map_2d(ctx, map, ptr, inner, outer, box_inner, box_outer, ld, false, swizzle_64);
 }
 int md_make_map_2d_bf16(md_ctx* ctx, CUtensorMap* map, const void* ptr, uint64_t inner, uint64_t outer, uint32_t box_inner,
                         uint32_t box_outer, bool swizzle_64) {
