@@ -800,6 +800,8 @@ struct MixParams {
     const __half *x, *w;              // [M][K], [N][K]
     float* part;                      // [parts][8 * N]
     int M, N, K, per_part;            // columns per part, a multiple of 32
+    int units;                        // CTAs of the product
+    md_ahead ahead;                   // requested by each of them behind its own weights
 };
 
 constexpr int MIX_WARPS = 8;
@@ -826,6 +828,7 @@ __device__ __forceinline__ void mix_product(const MixParams& p, int unit) {
             hi[u] = c < chunks ? ldg_nc16(w_hi + c * 32) : zero;
         }
         if (!waited) {
+            if (tid == 0) md_fetch_ahead(p.ahead, unit, p.units);
             asm volatile("griddepcontrol.wait;" ::: "memory");
             asm volatile("griddepcontrol.launch_dependents;");
         }
@@ -1214,7 +1217,7 @@ bool md_decode_mix_supported(size_t batch, size_t n_heads, size_t d, size_t N, s
 int md_launch_decode_mix_out(md_ctx* ctx, const __half* qkv, size_t qkv_stride, __half* const* kc, __half* const* vc, __half* attn,
                              size_t batch, size_t n_heads, size_t d, size_t max_seq, const int* const* pos_dev, size_t rot_dim, float theta,
                              const __half* x, const __half* w, float* part, size_t N, size_t K, size_t parts, const __half* w_out,
-                             __half* out, const md_epilogue& ep) {
+                             __half* out, const md_epilogue& ep, const md_ahead& ahead) {
     if (!md_decode_mix_supported(batch, n_heads, d, N, K) || rot_dim > DEC_D || !ep.bias || !ep.parts || !ep.bias2 || !ep.residual2 ||
         ep.gelu || ep.residual)
         return md_fail(ctx, MD_ERR_UNSUPPORTED, "decode_mix_out: unsupported shape");
@@ -1234,7 +1237,9 @@ int md_launch_decode_mix_out(md_ctx* ctx, const __half* qkv, size_t qkv_stride, 
     p.x = x; p.w = w; p.part = part;
     p.M = (int)batch; p.N = (int)N; p.K = (int)K;
     p.per_part = (int)((K / 32 + parts - 1) / parts * 32);
-    MD_TRY(md_launch_ex(ctx, decode_mix_kernel, dim3((unsigned)(p.attn_ctas + N / 16 * parts)), dim3(MIX_WARPS * 32), 0, "decode_mix_kernel", p));
+    p.units = (int)(N / 16 * parts);
+    p.ahead = ahead;
+    MD_TRY(md_launch_ex(ctx, decode_mix_kernel, dim3((unsigned)(p.attn_ctas + p.units)), dim3(MIX_WARPS * 32), 0, "decode_mix_kernel", p));
     OutParams o{};
     o.x = attn; o.w = w_out; o.out = out; o.ep = ep;
     o.M = (int)batch; o.N = (int)N;

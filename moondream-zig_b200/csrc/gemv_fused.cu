@@ -79,6 +79,7 @@ struct LnDualParams {
     int n1, n2, M;
     unsigned long long* amax;        // optional [M]: running argmax keys of out1 (greedy sampling), see below
     int gelu1;                       // GELU on segment 1 as well (fc1 alone as segment 1)
+    md_ahead ahead;                  // requested beside a CTA's last tile (beside its first they hold the others up)
 };
 
 // ONE: a single row, normalised by the whole CTA; else up to eight, a warp each.
@@ -216,6 +217,7 @@ gemv_ln_dual_kernel(LnDualParams p, int R) {
     int buf = 0;
     for (int row0 = first; row0 < end; row0 += 16, buf ^= 1) {
         const float own_bias = bias;
+        if (tid == 0 && row0 + 16 >= end) md_fetch_ahead(p.ahead, blockIdx.x, gridDim.x);
         locate(row0 + 16);
         float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -373,7 +375,7 @@ bool md_gemv_ln_dual_supported(size_t M, size_t K, size_t n1, size_t n2) {
 int md_launch_gemv_ln_dual(md_ctx* ctx, const __half* hidden, const __half* ln_w, const __half* ln_b, float eps,
                            const __half* w1, const __half* b1, __half* out1, size_t n1, const __half* w2,
                            const __half* b2, __half* out2, size_t n2, size_t M, size_t K, unsigned long long* amax,
-                           bool gelu1) {
+                           bool gelu1, const md_ahead& ahead) {
     if (!md_gemv_ln_dual_supported(M, K, n1, n2))
         return md_fail(ctx, MD_ERR_UNSUPPORTED, "gemv_ln_dual: unsupported shape M=%zu K=%zu n1=%zu n2=%zu", M, K, n1, n2);
     LnDualParams p;
@@ -382,6 +384,7 @@ int md_launch_gemv_ln_dual(md_ctx* ctx, const __half* hidden, const __half* ln_w
     p.n1 = (int)n1; p.n2 = (int)n2; p.M = (int)M;
     p.amax = amax;
     p.gelu1 = gelu1 ? 1 : 0;
+    p.ahead = ahead;
     // an equal share for every CTA that fits at once, in rows (fewer tiles than that: one each)
     const int total = (int)(n1 + n2), ctas = 2 * ctx->sm_count;
     const int R = total / 16 < ctas ? 16 : (total + ctas - 1) / ctas;

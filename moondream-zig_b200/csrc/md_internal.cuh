@@ -205,6 +205,17 @@ int md_finish_out(md_ctx* ctx, md_arg* out);
 int md_check_flags(md_ctx* ctx);
 
 // ---- kernel launchers (device pointers only) ------------------------------------
+// Weights that later kernels of a decode step read, brought into L2 by an earlier one: while a chain of small kernels waits for its
+// own results memory would stand still, and with it the weights that come next whatever those results are.
+struct md_ahead {
+    const char* p = nullptr;
+    unsigned bytes = 0;
+    md_ahead() = default;
+    md_ahead(const void* w, size_t n) {      // at least n bytes lie there
+        if ((reinterpret_cast<uintptr_t>(w) & 15) == 0) p = reinterpret_cast<const char*>(w), bytes = (unsigned)(n & ~(size_t)15);
+    }
+};
+
 struct md_epilogue {
     const __half* bias = nullptr;       // [N] or null
     const __half* residual = nullptr;   // [M,N] (or [residual_rows,N] repeated every residual_rows rows) or null
@@ -249,7 +260,8 @@ int md_launch_gemv_ln_dual(md_ctx* ctx, const __half* hidden, const __half* ln_w
                            const __half* w1, const __half* b1, __half* out1, size_t n1, const __half* w2,
                            const __half* b2, __half* out2, size_t n2, size_t M, size_t K,
                            unsigned long long* amax = nullptr,  // amax: optional [M] argmax keys of out1
-                           bool gelu1 = false);                 // GELU on segment 1 too
+                           bool gelu1 = false,                  // GELU on segment 1 too
+                           const md_ahead& ahead = md_ahead());
 bool md_gemv_dual_k_supported(size_t M, size_t N, size_t k1, size_t k2);
 int md_launch_gemv_dual_k(md_ctx* ctx, const __half* x1, const __half* w1, const __half* b1, size_t k1,
                           const __half* x2, const __half* w2, const __half* b2, size_t k2, __half* hidden, size_t N,
@@ -332,6 +344,12 @@ int md_launch_kv_active(md_ctx* ctx, const __half* kc, const __half* vc, __half*
 
 // ---- device helpers ----------------------------------------------------------------
 #ifdef __CUDACC__
+// By one thread of block `me` of `n`: this block's share of the weights ahead.  A hint: no result depends on it.
+__device__ __forceinline__ void md_fetch_ahead(const md_ahead& a, unsigned me, unsigned n) {
+    constexpr unsigned PIECE = 16384;
+    for (unsigned at = me * PIECE; at < a.bytes; at += n * PIECE)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a.p + at), "r"(min(PIECE, a.bytes - at)) : "memory");
+}
 // The reference's rounding points for the glue fused into GEMM epilogues.
 __device__ __forceinline__ float md_round_f16(float v) { return __half2float(__float2half_rn(v)); }
 

@@ -16,7 +16,7 @@ bool md_decode_mix_supported(size_t batch, size_t n_heads, size_t d, size_t N, s
 int md_launch_decode_mix_out(md_ctx* ctx, const __half* qkv, size_t qkv_stride, __half* const* kc, __half* const* vc, __half* attn,
                              size_t batch, size_t n_heads, size_t d, size_t max_seq, const int* const* pos_dev, size_t rot_dim, float theta,
                              const __half* x, const __half* w, float* part, size_t N, size_t K, size_t parts, const __half* w_out,
-                             __half* out, const md_epilogue& ep);
+                             __half* out, const md_epilogue& ep, const md_ahead& ahead);
 int md_launch_sdpa_decode_fused_devpos_batch(md_ctx* ctx, const __half* qkv, size_t qkv_stride, __half* const* kc,
                                              __half* const* vc, __half* out, size_t out_stride, size_t batch,
                                              size_t n_heads, size_t d, size_t max_seq, const int* const* pos_dev,
@@ -193,9 +193,17 @@ int text_layer(md_text_model* m, size_t layer, const LayerIO& io, size_t rows, b
         // Three kernels in one chain, each started under its predecessor with its first weights requested:
         //   [LayerNorm + qkv, fc1 + GELU] -> [attention, fc2 in four parts of its K sum] -> [out-proj + bias + the parts + hidden]
         // Same rounding points as below.
-        constexpr size_t PARTS = 4;
+        // The first kernel also brings the end of fc2's weights into L2 (its last CTAs read them), the second the beginning of the
+        // next layer's fc1 (of the head's, behind the last layer): 16 MB each, about what memory delivers between two kernels' streams.
+        // 32 steps of 1, 3 and 8 requests 19.6, 25.4, 29.7 ms -> 18.7, 24.8, 29.3; with 8 MB each 18.9, with the second alone 19.2.
+        constexpr size_t PARTS = 4, AHEAD = (size_t)16 << 20;
+        const size_t fc2_bytes = D * F * 2, end = std::min(fc2_bytes, AHEAD) & ~(size_t)15;
+        const bool last = layer + 1 == w.n_layers;
+        const md_ahead to_fc2(reinterpret_cast<const char*>(m->wfc2[layer]) + (fc2_bytes - end), end);
+        const md_ahead to_next(last ? w.lm_w : m->wfc1[layer + 1], std::min(AHEAD, (last ? w.vocab : F) * D * 2));
         MD_TRY(md_launch_gemv_ln_dual(ctx, io.hidden, H(m->ln_w[layer]), H(m->ln_b[layer]), eps_of(w.eps_f16), H(m->wqkv[layer]),
-                                      H(m->bqkv[layer]), io.qkv, 3 * D, H(m->wfc1[layer]), H(m->bfc1[layer]), io.fc1, F, rows, D));
+                                      H(m->bqkv[layer]), io.qkv, 3 * D, H(m->wfc1[layer]), H(m->bfc1[layer]), io.fc1, F, rows, D,
+                                      nullptr, false, to_fc2));
         __half *kc[8], *vc[8];
         const int* pos[8];
         for (size_t b = 0; b < rows; ++b) {
@@ -211,7 +219,7 @@ int text_layer(md_text_model* m, size_t layer, const LayerIO& io, size_t rows, b
         e_out.bias2 = H(m->bfc2[layer]);
         e_out.residual2 = io.hidden;    // updated in place: every element is read and written by one thread
         return md_launch_decode_mix_out(ctx, io.qkv, 3 * D, kc, vc, io.attn, rows, w.n_heads, w.head_dim, w.max_seq, pos, w.rot_dim,
-                                        w.rope_theta, io.fc1, H(m->wfc2[layer]), io.mlp_part, D, F, PARTS, H(m->wout[layer]), io.hidden, e_out);
+                                        w.rope_theta, io.fc1, H(m->wfc2[layer]), io.mlp_part, D, F, PARTS, H(m->wout[layer]), io.hidden, e_out, to_next);
     }
     if (decode && ctx->fused_decode && !ln_once && md_gemv_ln_dual_supported(rows, D, 3 * D, F) &&
         md_gemv_dual_k_supported(rows, D, D, F)) {
