@@ -948,6 +948,7 @@ int launch_decode(md_ctx* ctx, const md_latent& a) {
     const int D = a.dim, R = a.kv_rank, rot = a.rot, H = a.heads;
     const int row_blocks = (H * (D + rot) + 15) / 16;
     MD_TRY(md_launch_ex(ctx, latent_query_kernel, dim3((unsigned)(row_blocks + a.seqs)), dim3(UQ_WARPS * 32), 0, "latent_query_kernel", a, row_blocks));
+    if (a.queried) MD_CUDA(ctx, cudaEventRecord(a.queried, ctx->stream));
     MD_TRY(md_launch_ex(ctx, latent_absorb_kernel, dim3((unsigned)((R + 15) / 16), (unsigned)H), dim3(HEADS_WARPS * 32), 0, "latent_absorb_kernel", a));
     if (R <= 128) return launch_decode_as<64, 2>(ctx, a);
     if (R <= 256) return launch_decode_as<64, 4>(ctx, a);
@@ -970,6 +971,7 @@ int md_launch_rotation_table(md_ctx* ctx, float* table, size_t rows, size_t dims
 int md_launch_latent_attention(md_ctx* ctx, int dtype, const md_latent& a, bool decode) {
     const bool f32 = dtype == MD_DTYPE_F32;
     if (!f32 && decode && a.rows == 1 && decode_ok(a)) return launch_decode(ctx, a);
+    if (a.queried) MD_CUDA(ctx, cudaEventRecord(a.queried, ctx->stream));
     MD_TRY(f32 ? launch_norm<float>(ctx, a) : launch_norm<__nv_bfloat16>(ctx, a));
     const size_t rows = (size_t)a.rows * a.seqs;
     MD_TRY(md_linear(ctx, dtype, a.cq, a.w_uq, a.q, rows, (size_t)a.heads * (a.dim + a.rot), a.q_rank, md_lin()));

@@ -224,48 +224,28 @@ gemv_lin_kernel(const __half* A, const __half* __restrict__ Bt, __nv_bfloat16* C
     const int chunks = K / 32;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
     md_pdl_launch_dependents();
-    bool waited = false;
-    int ch = warp;
-    for (; ch + (UNROLL - 1) * WARPS < chunks; ch += UNROLL * WARPS) {
-        uint4 lo[UNROLL], hi[UNROLL], xv[UNROLL];
+    // UNROLL chunks stay in flight per lane: as soon as one is multiplied its registers take the request a round later.  (A round
+    // requested together and then waited for left a gap in the stream after each.  One Nuvezen chat 23.0 -> 22.75 ms, eight Korupel
+    // chats 38.55 -> 38.3.)
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    uint4 lo[UNROLL], hi[UNROLL], xv[UNROLL];
+    auto weights = [&](int u, int c) {
+        lo[u] = c < chunks ? ldg_stream(w_lo + c * 32) : zero;
+        hi[u] = c < chunks ? ldg_stream(w_hi + c * 32) : zero;
+    };
+    auto tokens = [&](int u, int c) { xv[u] = has_x && c < chunks ? ld_act(x + c * 32) : zero; };
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u) weights(u, warp + u * WARPS);
+    md_pdl_wait();
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u) tokens(u, warp + u * WARPS);
+    for (int ch = warp; ch < chunks; ch += UNROLL * WARPS) {
 #pragma unroll
         for (int u = 0; u < UNROLL; ++u) {
-            const int k = (ch + u * WARPS) * 32;
-            lo[u] = ldg_stream(w_lo + k);
-            hi[u] = ldg_stream(w_hi + k);
-        }
-        if (!waited) {
-            md_pdl_wait();
-            waited = true;
-        }
-#pragma unroll
-        for (int u = 0; u < UNROLL; ++u) xv[u] = has_x ? ld_act(x + (ch + u * WARPS) * 32) : make_uint4(0, 0, 0, 0);
-#pragma unroll
-        for (int u = 0; u < UNROLL; ++u) {
-            mma_16816_bf16(acc, lo[u].x, hi[u].x, lo[u].y, hi[u].y, xv[u].x, xv[u].y);
+            mma_16816_bf16(acc, lo[u].x, hi[u].x, lo[u].y, hi[u].y, xv[u].x, xv[u].y);     // zeros past the end
             mma_16816_bf16(acc, lo[u].z, hi[u].z, lo[u].w, hi[u].w, xv[u].z, xv[u].w);
-        }
-    }
-    // what is left of K: up to UNROLL - 1 chunks per warp, requested together
-    {
-        uint4 lo[UNROLL], hi[UNROLL], xv[UNROLL];
-#pragma unroll
-        for (int u = 0; u < UNROLL - 1; ++u) {
-            const int c = ch + u * WARPS;
-            const bool live = c < chunks;
-            lo[u] = live ? ldg_stream(w_lo + c * 32) : make_uint4(0, 0, 0, 0);
-            hi[u] = live ? ldg_stream(w_hi + c * 32) : make_uint4(0, 0, 0, 0);
-        }
-        if (!waited) md_pdl_wait();
-#pragma unroll
-        for (int u = 0; u < UNROLL - 1; ++u) {
-            const int c = ch + u * WARPS;
-            xv[u] = has_x && c < chunks ? ld_act(x + c * 32) : make_uint4(0, 0, 0, 0);
-        }
-#pragma unroll
-        for (int u = 0; u < UNROLL - 1; ++u) {
-            mma_16816_bf16(acc, lo[u].x, hi[u].x, lo[u].y, hi[u].y, xv[u].x, xv[u].y);
-            mma_16816_bf16(acc, lo[u].z, hi[u].z, lo[u].w, hi[u].w, xv[u].z, xv[u].w);
+            weights(u, ch + (UNROLL + u) * WARPS);
+            tokens(u, ch + (UNROLL + u) * WARPS);
         }
     }
     if (warp == 0 && chunks * 32 < K) {   // K % 32 != 0, still a multiple of 8

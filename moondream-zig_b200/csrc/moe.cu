@@ -499,8 +499,10 @@ int launch_few(md_ctx* ctx, const md_moe& m, const void* h, size_t rows, const m
     r.expert = reinterpret_cast<int*>(r.weight + 8 * (size_t)EA);
     const __nv_bfloat16* x = reinterpret_cast<const __nv_bfloat16*>(h);
     __nv_bfloat16* act = reinterpret_cast<__nv_bfloat16*>(b.act);
-    MD_TRY(md_launch_ex(ctx, moe_route_kernel, dim3((unsigned)((EA + 15) / 16)), dim3(512), 16 * (size_t)EA * sizeof(float), "moe_route_kernel",
-                        x, reinterpret_cast<const __nv_bfloat16*>(m.router), T, m.width, E, EA - E, m.top, m.router_kind, r));
+    if (m.part != md_moe::REST)
+        MD_TRY(md_launch_ex(ctx, moe_route_kernel, dim3((unsigned)((EA + 15) / 16)), dim3(512), 16 * (size_t)EA * sizeof(float), "moe_route_kernel",
+                            x, reinterpret_cast<const __nv_bfloat16*>(m.router), T, m.width, E, EA - E, m.top, m.router_kind, r));
+    if (m.part == md_moe::ROUTE) return MD_OK;
     const FewShared sh = {reinterpret_cast<const __nv_bfloat16*>(m.shared_gu), reinterpret_cast<const __nv_bfloat16*>(m.shared_down),
                           m.shared_pad, m.shared_limit};
     auto up = m.width <= 2048 ? moe_up_kernel<8, true> : moe_up_kernel<4, false>;
@@ -565,6 +567,7 @@ int md_launch_moe(md_ctx* ctx, int dtype, const md_moe& m, const void* h, size_t
     if (m.experts > MAX_EXPERTS || m.top > MAX_TOP || m.top > m.experts)
         return md_fail(ctx, MD_ERR_UNSUPPORTED, "mixture of experts: %d experts, %d per token", m.experts, m.top);
     if (!md_moe_sorted(dtype, m.width, rows)) return launch_few(ctx, m, h, rows, b);
+    if (m.part == md_moe::ROUTE) return MD_OK;
     return dtype == MD_DTYPE_F32 ? launch_sorted<float>(ctx, dtype, m, h, rows, b)
                                  : launch_sorted<__nv_bfloat16>(ctx, dtype, m, h, rows, b);
 }

@@ -133,6 +133,7 @@ struct md_latent {
     int heads = 0, dim = 0, rot = 0, vdim = 0, q_rank = 0, kv_rank = 0;
     float scale = 0.f, eps = 0.f;
     int window = 0;                         // <= 0: unlimited
+    cudaEvent_t queried = nullptr;          // recorded once the queries are there (one token per sequence) or before anything is launched
     const float *q_norm = nullptr, *kv_norm = nullptr, *sink = nullptr;
     const float* rope = nullptr;            // [max_seq][rot / 2] (cos, sin)
     const void* w_uq = nullptr;             // [heads * (dim + rot), q_rank]: per head [dim | rot]
@@ -192,6 +193,7 @@ struct md_moe {
     int shared_pad = 0;
     float shared_limit = 0.f;
     const void *shared_gu = nullptr, *shared_down = nullptr;            // [2 shared_pad, W], [W, shared_pad]
+    enum Part { ALL, ROUTE, REST } part = ALL;   // of a few rows: the router's kernel alone, or what follows it (for others ROUTE is nothing)
     int choices() const { return top + (shared_pad > 0 ? 1 : 0); }      // entries of a token in score and slot
 };
 struct md_moe_buffers {
