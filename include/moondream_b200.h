@@ -101,8 +101,9 @@ int md_set_gemm_mode(md_ctx* ctx, int mode);
  *   "skinny"        1 (default) = products with 8 < M <= 64 rows take the swapped-operand split-K kernel (weights on
  *                   the MMA's M side, K split over the CTAs of a thread-block cluster, ~2 CTAs per SM, partials
  *                   added through distributed shared memory), but for wide f16 ones of 32 rows and more with a short K and
- *                   no GELU, where the general kernel is the faster one
- *   "skinny_splits" -1 (default): that kernel is taken by shape; else it is taken wherever it can be, with an automatic (0) or
+ *                   no GELU, where the general kernel is the faster one; so do f16 products of 65 to 1024 rows with few
+ *                   columns and a long K, 64 rows per CTA, while the tcgen05 options above are at their defaults
+ *   "skinny_splits" -1 (default): that kernel is taken by shape; else it is taken wherever it can be for up to 64 rows, with an automatic (0) or
  *                   this number of K splits (rounded down to 1, 2, 4 or 8)
  *   "pdl"           1 = launch the GEMV kernels with programmatic dependent launch: a kernel starts
  *                   streaming its weights while its predecessor on the stream drains.  Only for streams

@@ -1,4 +1,5 @@
-// Skinny GEMM for sm_100a: C[M,N] = A[M,K] . B with 8 < M <= 64 (a short prefill: the reference's own hgemm
+// Skinny GEMM for sm_100a: C[M,N] = A[M,K] . B with 8 < M <= 64, and for narrow matrices with a long K some hundred rows, 64 of
+// them per CTA (a short prefill: the reference's own hgemm
 // benchmark shape is 64 x 2048 . 2048 x 8192, hgemm.zig:446-542).  Such a product is bound by HBM, not by the tensor
 // cores: B is read once (N*K*2 bytes) and everything else is small.  Two things keep the general tcgen05 kernel far
 // from the HBM rate at these shapes, and this kernel removes both:
@@ -21,6 +22,8 @@
 // [row][128 columns], then 16-byte pieces of rows go to the workspace or, through the glue, to C.
 // Every mbarrier wait is bounded as in the general kernel.
 // BF16: bfloat16 operands and output with the glue of md_lin (a gated product combines columns c and c + 32 of a tile).
+#include <algorithm>
+
 #include "md_internal.cuh"
 #include "tc_common.cuh"
 
@@ -39,11 +42,12 @@ constexpr int THREADS = 192;
 constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + 256;
 constexpr uint32_t TMEM_COLS = 64;
 constexpr int MAX_SPLITS = 8;          // portable cluster size
+constexpr int MAX_ROWS = 1024;         // 64 per CTA
 
 template <bool W_MN_MAJOR, bool BF16>
 __global__ void __launch_bounds__(THREADS, 2)
-gemm_skinny_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, __half* C, int M,
-                   int N, int K, int kb_per_split, int splits, int early, md_epilogue ep, md_devflags* flags, md_lin lin) {
+gemm_skinny_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, __half* C, int all_rows,
+                   int N, int K, int kb_per_split, int splits, int early, int wide_glue, md_epilogue ep, md_devflags* flags, md_lin lin) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
@@ -58,6 +62,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tile = blockIdx.x, split = blockIdx.y;
     const int n0 = tile * TILE_N;
+    const int m_first = blockIdx.z * XN, M = min(XN, all_rows - m_first);    // this CTA's rows of A and C
+    C += (size_t)m_first * (BF16 && lin.glu ? N / 2 : N);
     const int num_kb = (K + BLOCK_K - 1) / BLOCK_K;
     const int kb0 = split * kb_per_split;
     const int kbs = max(0, min(kb_per_split, num_kb - kb0));   // 0 for a split past the end of K: it contributes zeros
@@ -102,7 +108,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 }
             };
             auto load_x = [&](int stage, int kb) {
-                tma_load_2d(smem_x + stage * X_STAGE_BYTES, &tm_x, bar_full + 8 * stage, kb * BLOCK_K, 0);
+                tma_load_2d(smem_x + stage * X_STAGE_BYTES, &tm_x, bar_full + 8 * stage, kb * BLOCK_K, m_first);
             };
             // the first ring of weight tiles does not depend on the predecessor kernel (registered weights are
             // never written on the stream): request it before waiting for the activations' producer
@@ -217,8 +223,32 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 return;
             }
             if (n >= N || m >= M) return;   // N % 8 == 0: a piece of four columns is inside or outside C
-            const __half2 lo = __floats2half2_rn(md_epilogue_value(ep, acc.x, m, n, N), md_epilogue_value(ep, acc.y, m, n + 1, N));
-            const __half2 hi = __floats2half2_rn(md_epilogue_value(ep, acc.z, m, n + 2, N), md_epilogue_value(ep, acc.w, m, n + 3, N));
+            if (wide_glue) {     // every operand of the glue four at a time, all of them requested together
+                const int mr = m_first + m, rr = ep.residual_rows > 0 ? mr % ep.residual_rows : mr;
+                uint2 b = make_uint2(0, 0), r1 = b, r2 = b;
+                if (ep.bias) b = *reinterpret_cast<const uint2*>(ep.bias + n);
+                if (ep.residual) r1 = __ldcg(reinterpret_cast<const uint2*>(ep.residual + (size_t)rr * N + n));
+                if (ep.residual2) r2 = __ldcg(reinterpret_cast<const uint2*>(ep.residual2 + (size_t)mr * N + n));
+                __half2 h[2] = {__floats2half2_rn(acc.x, acc.y), __floats2half2_rn(acc.z, acc.w)};
+                auto add = [&](const uint2& u) {     // an f16 + f16 sum is exact in f32: one rounding either way
+                    h[0] = __hadd2(h[0], *reinterpret_cast<const __half2*>(&u.x));
+                    h[1] = __hadd2(h[1], *reinterpret_cast<const __half2*>(&u.y));
+                };
+                if (ep.bias) add(b);
+                if (ep.gelu) {
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const float2 f = __half22float2(h[j]);
+                        h[j] = __floats2half2_rn(md_gelu_f32(f.x), md_gelu_f32(f.y));
+                    }
+                }
+                if (ep.residual) add(r1);
+                if (ep.residual2) add(r2);
+                *reinterpret_cast<uint2*>(C + (size_t)m * N + n) = *reinterpret_cast<const uint2*>(h);
+                return;
+            }
+            const __half2 lo = __floats2half2_rn(md_epilogue_value(ep, acc.x, m_first + m, n, N), md_epilogue_value(ep, acc.y, m_first + m, n + 1, N));
+            const __half2 hi = __floats2half2_rn(md_epilogue_value(ep, acc.z, m_first + m, n + 2, N), md_epilogue_value(ep, acc.w, m_first + m, n + 3, N));
             uint2 pk;
             pk.x = *reinterpret_cast<const uint32_t*>(&lo);
             pk.y = *reinterpret_cast<const uint32_t*>(&hi);
@@ -274,12 +304,32 @@ int md_make_map_2d(md_ctx* ctx, CUtensorMap* map, const void* ptr, uint64_t inne
                    uint32_t box_outer, uint64_t ld, bool swizzle_64 = false);
 
 bool md_gemm_skinny_supported(const void* a, const void* b, const void* c, size_t M, size_t N, size_t K) {
-    if (M <= 8 || M > (size_t)XN || N == 0 || K == 0) return false;
+    if (M <= 8 || M > (size_t)MAX_ROWS || N == 0 || K == 0) return false;
     if ((K % 8) != 0 || (N % 8) != 0) return false;  // row strides must be multiples of 16 bytes for TMA
     if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) return false;
     if (reinterpret_cast<uintptr_t>(c) & 7) return false;  // 8-byte stores of four outputs
     return N <= (1u << 30) && K <= (1u << 30);
 }
+
+namespace {
+
+typedef void (*skinny_fn)(CUtensorMap, CUtensorMap, __half*, int, int, int, int, int, int, int, md_epilogue, md_devflags*, md_lin);
+
+int blocks_of(size_t M) { return (int)((M + XN - 1) / XN); }
+
+// Splits of K = CTAs per cluster, up to the portable cluster size, at least two k-blocks each.  One block of rows: about two CTAs per
+// SM, a power of two.  Several: what one wave of clusters holds, 7/4 CTAs per SM, since a cluster keeps to one part of the chip
+// (192 rows of 2048 x 8192: 16.0 us in four splits, 22.8 in six, whose last clusters wait for the first).
+int splits_for(const md_ctx* ctx, size_t M, size_t N, size_t K) {
+    const int units = (int)((N + TILE_N - 1) / TILE_N) * blocks_of(M), most = std::min((int)((K + BLOCK_K - 1) / BLOCK_K) / 2, MAX_SPLITS);
+    if (M > (size_t)XN) return std::max(1, std::min(ctx->sm_count * 7 / 4 / units, most));
+    const int want = std::min(ctx->skinny_splits > 0 ? ctx->skinny_splits : (2 * ctx->sm_count) / units, most);
+    int splits = 1;
+    while (splits * 2 <= want) splits *= 2;
+    return splits;
+}
+
+}  // namespace
 
 // Against the general kernel's tiles of 64 columns, for f16 products.  That one takes 0.2 to 0.25 us per k-block whatever its
 // bytes (the issuing thread's waits, MMAs and commit), rounds over the SMs one after the other, and hardly more for more rows;
@@ -293,25 +343,35 @@ bool md_gemm_skinny_supported(const void* a, const void* b, const void* c, size_
 // A fused GELU stays here: this epilogue has tanhf, the general one the hardware's tanh, whose error of 2^-11 is up to 15 places of
 // the f16 result at -2, where tanh is near -1 and the GELU is what is left of it.
 bool md_gemm_skinny_wanted(const md_ctx* ctx, size_t M, size_t N, size_t K, bool gelu) {
-    if (ctx->skinny_splits >= 0 || gelu) return true;
-    const size_t tiles = (N + 63) / 64, rounds = (tiles + ctx->sm_count - 1) / ctx->sm_count, kblocks = (K + BLOCK_K - 1) / BLOCK_K;
+    if (ctx->skinny_splits >= 0) return M <= (size_t)XN;
+    const size_t kblocks = (K + BLOCK_K - 1) / BLOCK_K;
+    if (M > (size_t)XN) {
+        // More rows, 64 per CTA: narrow products with a long K, which leave the general kernel a few CTAs with all of K each, 0.14 us
+        // per k-block.  Here 4.8 us, 0.225 per k-block of a split, the weights once and 0.2 per block of rows.  us here and there:
+        //   2048 x 8192: 65 rows 12.1 and 21.2   128: 13.0 and 21.3   192: 15.2 and 21.0   256: 16.3 and 21.0   320: 19.2 and 21.5
+        //   1152 x 4352: 65 rows 7.5 and 11.4    256: 10.0 and 11.9   384: 11.0 and 12.0      512 x 8192: 1024 rows 15.5 and 19.8
+        //   2048 x 2048: 65 rows 6.9 and 6.4     2048 x 3072: 192 rows 9.8 and 9.5            3072 x 4096: 100 rows 14.4 and 13.5
+        // The line is at four fifths of that time: this kernel takes every SM, and a product with less to gain costs more than that
+        // where another one runs beside it (a Phi prompt of 300 rows 2.49 -> 2.66 ms with the line at 0.95).  With it, f16 prompts
+        // of 70, 100, 128 and 192 rows of the 24 layers: 2.26 -> 2.18, 2.28 -> 2.22, 2.29 -> 2.21 and 2.50 -> 2.35 ms.
+        // The bfloat16 products of the layer stacks keep the general kernel: prompts of 70 to 320 rows were 2 % faster to 1 % slower.
+        if (ctx->tc_block_n || ctx->tc_pair >= 0 || ctx->tc_splitk) return false;
+        const int splits = splits_for(ctx, M, N, K);
+        const double here = 4.8 + 0.225 * (double)((kblocks + splits - 1) / splits) + 0.24e-6 * (double)N * (double)K + 0.2 * blocks_of(M);
+        return splits > 1 && here < 0.8 * md_gemm_tc_time(ctx, M, N, K);
+    }
+    if (gelu) return true;
+    const size_t tiles = (N + 63) / 64, rounds = (tiles + ctx->sm_count - 1) / ctx->sm_count;
     return tiles < 96 || rounds * kblocks + 24 > M;
 }
 
 namespace {
 
-typedef void (*skinny_fn)(CUtensorMap, CUtensorMap, __half*, int, int, int, int, int, int, md_epilogue, md_devflags*, md_lin);
-
 int launch_splits(md_ctx* ctx, skinny_fn kern, uint32_t cfg_bit, const CUtensorMap& tm_w, const CUtensorMap& tm_x, __half* c, size_t M,
                   size_t N, size_t K, const md_epilogue& ep, const md_lin& lin) {
     const int tiles = (int)((N + TILE_N - 1) / TILE_N);
     const int num_kb = (int)((K + BLOCK_K - 1) / BLOCK_K);
-    // splits of K = CTAs per cluster: about two CTAs per SM in one wave, a power of two up to the portable cluster
-    // size of 8, at least two k-blocks per split
-    int want = ctx->skinny_splits > 0 ? ctx->skinny_splits : (2 * ctx->sm_count) / tiles;
-    if (want > num_kb / 2) want = num_kb / 2;
-    int splits = 1;
-    while (splits * 2 <= want && splits * 2 <= MAX_SPLITS) splits *= 2;
+    const int splits = splits_for(ctx, M, N, K);
     const int kb_per_split = (num_kb + splits - 1) / splits;
     if (!(ctx->tc_configured & cfg_bit)) {
         MD_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
@@ -319,7 +379,7 @@ int launch_splits(md_ctx* ctx, skinny_fn kern, uint32_t cfg_bit, const CUtensorM
     }
     ctx->last_tc_tile = 1000 + splits;   // md_get_option("last_tc_tile"): 1000 + S = the skinny kernel with S splits
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)tiles, (unsigned)splits);
+    cfg.gridDim = dim3((unsigned)tiles, (unsigned)splits, (unsigned)blocks_of(M));
     cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = SMEM_BYTES;
     cfg.stream = ctx->stream;
@@ -340,7 +400,9 @@ int launch_splits(md_ctx* ctx, skinny_fn kern, uint32_t cfg_bit, const CUtensorM
     cfg.attrs = attr;
     cfg.numAttrs = na;
     const int Mi = (int)M, Ni = (int)N, Ki = (int)K;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tm_w, tm_x, c, Mi, Ni, Ki, kb_per_split, splits, md_launch_early(ctx), ep, ctx->flags, lin);
+    const uintptr_t glue = reinterpret_cast<uintptr_t>(ep.bias) | reinterpret_cast<uintptr_t>(ep.residual) | reinterpret_cast<uintptr_t>(ep.residual2);
+    const int wide_glue = (glue & 7) == 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tm_w, tm_x, c, Mi, Ni, Ki, kb_per_split, splits, md_launch_early(ctx), wide_glue, ep, ctx->flags, lin);
     if (e != cudaSuccess) return md_fail(ctx, MD_ERR_CUDA, "launch of gemm_skinny_kernel failed: %s", cudaGetErrorString(e));
     ctx->launches++;
     return MD_OK;
@@ -351,7 +413,7 @@ int launch_splits(md_ctx* ctx, skinny_fn kern, uint32_t cfg_bit, const CUtensorM
 int md_launch_gemm_skinny(md_ctx* ctx, const __half* a, const __half* b, __half* c, size_t M, size_t N, size_t K,
                           int b_layout, const md_epilogue& ep) {
     if (!md_gemm_skinny_supported(a, b, c, M, N, K))
-        return md_fail(ctx, MD_ERR_UNSUPPORTED, "skinny GEMM needs 8 < M <= 64, K %% 8 == 0, N %% 8 == 0 and 16-byte aligned operands");
+        return md_fail(ctx, MD_ERR_UNSUPPORTED, "skinny GEMM needs 8 < M <= 1024, K %% 8 == 0, N %% 8 == 0 and 16-byte aligned operands");
     const bool mn = (b_layout == 0);
     CUtensorMap tm_w, tm_x;
     if (mn) MD_TRY(md_make_map_2d(ctx, &tm_w, b, N, K, 64, BLOCK_K, 0));
@@ -363,7 +425,7 @@ int md_launch_gemm_skinny(md_ctx* ctx, const __half* a, const __half* b, __half*
 
 int md_launch_gemm_skinny_lin(md_ctx* ctx, const void* a, const void* b, void* c, size_t M, size_t N, size_t K, const md_lin& lin) {
     if (!md_gemm_skinny_supported(a, b, c, M, N, K) || lin.tile_expert || lin.out_f32)
-        return md_fail(ctx, MD_ERR_UNSUPPORTED, "skinny GEMM needs 8 < M <= 64, K %% 8 == 0, N %% 8 == 0 and 16-byte aligned operands");
+        return md_fail(ctx, MD_ERR_UNSUPPORTED, "skinny GEMM needs 8 < M <= 1024, K %% 8 == 0, N %% 8 == 0 and 16-byte aligned operands");
     CUtensorMap tm_w, tm_x;
     MD_TRY(md_make_map_2d_bf16(ctx, &tm_w, b, K, N, BLOCK_K, TILE_N, false));
     MD_TRY(md_make_map_2d_bf16(ctx, &tm_x, a, K, M, BLOCK_K, XN, false));

@@ -644,7 +644,7 @@ int launch(md_ctx* ctx, const __half* a, const __half* b, __half* c, size_t M, s
     return launch_as<BLOCK_N, B_MN_MAJOR, MT, false>(ctx, a, b, c, M, N, K, ep, ldc, push, lda, splits);
 }
 
-struct TileChoice { int bn = 64, mt = 1; bool pair = false; };
+struct TileChoice { int bn = 64, mt = 1; bool pair = false; double us = 0.0; };
 
 // The tile of a product that covers the machine many times over: the bytes an SM pulls from L2 per k-block, (rows + columns) x 128,
 // decide (there the clock under the power cap follows them too).  Cost = (waves over the SMs) x (rows + columns); the 256 x 256 tile
@@ -702,12 +702,15 @@ TileChoice choose_tile(const md_ctx* ctx, size_t M, size_t N, size_t K, bool glu
         const size_t n = ((M + rows - 1) / rows) * ((N + t.bn - 1) / t.bn), waves = (n + at_once - 1) / at_once;
         const double l2 = (double)n * kblocks * (double)(rows + t.bn) * BLOCK_K * 2 / 20e6, sm = (double)waves * (kblocks * t.kb + t.wave);
         const double cost = t.fixed + (glue ? t.with_glue : 0.0) + (l2 > sm ? l2 : sm);
-        if (best < 0.0 || cost < best) { best = cost; c.bn = t.bn; c.mt = t.mt; c.pair = t.pair; }
+        if (best < 0.0 || cost < best) { best = cost; c.bn = t.bn; c.mt = t.mt; c.pair = t.pair; c.us = cost; }
     }
     return c;
 }
 
 }  // namespace
+
+// (nothing for products above the few-wave rule: those are not split)
+double md_gemm_tc_time(const md_ctx* ctx, size_t M, size_t N, size_t K) { return choose_tile(ctx, M, N, K, false).us; }
 
 bool md_gemm_tc_supported(const void* a, const void* b, const void* c, size_t M, size_t N, size_t K, int b_layout) {
     (void)b_layout;

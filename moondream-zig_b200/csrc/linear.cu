@@ -92,7 +92,7 @@ int md_linear(md_ctx* ctx, int dtype, const void* a, const void* w, void* c, siz
         }
         if ((N % 8) == 0 && !ep.out_f32) {
             const bool bias_ok = (reinterpret_cast<uintptr_t>(ep.bias) & 15) == 0;   // the general kernel reads four values at a time
-            if (!ep.tile_expert && ctx->skinny && md_gemm_skinny_supported(a, w, c, M, N, K))
+            if (!ep.tile_expert && ctx->skinny && M <= 64 && md_gemm_skinny_supported(a, w, c, M, N, K))
                 return md_launch_gemm_skinny_lin(ctx, a, w, c, M, N, K, ep);
             if (bias_ok) return md_launch_gemm_tc_lin(ctx, a, w, c, M, N, K, ep);
         }

@@ -77,7 +77,7 @@ struct md_ctx {
     uint32_t lin_configured = 0;   // bfloat16 GEMM kernels whose dynamic shared memory limit has been raised
     uint32_t pair_configured = 0;  // the same for the instantiations of gemm_pair_kernel
     uint32_t tc_configured = 0;  // tcgen05 kernels whose dynamic shared memory limit has been raised
-    int skinny = 1;          // md_set_option("skinny"): 8 < M <= 64 takes the swapped-operand split-K kernel
+    int skinny = 1;          // md_set_option("skinny"): few rows take the swapped-operand split-K kernel
     int skinny_splits = -1;  // md_set_option("skinny_splits"): -1 = by shape, where the shape wants that kernel; otherwise it is taken
                              // wherever it can be, with an automatic (0) or this number of K splits
     bool sdpa_mma_configured = false;  // the same for the mma.sync attention kernels
@@ -270,6 +270,7 @@ int md_launch_gemv_dual_k(md_ctx* ctx, const __half* x1, const __half* w1, const
 int md_launch_gemm_simt(md_ctx* ctx, const __half* a, const __half* b, __half* c, size_t M, size_t N, size_t K,
                         int b_layout, const md_epilogue& ep);
 // gemm_tc.cu: tcgen05 + TMA; returns MD_ERR_UNSUPPORTED when alignment rules are not met.
+double md_gemm_tc_time(const md_ctx* ctx, size_t M, size_t N, size_t K);   // us that the tile it would take is expected to need
 bool md_gemm_tc_supported(const void* a, const void* b, const void* c, size_t M, size_t N, size_t K, int b_layout);
 int md_launch_gemm_tc(md_ctx* ctx, const __half* a, const __half* b, __half* c, size_t M, size_t N, size_t K,
                       int b_layout, const md_epilogue& ep);
@@ -280,7 +281,7 @@ int md_launch_gemm_tc_ex(md_ctx* ctx, const __half* a, const __half* b, __half* 
 // comm.cu: gathered [world][M][n_local] -> c [M][world * n_local] (n_local % 8 == 0, 16-byte aligned)
 int md_launch_gather_colblocks(md_ctx* ctx, const uint16_t* gathered, uint16_t* c, size_t world, size_t M, size_t n_local);
 
-// gemm_skinny.cu: 8 < M <= 64, weights as the MMA's M side, split-K over a thread-block cluster
+// gemm_skinny.cu: 8 < M <= 1024 (64 rows per CTA), weights as the MMA's M side, split-K over a thread-block cluster
 bool md_gemm_skinny_supported(const void* a, const void* b, const void* c, size_t M, size_t N, size_t K);
 bool md_gemm_skinny_wanted(const md_ctx* ctx, size_t M, size_t N, size_t K, bool gelu);   // rather than the general kernel
 int md_launch_gemm_skinny(md_ctx* ctx, const __half* a, const __half* b, __half* c, size_t M, size_t N, size_t K,

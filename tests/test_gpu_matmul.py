@@ -457,6 +457,45 @@ def test_few_rows_take_the_faster_of_two_kernels(pkg, oracle, m, n, k, general):
     ctx.close()
 
 
+@pytest.mark.parametrize("layout", [0, 1])
+@pytest.mark.parametrize("m,n,k,few", [(65, 8, 8192, True), (128, 136, 4104, True), (129, 1000, 8192, True), (192, 2048, 8192, True),
+                                       (1024, 512, 8192, True), (100, 1152, 4352, True), (256, 2048, 8192, False),
+                                       (1025, 512, 8192, False), (65, 2048, 2048, False), (100, 8192, 8192, False)])
+def test_many_rows_of_a_narrow_product(pkg, oracle, m, n, k, few, layout):
+    """More than 64 rows: narrow products with a long K take the split-K kernel with 64 rows per CTA, up to 1024 rows; a last block of
+    one row, ragged N and K, the glue (the residual's row is that of the whole product, not that of its block), and a bias at 2 bytes
+    past a boundary, which leaves these row counts to the kernel they had.  Against the oracle and, as for up to 64 rows, the general
+    kernel, whose hardware tanh is 2^-11 off."""
+    ctx = pkg.Context(0)
+    rng = np.random.default_rng(m + n + k)
+    a, w_kn = f16_normal(rng, (m, k)), f16_normal(rng, (k, n), 0.05)
+    w = w_kn if layout == 0 else np.ascontiguousarray(w_kn.T)
+    bias, res = f16_normal(rng, (n,), 0.5), f16_normal(rng, (m, n))
+    plain = oracle.hgemm_nn(a, w_kn)
+    da, dw, out = ctx.upload(a), ctx.upload(w), ctx.alloc((m, n))
+    (ctx.hgemm_nt if layout else ctx.hgemm_nn)(da, dw, m, n, k, out=out)
+    ctx.sync()
+    assert (ctx.get_option("last_tc_tile") >= 1000) == few
+    assert_close_ref(out.numpy(), plain, f"{m}x{n}x{k}")
+    ref = oracle.add(oracle.gelu(oracle.bias_add(plain, bias)), res)
+    db, dr = ctx.upload(bias), ctx.upload(res)
+    ctx.hgemm_fused(da, dw, out, m, n, k, layout, bias=db, gelu=True, residual=dr)
+    ctx.sync()
+    assert (ctx.get_option("last_tc_tile") >= 1000) == few
+    got = out.numpy()
+    assert_close_ref(got, ref, f"{m}x{n}x{k} with glue")
+    ctx.set_option("skinny", 0)
+    ctx.hgemm_fused(da, dw, out, m, n, k, layout, bias=db, gelu=True, residual=dr)
+    ctx.sync()
+    assert ctx.get_option("last_tc_tile") < 1000
+    assert_close_ref(got, out.numpy(), "against the general kernel", rel=2e-3)
+    ctx.set_option("skinny", 1)
+    moved = ctx.upload(np.concatenate([np.zeros(1, np.float16), bias]))
+    ctx.hgemm_fused(da, dw, out, m, n, k, layout, bias=moved.ptr + 2, gelu=True, residual=dr)
+    assert_close_ref(out.numpy(), ref, f"{m}x{n}x{k} with a bias at 2 bytes past a boundary")
+    ctx.close()
+
+
 @pytest.mark.parametrize("bytes_off", [2, 4, 8, 16])
 @pytest.mark.parametrize("m,n,k", [(7, 512, 256), (40, 512, 256), (64, 8192, 512), (65, 512, 256), (300, 1032, 520)])
 def test_glue_operands_at_any_address(pkg, oracle, m, n, k, bytes_off):
