@@ -5,7 +5,7 @@
 // Structure (one persistent CTA per SM, 320 threads):
 //   warp 0      TMA producer: cp.async.bulk.tensor loads of the A tile (128 x 64) and the
 //               B tile (BLOCK_N x 64) into a ring of shared-memory stages, 128-byte swizzle.
-//   warp 1      MMA issuer: one lane issues tcgen05.mma (128 x BLOCK_N x 16, kind::f16) with
+//   warp 1      MMA issuer: one elected lane issues tcgen05.mma (128 x BLOCK_N x 16, kind::f16) with
 //               shared-memory descriptors; accumulators live in TMEM, two buffers of
 //               BLOCK_N columns so the epilogue of tile i overlaps the main loop of tile i+1.
 //               tcgen05.commit releases smem stages and publishes finished accumulators.
@@ -14,7 +14,8 @@
 //               256-511), because the kernel is bound by the bytes an SM pulls from L2 per flop:
 //               64 KB per 1024 tensor cycles instead of 48 KB per 512.
 //   warps 2..9  epilogue: tcgen05.ld (32 lanes x 32 columns) -> fused glue -> f16 ->
-//               swizzled smem -> TMA store (clips the M and N tails).
+//               swizzled smem -> TMA store (clips the M and N tails), 32 columns at a time through
+//               two buffers per warp (64 in the column-split form: one buffer).
 //               Column-split GEMM (push.tma): every staged chunk also leaves as one TMA store per peer into
 //               the other GPUs' copies of C; the warp goes on when the stores have read the chunk.
 //   warps 10..17 (column-split GEMM with push.tma = 0) push: once a tile's TMA stores have completed they read
@@ -46,7 +47,7 @@ namespace {
 
 constexpr int BLOCK_M = 128, BLOCK_K = 64, UMMA_K = 16;
 constexpr int A_STAGE_BYTES = BLOCK_M * BLOCK_K * 2;     // 16 KiB
-constexpr int EPI_WARPS = 8, EPI_BUF_BYTES = 32 * 128;   // 32 rows x 64 f16 per epilogue warp
+constexpr int EPI_WARPS = 8, EPI_BUF_BYTES = 32 * 128;   // per epilogue warp: two buffers of 32 rows x 32 f16, or one of 64
 constexpr int EPI_BYTES = EPI_WARPS * EPI_BUF_BYTES;     // 32 KiB
 constexpr int NUM_THREADS = (2 + EPI_WARPS) * 32;
 constexpr int PUSH_WARPS = 8;                            // extra warps of the column-split form
@@ -691,8 +692,8 @@ TileChoice choose_tile_large(const md_ctx* ctx, size_t M, size_t N, size_t K, bo
 TileChoice choose_tile(const md_ctx* ctx, size_t M, size_t N, size_t K, bool glue) {
     if (((M + BLOCK_M - 1) / BLOCK_M) * ((N + 255) / 256) > 2 * (size_t)ctx->sm_count) return choose_tile_large(ctx, M, N, K, glue, 0);
     struct Tile { int bn, mt; bool pair; double kb, fixed, wave, with_glue; };
-    static const Tile tiles[5] = {{64, 1, false, 0.14, 2.9, 0.15, 0.3}, {128, 1, false, 0.165, 3.7, 0.4, 0.6}, {256, 1, false, 0.28, 5.1, 0.3, 1.2},
-                                  {256, 1, true, 0.29, 5.1, 0.3, 1.2}, {256, 2, false, 0.55, 5.8, 4.2, 2.0}};
+    static const Tile tiles[4] = {{64, 1, false, 0.14, 2.9, 0.15, 0.3}, {128, 1, false, 0.165, 3.7, 0.4, 0.6}, {256, 1, false, 0.28, 5.1, 0.3, 1.2},
+                                  {256, 1, true, 0.29, 5.1, 0.3, 1.2}};     // (256 x 256 on one CTA, 0.55 us per k-block, never wins here)
     const double kblocks = (double)((K + BLOCK_K - 1) / BLOCK_K);
     TileChoice c;
     double best = -1.0;
