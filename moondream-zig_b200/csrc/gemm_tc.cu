@@ -590,7 +590,7 @@ int launch_as(md_ctx* ctx, const __half* a, const __half* b, __half* c, size_t M
     memset(&pm, 0, sizeof(pm));
     if (PUSH && push.tma)
         for (int i = 0; i < push.n; ++i) MD_TRY(make_map_2d(ctx, &pm.m[i], push.base[i], N, M, 64, 32, ldc));
-    const int early = ctx->pdl && md_launch_early(ctx) && !PUSH;
+    const int early = md_launch_early_rows(ctx) && !PUSH;
     const int units = num_tiles * splits;
     const int grid = units < ctx->sm_count ? units : ctx->sm_count;
     // the split-K instantiation exists for single 128-row tiles of 256 columns without peers only
@@ -623,7 +623,7 @@ int launch_lin(md_ctx* ctx, const void* a, const void* b, void* c, size_t M, siz
     MD_TRY(make_map_2d(ctx, &tm_c, c, lin.glu ? N / 2 : N, M, 32, 32, 0, true, true));
     const int tiles_m = (int)((M + MT * BLOCK_M - 1) / (MT * BLOCK_M)), tiles_n = (int)((N + BLOCK_N - 1) / BLOCK_N);
     const int num_tiles = tiles_m * tiles_n, grid = num_tiles < ctx->sm_count ? num_tiles : ctx->sm_count;
-    const int early = ctx->pdl && md_launch_early(ctx) && !lin.tile_expert;
+    const int early = md_launch_early_rows(ctx) && !lin.tile_expert;
     auto kern = gemm_tc_kernel<BLOCK_N, false, MT, false, false, true>;
     constexpr int smem = smem_bytes(BLOCK_N, MT);
     const uint32_t bit = 1u << (MT == 2 ? 3 : BLOCK_N == 256 ? 0 : BLOCK_N == 128 ? 1 : 2);

@@ -525,6 +525,29 @@ def test_many_rows_of_a_narrow_product(pkg, oracle, m, n, k, few, layout):
     ctx.close()
 
 
+@pytest.mark.parametrize("m,n,k,few", [(128, 512, 8192, True), (300, 1024, 2048, False), (1024, 2048, 2048, False)])
+def test_products_of_two_activations_back_to_back_under_the_pdl_option(pkg, m, n, k, few):
+    """Option pdl lets kernels request weights ahead of the call before them.  A product of more than 64 rows may have as its B what the
+    call before it wrote: B = X . W^T of changing X, then A . B^T, in a row without a synchronisation, is what it is without the option."""
+    ctx = pkg.Context(0)
+    rng = np.random.default_rng(n)
+    da, out = ctx.upload(f16_normal(rng, (m, k))), [ctx.alloc((m, n)) for _ in range(8)]
+    dx, dw = [ctx.upload(f16_normal(rng, (n, 64), 0.3)) for _ in range(8)], ctx.upload(f16_normal(rng, (k, 64), 0.3))
+    b = ctx.alloc((n, k))
+    runs = []
+    for pdl in (0, 1):
+        ctx.set_option("pdl", pdl)
+        for i in range(8):
+            ctx.hgemm_nt(dx[i], dw, n, k, 64, out=b)
+            ctx.hgemm_nt(da, b, m, n, k, out=out[i])
+        ctx.sync()
+        assert (ctx.get_option("last_tc_tile") >= 1000) == few
+        runs.append([o.numpy().copy() for o in out])
+    for i in range(8):
+        np.testing.assert_array_equal(runs[0][i], runs[1][i])
+    ctx.close()
+
+
 @pytest.mark.parametrize("bytes_off", [2, 4, 8, 16])
 @pytest.mark.parametrize("m,n,k", [(7, 512, 256), (40, 512, 256), (64, 8192, 512), (65, 512, 256), (300, 1032, 520)])
 def test_glue_operands_at_any_address(pkg, oracle, m, n, k, bytes_off):
